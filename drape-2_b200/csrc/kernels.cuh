@@ -101,7 +101,9 @@ struct Params {
   int pcgVariant;       // the block-Jacobi PCG form: 0 reference order (resident rows where the scene fits), 1 pipelined,
                         // 2 Chronopoulos-Gear, 3 reference order on the 1024-thread kernel (kept in the view so that
                         // captured frame graphs are recaptured when it changes)
-  uint32_t slicedSlots; // k_solve_rows: padded slots of the sliced layout a block may hold in shared memory
+  uint32_t slicedSlots; // k_solve_rows_learned: padded slots of the sliced layout a block may hold in shared memory
+  uint32_t residentSlots, residentNodes;  // k_solve_rows: a block's padded slots and its rows and halo, in shared memory
+  uint32_t haloStride;  // entries of `halo` per solve block
   unsigned long long barrierLimitNs;
 };
 
@@ -136,7 +138,11 @@ struct Dev {
   float* blocks;   // 9 planes of slotsPadded floats, component 3*row+col
   float4* precond; // 3 float4 (rows) per particle
   Contact* contact;
+  const uint16_t* localCol;   // per slot: its column among its solve block's rows and halo (k_localize)
+  const uint32_t *halo, *haloCount;
   double* partials;
+  struct MailWord* mail;      // the solve grid's mailbox and the number of the last exchange (exchange.cuh)
+  unsigned long long* mailSeq;
   Control* ctl;
   int* cgLog;  // kCgLogCapacity entries
 };
@@ -217,6 +223,12 @@ struct GridSync {
     return ok != 0;
   }
 };
+
+}  // namespace dcu
+
+#include "exchange.cuh"
+
+namespace dcu {
 
 // Block-wide FP64 sums (or maxima); thread 0 gets the result in out. Fixed tree shape, so deterministic.
 template <int K, bool Max = false>
@@ -1000,18 +1012,355 @@ __device__ inline int pcgReferenceOrder(const Dev& D, GridSync& gs, const SmemMa
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// Reference-order PCG with resident rows (k_solve_rows; the form pcgVariant 0 runs where a scene fits it). One thread owns one row of its block for the
-// whole solve and keeps the row's PCG state (p, A p and its filtered copy, r, step, resid, z, the contact plane and
-// the preconditioner block) in registers, so an iteration's only global traffic is the gather of z_j over the row's
-// columns and the store of the new z_i: the reference-order kernel re-reads the row vectors from L2 in both passes.
-// The block's slots sit in shared memory in a sliced layout: the rows in warps of 32, warp w's slots padded to its
-// longest row L_w, slot k of lane l at base_w + 32 k + l (nine planes, then the columns; padding holds kPinnedBit),
-// so a warp's 32 row threads read 32 consecutive words. The row's product keeps the two-lane order of
-// pcgReferenceOrder<2> (the even slots in one sum, the odd slots in another, added at the end) and the FP64 partials
-// are grouped as that kernel groups them (p.Ap by half-warps; the others fall on the same threads), so the iterates
-// are that kernel's bit for bit.
-constexpr int kRowThreads = 512;     // k_solve_rows block size: a block's rows must not exceed it
-constexpr int kResidentRows = 4;     // the solve templates' Variant value of this form
+// Reference-order PCG with resident rows (k_solve_rows; the form pcgVariant 0 runs where a scene fits it). One thread
+// owns one row of its block for the whole solve and keeps the row's PCG state (p, A p and its filtered copy, r, step,
+// resid, z, the contact plane and the preconditioner block) and its first kRegSlots matrix blocks in registers; the
+// other blocks sit in shared memory in a sliced layout (the rows in warps of 32, warp w's rows padded to its longest,
+// slot k of lane l at base_w + 32 k + l), beside the z of every particle the block's rows couple to (its own rows, then
+// its halo: the other blocks' particles, listed once per build by k_localize, which also gives every slot the index of
+// its column among them). The row's product keeps the two-lane order of pcgReferenceOrder<2> (the even slots in one
+// sum, the odd slots in another, added at the end), so the iterates are that kernel's.
+//
+// The blocks exchange by messages (exchange.cuh). The new z carries the iteration's tag in its fourth component, so a
+// block takes its halo as soon as it is there, with no barrier; and since A p = A z + beta A pPrev, the sums r.r and r.z
+// that give beta travel while the rows form A z. Only the sum p.Ap, which gives alpha, is waited for. One warp of the
+// block does the sums, the scalars and the stopping tests; the others hold the rows.
+//
+// Measured (us per PCG iteration, one B200; with a counter barrier for each sum, z gathered from the L2 and the matrix
+// read four bytes at a time before): 1,600 particles 2.9 (was 6.9), 10k 3.0 (7.2), 60k 4.3 (8.4). What bounds it now: for
+// small scenes the two exchanges one after the other (about 1.1 us each with their block sums) and the FP64 division
+// and square root between them; at 60k the way of z to the neighbours (about 0.8 us), then the product (38 bytes of
+// shared memory a slot and 16 a gathered z, against 128 bytes a clock: 1.3 us), then one exchange. Fewer blocks than SMs
+// for small scenes: 2.7-2.9 us for 8 to 148 blocks at 1,600 particles, slower at 4,000 and 10k. A row's slots four at a
+// time with two slots in registers: 4.31 us at 60k; two at a time 4.39, six 4.43; four or six slots in registers spill
+// (4.30-4.32). Exchange delays of 500-900 cycles are within 3 % of each other; none costs 8-15 % on small scenes.
+constexpr int kRowThreads = 512;    // k_solve_rows block size
+constexpr int kRowWorkers = 480;    // of these, the threads that own a row each; the last warp does the exchanges
+constexpr int kResidentRows = 4;    // the solve templates' Variant value of this form
+constexpr int kRegSlots = 2;        // slots of each row kept in registers (even, so that slot parity is the same)
+constexpr int kExchangeDelay = 700; // clock cycles before an exchange's first poll
+constexpr uint32_t kNoColumn = 0xFFFFu;  // localCol of a pinned column
+
+// Shared memory of one padded slot (nine floats and a 16-bit column) and of one particle's z.
+constexpr uint32_t kResidentSlotBytes = 38, kResidentNodeBytes = 16;
+
+struct ResidentMatrix {
+  const float4 *a, *b;     // blocks of the slots in shared memory: components 0-3 and 4-7
+  const float* c;          // component 8
+  const uint32_t* cols;    // columns of slots 2m and 2m + 1: 16 bits each, at base_w / 2 + 32 m + lane
+  float4* z;               // z of the block's rows, then of its halo; the last entry is zero
+  uint32_t base, len;      // this thread's warp: its first position and its padded slots (even)
+  uint32_t rows, haloSize;
+  const uint32_t* halo;    // the halo's particles
+  float reg[kRegSlots][9];
+  uint32_t regCols[kRegSlots / 2];
+};
+
+// What the exchange warp tells the row warps, and their sums on the way to it.
+struct ResidentShared {
+  double red[2][kRowWorkers / 32];
+  float factor;  // beta, or alpha
+  int code;      // 0 go on, 1 stop, 2 an exchange gave up
+  int failed;    // a halo wait gave up
+};
+
+// Copies this block's rows [r0, r1) into registers and the sliced layout (all threads; ends with a block barrier).
+// Returns false, after raising error 4, when the block does not fit what the host sized (P.residentSlots,
+// P.residentNodes; the host picks k_solve_rows only for scenes whose every block fits, so this is a guard).
+__device__ inline bool stageResident(const Dev& D, uint32_t rank, uint32_t r0, uint32_t r1, ResidentMatrix& A) {
+  constexpr int kWarps = kRowWorkers / 32;
+  // The rows' first slots relative to the block's first, bit 31 set for pinned rows (they take no product).
+  __shared__ uint32_t off[kRowWorkers + 1];
+  __shared__ uint32_t warpLen[kWarps], warpBase[kWarps + 1];
+  const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5;
+  const uint32_t R = r1 - r0;
+  A.rows = R;
+  A.haloSize = __ldg(D.haloCount + rank);
+  A.halo = D.halo + static_cast<size_t>(rank) * D.P.haloStride;
+  if (R > static_cast<uint32_t>(kRowWorkers) || blockDim.x != static_cast<unsigned>(kRowThreads) ||
+      R + A.haloSize >= D.P.residentNodes) {
+    if (t == 0) atomicExch(&D.ctl->error, 4);
+    return false;
+  }
+  const uint32_t first = __ldg(D.rowStart + r0);  // r0 <= n: rowStart has n + 1 entries
+  uint32_t count = 0, rs = first;
+  if (t < R) {
+    rs = __ldg(D.rowStart + r0 + t);
+    const bool pinned = D.particle[r0 + t].pinned != 0u;
+    off[t] = (rs - first) | (pinned ? kPinnedBit : 0u);
+    if (!pinned) count = __ldg(D.rowStart + r0 + t + 1) - rs;
+  }
+  if (t == 0) off[R] = __ldg(D.rowStart + r1) - first;
+  const uint32_t longest = __reduce_max_sync(0xffffffffu, count);
+  if (lane == 0 && w < kWarps) warpLen[w] = longest > kRegSlots ? (longest - kRegSlots + 1u) & ~1u : 0u;
+  __syncthreads();
+  if (t == 0) {
+    uint32_t acc = 0;
+    for (int k = 0; k < kWarps; ++k) {
+      warpBase[k] = acc;
+      acc += 32u * warpLen[k];
+    }
+    warpBase[kWarps] = acc;
+  }
+  __syncthreads();
+  const uint32_t total = warpBase[kWarps], cap = D.P.residentSlots;
+  if (total > cap) {
+    if (t == 0) atomicExch(&D.ctl->error, 4);
+    return false;
+  }
+  float4* a = solveSmem;
+  float4* b = a + cap;
+  A.z = b + cap;
+  float* c = reinterpret_cast<float*>(A.z + D.P.residentNodes);
+  uint16_t* cols = reinterpret_cast<uint16_t*>(c + cap);
+  A.a = a;
+  A.b = b;
+  A.c = c;
+  A.cols = reinterpret_cast<const uint32_t*>(cols);
+  A.base = w < kWarps ? warpBase[w] : 0u;
+  A.len = w < kWarps ? warpLen[w] : 0u;
+  const uint32_t SP = D.P.slotsPadded, zeroNode = D.P.residentNodes - 1;
+  if (t == 0) A.z[zeroNode] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  // The row's first slots, and the padding of its lane.
+  uint32_t rc[kRegSlots];
+#pragma unroll
+  for (int k = 0; k < kRegSlots; ++k) {
+    const uint32_t col = static_cast<uint32_t>(k) < count ? __ldg(D.localCol + rs + k) : kNoColumn;
+    rc[k] = col == kNoColumn ? zeroNode : col;
+#pragma unroll
+    for (int q = 0; q < 9; ++q) A.reg[k][q] = col == kNoColumn ? 0.0f : __ldg(D.blocks + q * SP + rs + k);
+  }
+#pragma unroll
+  for (int k = 0; k < kRegSlots / 2; ++k) A.regCols[k] = rc[2 * k] | rc[2 * k + 1] << 16;
+  // 16-bit column of slot j (of those in shared memory) of the row at lane l of the warp whose slots start at `base`.
+  auto colAt = [](uint32_t base, uint32_t j, uint32_t l) { return base + (32u * (j >> 1) + l) * 2u + (j & 1u); };
+  for (uint32_t j = count > kRegSlots ? count - kRegSlots : 0u; j < A.len; ++j) {
+    const uint32_t pos = A.base + 32u * j + lane;
+    a[pos] = b[pos] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    c[pos] = 0.0f;
+    cols[colAt(A.base, j, lane)] = static_cast<uint16_t>(zeroNode);
+  }
+  // The slots, read in slot order (coalesced); each finds its row by bisection over off[].
+  const uint32_t S = off[R];
+  for (uint32_t k = t; k < S; k += blockDim.x) {
+    uint32_t lo = 0, hi = R;  // row lo's first slot <= k < row hi's first slot
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if ((off[mid] & ~kPinnedBit) <= k) lo = mid; else hi = mid;
+    }
+    if (off[lo] & kPinnedBit) continue;  // a pinned row's slot
+    const uint32_t j = k - off[lo];
+    if (j < kRegSlots) continue;
+    const uint32_t pos = warpBase[lo >> 5] + 32u * (j - kRegSlots) + (lo & 31u);
+    const uint32_t s = first + k;
+    const uint32_t col = __ldg(D.localCol + s);
+    float m[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) m[q] = col == kNoColumn ? 0.0f : __ldg(D.blocks + q * SP + s);
+    a[pos] = make_float4(m[0], m[1], m[2], m[3]);
+    b[pos] = make_float4(m[4], m[5], m[6], m[7]);
+    c[pos] = m[8];
+    cols[colAt(warpBase[lo >> 5], j - kRegSlots, lo & 31u)] = static_cast<uint16_t>(col == kNoColumn ? zeroNode : col);
+  }
+  __syncthreads();
+  return true;
+}
+
+// U of this thread's slots (U even) from slot k on: all their loads are issued before the first product.
+template <int U>
+__device__ __forceinline__ void residentSlots(const ResidentMatrix& A, uint32_t k, float3 (&acc)[2]) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t cc[U / 2];
+  float4 a[U], b[U], x[U];
+  float c[U];
+#pragma unroll
+  for (int u = 0; u < U / 2; ++u) cc[u] = A.cols[A.base / 2 + 16u * k + 32u * u + lane];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const uint32_t pos = A.base + 32u * (k + u) + lane;
+    a[u] = A.a[pos];
+    b[u] = A.b[pos];
+    c[u] = A.c[pos];
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) x[u] = A.z[(u & 1) ? cc[u / 2] >> 16 : cc[u / 2] & 0xFFFFu];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const float m[9] = {a[u].x, a[u].y, a[u].z, a[u].w, b[u].x, b[u].y, b[u].z, b[u].w, c[u]};
+    blockMulAddRn(acc[u & 1], m, xyz(x[u]));
+  }
+}
+
+// y_i (unfiltered) = sum over the row's unpinned columns j of A_ij z_j, for this thread's row, in pcgReferenceOrder<2>'s
+// order: slot k of the row into sum k mod 2, each sum in slot order, the odd sum added to the even one last. Pinned
+// columns and padding hold zero blocks and name the zero particle: they add +0 to a sum that is never -0.
+__device__ __forceinline__ float3 residentProduct(const ResidentMatrix& A) {
+  float3 acc[2] = {mk(0, 0, 0), mk(0, 0, 0)};
+  {
+    float4 x[kRegSlots];
+#pragma unroll
+    for (int k = 0; k < kRegSlots; ++k) x[k] = A.z[(k & 1) ? A.regCols[k / 2] >> 16 : A.regCols[k / 2] & 0xFFFFu];
+#pragma unroll
+    for (int k = 0; k < kRegSlots; ++k) blockMulAddRn(acc[k & 1], A.reg[k], xyz(x[k]));
+  }
+  uint32_t k = 0;
+  for (; k + 4 <= A.len; k += 4) residentSlots<4>(A, k, acc);
+  if (k < A.len) residentSlots<2>(A, k, acc);
+  return mk(__fadd_rn(acc[0].x, acc[1].x), __fadd_rn(acc[0].y, acc[1].y), __fadd_rn(acc[0].z, acc[1].z));
+}
+
+// This iteration's z of the halo into shared memory, each particle's as soon as it carries `tag`. Returns false when a
+// wait gave up.
+__device__ __forceinline__ bool takeHalo(const Dev& D, const ResidentMatrix& A, const float4* global, uint32_t tag) {
+  constexpr uint32_t kStep = kRowWorkers;
+  bool ok = true;
+  BoundedWait wait;
+  for (uint32_t h = threadIdx.x; h < A.haloSize && ok; h += 2 * kStep) {
+    const bool two = h + kStep < A.haloSize;
+    const float4* p0 = global + __ldg(A.halo + h);
+    const float4* p1 = global + __ldg(A.halo + (two ? h + kStep : h));
+    float3 v0, v1;
+    for (;;) {
+      const uint32_t t0 = loadTagged(p0, v0), t1 = loadTagged(p1, v1);
+      if (t0 == tag && t1 == tag) break;
+      if (wait.expired(D.ctl, D.P.barrierLimitNs)) {
+        ok = false;
+        break;
+      }
+    }
+    A.z[A.rows + h] = f4(v0);
+    if (two) A.z[A.rows + h + kStep] = f4(v1);
+  }
+  return ok;
+}
+
+// The reference-order PCG of pcgReferenceOrder (same recurrences, same stopping tests) over resident rows. Writes
+// step and resid of the block's rows; returns the iteration count, or -1 when an exchange gave up.
+//
+// Barriers: 1 hands the row warps' sums to the exchange warp (they only arrive), 3 its scalars to the row warps (it only
+// arrives), 2 is the row warps' own, between the z in shared memory and the product. The exchange warp evaluates every
+// stopping test, so all warps leave after the same exchange; a row warp whose halo wait gave up says so through `failed`
+// and leaves like the others.
+__device__ inline int pcgResident(const Dev& D, GridSync& gs, ResidentMatrix& A) {
+  constexpr int kWarps = kRowWorkers / 32;
+  __shared__ ResidentShared sh;
+  const int maxCg = D.P.maxCg;
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  const unsigned long long base = __ldcg(D.mailSeq);
+  if (threadIdx.x == 0) sh.failed = 0;
+  __syncthreads();
+  int it = 0, code = 0;
+  if (w == kWarps) {  // the exchange warp
+    double rz = 0.0, r0 = 0.0;
+    unsigned long long seq = base;
+    while (it < maxCg) {
+      namedSync<1>(kRowThreads);
+      double part[2], sum[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) part[k] = warpSum(lane < kWarps ? sh.red[k][lane] : 0.0);
+      float factor = 0.0f;
+      if (!mailSum<2>(D.mail, D.ctl, D.P.barrierLimitNs, gs.rank, gs.size, ++seq, part, sum, kExchangeDelay)) {
+        code = 2;
+      } else if (it == 0) {
+        r0 = sqrt(sum[0]);
+        code = r0 > 0.0 ? 0 : 1;
+      } else {
+        code = sqrt(sum[0]) <= D.P.cgTolerance * r0 ? 1 : 0;
+        factor = static_cast<float>(sum[1] / rz);
+      }
+      rz = sum[1];
+      if (lane == 0) {
+        sh.code = code;
+        sh.factor = factor;
+      }
+      namedArrive<3>(kRowThreads);
+      if (code) break;
+      namedSync<1>(kRowThreads);
+      double pap[1] = {warpSum(lane < kWarps ? sh.red[0][lane] : 0.0)}, pAp[1];
+      if (sh.failed || !mailSum<1>(D.mail, D.ctl, D.P.barrierLimitNs, gs.rank, gs.size, ++seq, pap, pAp, kExchangeDelay))
+        code = 2;
+      else
+        code = pAp[0] > 0.0 ? 0 : 1;
+      if (lane == 0) {
+        sh.code = code;
+        sh.factor = code ? 0.0f : static_cast<float>(rz / pAp[0]);
+      }
+      namedArrive<3>(kRowThreads);
+      if (code) break;
+      ++it;
+    }
+    if (gs.rank == 0 && lane == 0) *D.mailSeq = seq;  // every block has sent a message, so has read the number
+  } else {
+    uint32_t r0i, r1i;
+    blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
+    const uint32_t i = r0i + threadIdx.x;
+    const bool own = i < r1i, busy = 32u * w < r1i - r0i;  // busy: a row of this warp is owned
+    Contact c{};
+    M3 M{};
+    float3 step = mk(0, 0, 0), resid = mk(0, 0, 0), r = mk(0, 0, 0), z = mk(0, 0, 0);
+    float3 p = mk(0, 0, 0), apFull = mk(0, 0, 0), ap = mk(0, 0, 0);
+    // CG init (kernels.h:252-268): step = 0, resid = -grad, r = filter(resid), z = filter(M r).
+    if (own) {
+      c = D.contact[i];
+      M = loadPrecond(D, i);
+      resid = -ld3(D.grad, i);
+      r = filterRn(c, resid);
+      z = filterRn(c, mulRn(M, r));
+    }
+    if (!busy && lane == 0) sh.red[0][w] = sh.red[1][w] = 0.0;
+    while (it < maxCg) {
+      const uint32_t tag = static_cast<uint32_t>(base + 1 + 2 * static_cast<unsigned long long>(it)) | 0x80000000u;
+      if (own) {
+        storeTagged(D.z + i, z, tag);
+        A.z[threadIdx.x] = f4(z);
+      }
+      if (busy) {
+        const double rr = warpSum(dotd3(r, r)), rz = warpSum(dotd3(r, z));  // zero where no row is owned
+        if (lane == 0) {
+          sh.red[0][w] = rr;
+          sh.red[1][w] = rz;
+        }
+      }
+      namedArrive<1>(kRowThreads);
+      if (!takeHalo(D, A, D.z, tag)) sh.failed = 1;
+      namedSync<2>(kRowWorkers);
+      const float3 az = busy ? residentProduct(A) : mk(0, 0, 0);
+      namedSync<3>(kRowThreads);
+      code = sh.code;
+      if (code) break;
+      // A p = A z + beta A pPrev, p = z + beta pPrev (the direction update folded into the product).
+      const float fb = sh.factor;
+      if (busy) {
+        p = it == 0 ? z : axpyRn(p, fb, z);
+        apFull = it == 0 ? az : axpyRn(apFull, fb, az);
+        ap = filterRn(c, apFull);
+        const double pap = warpSum(dotd3(p, ap));
+        if (lane == 0) sh.red[0][w] = pap;
+      }
+      namedArrive<1>(kRowThreads);
+      namedSync<3>(kRowThreads);
+      code = sh.code;
+      if (code) break;
+      const float fa = sh.factor;
+      ++it;
+      // Update (kernels.h:304-315) fused with the preconditioner apply (kernels.h:324-332).
+      step = axpyRn(p, fa, step);
+      r = axpyRn(ap, -fa, r);
+      resid = axpyRn(apFull, -fa, resid);
+      z = filterRn(c, mulRn(M, r));
+    }
+    if (own) {
+      D.step[i] = f4(step);
+      D.resid[i] = f4(resid);
+    }
+  }
+  __syncthreads();
+  return code == 2 ? -1 : it;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// The learned PCG's resident rows: the matrix in a sliced layout in shared memory (nine planes, then the columns; padding
+// holds kPinnedBit), the vectors' gathers from global memory.
 constexpr int kSlicedDepth = 12;     // gathers a row thread has in flight (even, so k0 + k has the parity of k)
 
 struct SlicedMatrix {
@@ -1682,12 +2031,19 @@ template <bool Learned, int PL, int Variant = 0>
 __device__ inline int pcgSolve(const Dev& D, GridSync& gs) {
   uint32_t r0i, r1i;
   blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
-  if constexpr (Variant == kResidentRows) {
+  if constexpr (Variant == kResidentRows && !Learned) {
+    ResidentMatrix A;
+    if (!stageResident(D, gs.rank, r0i, r1i, A)) return -1;
+    const unsigned long long t0 = globalTimerNs();
+    const int it = pcgResident(D, gs, A);
+    if (gs.rank == 0 && threadIdx.x == 0) D.ctl->pcgNs += static_cast<long long>(globalTimerNs() - t0);
+    return it;
+  } else if constexpr (Variant == kResidentRows) {
     SlicedMatrix A;
     if (!stageSliced(D, r0i, r1i, A)) return -1;
     const unsigned long long t0 = globalTimerNs();
     int it;
-    if constexpr (Learned) {
+    {
       // The learned schedule without block-Jacobi iterations first (the host picks this kernel only then): a learned
       // solve that breaks down is followed by a full block-Jacobi solve, as in pcgSolveStaged.
       it = pcgLearnedResident(D, gs, A);
@@ -1697,8 +2053,6 @@ __device__ inline int pcgSolve(const Dev& D, GridSync& gs) {
         const int jac = pcgResidentRows(D, gs, A);
         it = jac < 0 ? jac : jac + (-2 - it);
       }
-    } else {
-      it = pcgResidentRows(D, gs, A);
     }
     if (gs.rank == 0 && threadIdx.x == 0) D.ctl->pcgNs += static_cast<long long>(globalTimerNs() - t0);
     return it;

@@ -53,9 +53,30 @@ static uint32_t maxBlockSlots(const uint32_t* rowStart, uint32_t n, int grid) {
   return most;
 }
 
-// Padded slots of the sliced layout k_solve_rows stages for its largest block (the rows in warps of 32, each warp's
+// Padded shared-memory slots of k_solve_rows's largest block (the rows in warps of 32, each warp's rows padded to its
+// longest unpinned row, whose first kRegSlots slots sit in registers), or UINT32_MAX when a block has more rows than
+// k_solve_rows has row threads.
+static uint32_t maxResidentSlots(const uint32_t* rowStart, const uint8_t* pinned, uint32_t n, int grid) {
+  const uint32_t per = (n + static_cast<uint32_t>(grid) - 1) / static_cast<uint32_t>(grid);
+  if (per > static_cast<uint32_t>(dcu::kRowWorkers)) return UINT32_MAX;
+  uint32_t most = 0;
+  for (int b = 0; b < grid; ++b) {
+    const uint32_t r0 = std::min<uint32_t>(n, static_cast<uint32_t>(b) * per), r1 = std::min<uint32_t>(n, r0 + per);
+    uint32_t total = 0;
+    for (uint32_t w0 = r0; w0 < r1; w0 += 32) {
+      uint32_t len = 0;
+      for (uint32_t i = w0; i < std::min(r1, w0 + 32); ++i)
+        if (!pinned[i]) len = std::max(len, rowStart[i + 1] - rowStart[i]);
+      total += len > dcu::kRegSlots ? 32 * ((len - dcu::kRegSlots + 1) & ~1u) : 0u;
+    }
+    most = std::max(most, total);
+  }
+  return most;
+}
+
+// Padded slots of the sliced layout k_solve_rows_learned stages for its largest block (the rows in warps of 32, each warp's
 // rows padded to its longest unpinned row; pinned rows take no slots), or UINT32_MAX when a block has more rows than
-// k_solve_rows has threads.
+// it has threads.
 static uint32_t maxSlicedSlots(const uint32_t* rowStart, const uint8_t* pinned, uint32_t n, int grid) {
   const uint32_t per = (n + static_cast<uint32_t>(grid) - 1) / static_cast<uint32_t>(grid);
   if (per > static_cast<uint32_t>(dcu::kRowThreads)) return UINT32_MAX;
@@ -86,7 +107,8 @@ struct drape_solver {
   int failAfter = -1;
   static constexpr int kFrameSlots = 32;  // most frames one advanceFrames call runs before its host wait
   uint32_t solveSmemCap = 0;       // block slots one solve block can keep in shared memory
-  uint32_t rowsSmemCap = 0;        // padded slots one k_solve_rows block can keep in shared memory
+  uint32_t rowsSmemCap = 0;        // padded slots one k_solve_rows_learned block can keep in shared memory
+  size_t residentSmemCap = 0;      // dynamic shared memory a k_solve_rows block can have
   // Learned preconditioner: the solver's own copy of the network and its workspace on this solver's CSR.
   std::unique_ptr<net::Network> net;
   net::GraphHandle netGraph;
@@ -96,7 +118,8 @@ struct drape_solver {
   int pcgVariant = 0;               // block-Jacobi PCG form (drape_cuda_set_pcg_variant)
   uint64_t netNewtonCounter = 0;
   size_t solveSmemBytes = 0;       // dynamic shared memory of the solve launch for the built scene
-  size_t rowsSmemBytes = 0;        // k_solve_rows's, when the built scene fits it (0: it does not)
+  size_t rowsSmemBytes = 0;        // k_solve_rows_learned's, when the built scene fits it (0: it does not)
+  size_t residentSmemBytes = 0;    // k_solve_rows's, likewise
 
   DBuf<dcu::Particle> particle;
   DBuf<dcu::Fabric> fabric;
@@ -111,6 +134,10 @@ struct drape_solver {
   DBuf<float4> stretchDer, hingeDer;
   DBuf<dcu::Contact> contact;
   DBuf<double> partials, statsPartials;
+  DBuf<uint16_t> localCol;  // k_solve_rows: each slot's column among its block's rows and halo
+  DBuf<uint32_t> halo, haloCount;
+  DBuf<dcu::MailWord> mail;
+  DBuf<unsigned long long> mailSeq;
   DBuf<dcu::Control> ctl;
   DBuf<dcu::StatsOut> statsOut;
   DBuf<unsigned int> statsDone;
@@ -201,22 +228,20 @@ struct drape_solver {
       if (perSM < 1) throw std::runtime_error("cuda: the solve kernel does not fit on an SM");
     }
     {
-      const void* rowKernels[] = {reinterpret_cast<const void*>(dcu::k_solve_rows),
-                                  reinterpret_cast<const void*>(dcu::k_solve_rows_learned)};
-      size_t rowsStatic = 0;
-      for (const void* k : rowKernels) {
+      // The most dynamic shared memory each of the two resident-row kernels can have.
+      auto allow = [&](const void* k) {
         cudaFuncAttributes fa{};
         CK(cudaFuncGetAttributes(&fa, k));
-        rowsStatic = std::max(rowsStatic, fa.sharedSizeBytes);
-      }
-      rowsSmemCap = static_cast<uint32_t>((prop.sharedMemPerBlockOptin - rowsStatic) / dcu::kSmemSlotBytes);
-      const int rowsMax = static_cast<int>(rowsSmemCap * dcu::kSmemSlotBytes);
-      for (const void* k : rowKernels) {
-        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, rowsMax));
+        const size_t most = (prop.sharedMemPerBlockOptin - fa.sharedSizeBytes) & ~static_cast<size_t>(15);
+        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)));
         int perSM = 0;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k, dcu::kRowThreads, rowsMax));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, k, dcu::kRowThreads, most));
         if (perSM < 1) throw std::runtime_error("cuda: the resident-row solve kernel does not fit on an SM");
-      }
+        return most;
+      };
+      rowsSmemCap = static_cast<uint32_t>(allow(reinterpret_cast<const void*>(dcu::k_solve_rows_learned)) /
+                                          dcu::kSmemSlotBytes);
+      residentSmemCap = allow(reinterpret_cast<const void*>(dcu::k_solve_rows));
     }
     solveGrid = numSMs;  // one 1024-thread block per SM: fewest barrier arrivals
     pointGrid = numSMs * 8;
@@ -225,6 +250,8 @@ struct drape_solver {
     hStats.alloc(kFrameSlots);
     ctl.alloc(1);
     partials.alloc(2 * static_cast<size_t>(solveGrid) * dcu::kPartialStride);  // two halves, alternating
+    mail.alloc(dcu::mailWords(static_cast<size_t>(solveGrid)));
+    mailSeq.alloc(1);  // the zeroed mailbox carries no number an exchange waits for: the first is 1
     statsPartials.alloc(static_cast<size_t>(statsGrid) * 8);
     statsOut.alloc(kFrameSlots);
     statsDone.alloc(1);
@@ -313,6 +340,7 @@ struct drape_solver {
       d.P.slicedSlots = fits ? std::max<uint32_t>(sliced, 1u) : 0u;
       rowsSmemBytes = fits ? static_cast<size_t>(d.P.slicedSlots) * dcu::kSmemSlotBytes : 0;
     }
+    localize(n, B, d);
     d.fieldValues = fieldValues.p;
     d.particle = particle.p;
     d.fabric = fabric.p;
@@ -354,6 +382,8 @@ struct drape_solver {
     d.precond = precond.p;
     d.contact = contact.p;
     d.partials = partials.p;
+    d.mail = mail.p;
+    d.mailSeq = mailSeq.p;
     d.ctl = ctl.p;
     d.cgLog = cgLog.p;
     dev = d;
@@ -366,6 +396,43 @@ struct drape_solver {
                                                                       static_cast<size_t>(numSMs) * 16)));
     CK(cudaStreamSynchronize(s));
     built = true;
+  }
+
+  // Whether every solve block fits k_solve_rows (its padded slots, its rows and its halo in shared memory), and if so the
+  // columns as indices into a block's rows and halo.
+  void localize(uint32_t n, uint32_t B, dcu::Dev& d) {
+    residentSmemBytes = 0;
+    const uint32_t slots = maxResidentSlots(m.rowStart.data(), m.pinned.data(), n, solveGrid);
+    if (n == 0 || slots == UINT32_MAX) return;
+    const uint32_t words = (n + 31u) / 32u;  // n <= kRowWorkers * solveGrid: at most 18 KB of bitmap and counts
+    const size_t bitmapBytes = 2 * sizeof(uint32_t) * static_cast<size_t>(words);
+    haloCount.alloc(solveGrid);
+    dcu::k_localize<<<solveGrid, 512, bitmapBytes, stream>>>(n, solveGrid, rowStart.p, colIndex.p, words, haloCount.p, 0,
+                                                             nullptr, nullptr);
+    CK(cudaGetLastError());
+    std::vector<uint32_t> counts(solveGrid);
+    CK(cudaMemcpyAsync(counts.data(), haloCount.p, sizeof(uint32_t) * counts.size(), cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
+    const uint32_t per = (n + static_cast<uint32_t>(solveGrid) - 1) / static_cast<uint32_t>(solveGrid);
+    uint32_t most = 0;
+    for (uint32_t c : counts) most = std::max(most, c);
+    const uint32_t nodes = per + most + 1;  // and the zero particle
+    const size_t bytes = (static_cast<size_t>(slots) * dcu::kResidentSlotBytes + 15) / 16 * 16 +
+                         static_cast<size_t>(nodes) * dcu::kResidentNodeBytes;
+    if (nodes >= dcu::kNoColumn || bytes > residentSmemCap) return;
+    const uint32_t stride = std::max<uint32_t>(most, 1u);
+    halo.alloc(static_cast<size_t>(stride) * solveGrid);
+    localCol.alloc(B);
+    dcu::k_localize<<<solveGrid, 512, bitmapBytes, stream>>>(n, solveGrid, rowStart.p, colIndex.p, words, haloCount.p,
+                                                             stride, halo.p, localCol.p);
+    CK(cudaGetLastError());
+    d.P.residentSlots = slots;
+    d.P.residentNodes = nodes;
+    d.P.haloStride = stride;
+    d.halo = halo.p;
+    d.haloCount = haloCount.p;
+    d.localCol = localCol.p;
+    residentSmemBytes = bytes;
   }
 
   // The network's workspace on this solver's CSR; the learned factor and transposed-slot map go into the device view.
@@ -461,13 +528,20 @@ struct drape_solver {
     c.error = 0;
     c.barrierArrivals = 0;
     CK(cudaMemcpy(ctl.p, &c, sizeof(c), cudaMemcpyHostToDevice));
+    // Blocks may have left an abandoned solve after different exchanges: go on with numbers none of them reached (nor
+    // any tag, a number's low bits).
+    unsigned long long seq = 0;
+    CK(cudaMemcpy(&seq, mailSeq.p, sizeof(seq), cudaMemcpyDeviceToHost));
+    seq += 1ull << 24;
+    CK(cudaMemcpy(mailSeq.p, &seq, sizeof(seq), cudaMemcpyHostToDevice));
   }
 
   // The reference-order PCG runs over resident rows (k_solve_rows) where the built scene fits it; bit-identical to
   // k_solve<false, 0>, which variant 3 forces. The learned preconditioner runs over resident rows too
   // (k_solve_rows_learned) unless block-Jacobi iterations come first (precondSwitch) or variant 3 forces k_solve<true>.
   bool usesResidentRows(const dcu::Dev& d) const {
-    return d.P.pcgVariant == 0 && rowsSmemBytes > 0 && (!(learnedOn && netGraph) || precondSwitch == 0);
+    if (d.P.pcgVariant != 0) return false;
+    return learnedOn && netGraph ? rowsSmemBytes > 0 && precondSwitch == 0 : residentSmemBytes > 0;
   }
 
   void launchSolve(const dcu::Dev& d) {
@@ -475,7 +549,7 @@ struct drape_solver {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(solveGrid);
     cfg.blockDim = dim3(rows ? dcu::kRowThreads : dcu::kSolveThreads);
-    cfg.dynamicSmemBytes = rows ? rowsSmemBytes : solveSmemBytes;
+    cfg.dynamicSmemBytes = !rows ? solveSmemBytes : learnedOn && netGraph ? rowsSmemBytes : residentSmemBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;  // co-resident blocks for the grid barrier; capturable in a graph
@@ -1741,6 +1815,16 @@ int drape_cuda_test_barrier_timeout(int device, int blocks, uint64_t nanoseconds
     c.alloc(1);
     out.alloc(1);
     dcu::k_barrier_probe<<<blocks, 32>>>(c.p, nanoseconds, out.p);
+    CK(cudaGetLastError());
+    CK(cudaDeviceSynchronize());
+    CK(cudaMemcpy(status, out.p, sizeof(int), cudaMemcpyDeviceToHost));
+    if (*status != 1) return;
+    // And the exchange of messages, with a control block of its own.
+    DBuf<dcu::Control> c2;
+    DBuf<dcu::MailWord> mail;
+    c2.alloc(1);
+    mail.alloc(dcu::mailWords(static_cast<size_t>(blocks) + 1));
+    dcu::k_mail_probe<<<blocks, 32>>>(c2.p, mail.p, nanoseconds, out.p);
     CK(cudaGetLastError());
     CK(cudaDeviceSynchronize());
     CK(cudaMemcpy(status, out.p, sizeof(int), cudaMemcpyDeviceToHost));

@@ -229,8 +229,8 @@ int drape_cuda_set_host_wait(drape_solver* s, uint32_t spin_microseconds);
 /* The block-Jacobi PCG's form (no reference counterpart; each solves the reference's contact-filtered system with its
    stopping tests, cpu_solver.cpp:169-213): 0 (the default) the reference's order, two grid-wide reductions per
    iteration, run over resident rows (one 512-thread block per SM, each row's PCG state in its thread's registers, the
-   block's matrix in a sliced layout in shared memory) where every block has at most 512 rows and its sliced matrix fits
-   in shared memory, else on one 1024-thread block per SM: the two kernels give bit-identical results; 1 pipelined
+   block's matrix in a sliced layout in shared memory) where every block has at most 480 rows and its sliced matrix, its
+   rows' z and its neighbours' fit in shared memory, else on one 1024-thread block per SM: the two kernels give bit-identical results; 1 pipelined
    (Ghysels and Vanroose 2014), one reduction per iteration and three more work vectors, its FP32 recurrences drifting
    further from the products they stand for; 2 Chronopoulos-Gear, one reduction and one plain barrier per iteration
    with the reference order's recurrences; 3 the reference's order on the 1024-thread kernel whatever the scene (for
@@ -252,8 +252,9 @@ int drape_cuda_set_barrier_limit(drape_solver* s, uint64_t nanoseconds);
    reduction; 3: two plain barriers; 4-7: modes 0-3 on one 512-thread block per SM (the resident-row form's grid). */
 int drape_cuda_reduction_floor(int device, int mode, int iterations, double* ns_per_iteration);
 /* Test hook: runs a grid barrier that can only end by its time limit (it waits for one more block than it has) on
-   `blocks` blocks with the given limit, and returns the status the blocks read back in *status (0: released, which
-   cannot happen; 1: timed out). Exercises the bounded wait without a device fault. */
+   `blocks` blocks with the given limit, then an exchange of messages one of which nobody sends, and returns the status
+   the blocks read back in *status (0: released, which cannot happen; 1: both timed out). Exercises the bounded waits
+   without a device fault. */
 int drape_cuda_test_barrier_timeout(int device, int blocks, uint64_t nanoseconds, int* status);
 /* Test hook: make the next step fail with DRAPE_DEVICE_ERROR after `steps` more successful steps (-1: never), to
    exercise the caller's GPU -> CPU fallback (sim_controller.cpp:155-176) without a device fault. */

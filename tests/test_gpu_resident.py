@@ -1,0 +1,64 @@
+"""The resident-row solve kernel at the edges of its layout: fewer particles than blocks, blocks with no rows, ragged
+warps and rows, pinned rows and columns, halos that span most of the garment, and scenes near its size limit. Its oracle
+is the 1024-thread reference-order kernel (variant 3), whose row products and recurrences it repeats in the same order:
+bit-identical positions and the same PCG counts."""
+import numpy as np
+import pytest
+
+from drape_b200 import scenes as S
+
+pytestmark = pytest.mark.gpu
+
+
+def _hanging(n):
+    g = S.piece_garment("sheet", 0.5, 0.5, n, n, S.jersey_fabric())
+    g.initial_positions = np.stack([g.rest[:, 0], 0.5 + g.rest[:, 1], np.zeros(g.vertex_count)], axis=1)
+    scene = S.Scene([g])
+    for v in list(range(0, n * n, max(1, n // 3))):  # pins in every block, corners and interior
+        scene.pins.append((v, tuple(g.initial_positions[v])))
+    return scene
+
+
+def _shuffled(n, seed):
+    """A sheet whose vertices are numbered at random: every block's halo holds most of the garment."""
+    sc = S.sheet_on_sphere(n=n, height=0.16, cg_tolerance=1e-2, max_cg=50)
+    g = sc.garments[0]
+    perm = np.random.default_rng(seed).permutation(g.vertex_count)
+    inv = np.argsort(perm).astype(np.uint32)
+    sc.garments[0] = S.Garment(g.id, g.rest[perm], g.vertex_piece[perm], g.vertex_area[perm],
+                               inv[g.triangles.astype(np.int64)], g.triangle_piece, g.piece_grain, g.piece_fabric,
+                               g.seam_pairs, g.initial_positions[perm], g.boundary[perm])
+    return sc
+
+
+CASES = {
+    "sheet_4x4": lambda: S.sheet_on_sphere(n=4, height=0.16, cg_tolerance=1e-2, max_cg=50),
+    "sheet_12x12": lambda: S.sheet_on_sphere(n=12, height=0.16, cg_tolerance=1e-2, max_cg=50),
+    "sheet_13x13": lambda: S.sheet_on_sphere(n=13, height=0.16, cg_tolerance=1e-2, max_cg=50),
+    "sheet_70x70": lambda: S.sheet_on_sphere(n=70, height=0.16, cg_tolerance=1e-6, max_cg=200),
+    "pinned_37x37": lambda: _hanging(37),
+    "shuffled_60x60": lambda: _shuffled(60, 3),
+    "tube_66k": lambda: S.seamed_tube(161, 205, field_n=64, field_cell=0.012),
+}
+
+
+def _run(gpu, scene, variant, frames=3):
+    s = gpu.CudaSolver(0)
+    s.set_pcg_variant(variant)
+    s.build(scene)
+    threads = s.solve_threads()
+    for _ in range(frames):
+        s.step(1.0 / 60.0, 1, 2)
+    out = s.positions(), s.velocities(), s.cg_history(), threads
+    s.close()
+    return out
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_resident_rows_match_the_1024_thread_kernel(gpu, name):
+    x3, v3, h3, t3 = _run(gpu, CASES[name](), 3)
+    x0, v0, h0, t0 = _run(gpu, CASES[name](), 0)
+    assert (t3, t0) == (1024, 512)
+    assert np.isfinite(x0).all()
+    assert np.array_equal(h0, h3), (h0, h3)
+    assert np.array_equal(x0, x3) and np.array_equal(v0, v3), np.abs(x0 - x3).max()
