@@ -5,13 +5,16 @@
 //
 // What bounds it is the way to the L2 and back (measured on a B200: 0.29 us from a store to the poll that sees it within
 // a die, 0.5 us across the dies) and the polls themselves: a poll of a word that has not been written yet takes the line
-// into the reader's die, and the write then has to fetch it back. Each block therefore writes its message to
-// kMailReplicas copies, each read by a quarter of the blocks, each message has 64 bytes to itself, and a block may let
-// `delay` clock cycles pass between its message and its first poll, by when the others' words are there if they all sent
-// at about the same time. One sum over 148 blocks of 512 threads, block sums included: 1.3 us (0.97-1.2 us with a delay
-// of 400-800 cycles in lockstep), against 2.09 us for a counter barrier followed by a read of every block's partial sum
-// and 3.1-4.3 us for one copy without a delay; 2 or 8 copies 1.32-1.42 us, 32-byte slots 1.36-1.50 us; a two-level tree
-// of blocks 1.6-1.8 us.
+// into the reader's die, and the write then has to fetch it back. So a block lets some clock cycles pass between its
+// message and its first poll, by when the others' words are usually there, and adapts them: a little less after each
+// exchange whose first poll saw everything, more after one that did not. The words of one value lie side by side (a
+// warp's poll reads 512 contiguous bytes), all loads are issued before any tag is looked at, and one copy of the messages
+// serves all readers. One sum over 148 blocks of 512 threads, block sums included, in lockstep: 0.97-1.1 us, against
+// 2.09 us for a counter barrier followed by a read of every block's partial sum; polling at once 1.3-4.3 us depending on
+// the copies and their spacing. In the PCG (us per iteration at 1,600, 10k and 60k particles): adapted 2.82, 2.85, 4.25;
+// a fixed delay of 500 cycles 2.72, 2.92, 5.40, of 700 2.86, 2.86, 4.74, of 900 3.02, 2.85, 4.41; adapted with two copies
+// 3.06, 3.05, 4.21; four copies 64 bytes apart at 700 cycles 2.9-3.4, 3.0-3.4, 4.3. A two-level tree of blocks takes
+// 1.6-1.8 us a sum.
 #pragma once
 
 #include <cstdint>
@@ -23,11 +26,12 @@ struct __align__(16) MailWord {
   unsigned long long tag;
 };
 
-constexpr uint32_t kMailReplicas = 4;  // copies of each message
-constexpr uint32_t kMailWords = 4;     // words of a message's slot (64 bytes): up to this many values a message
+constexpr uint32_t kMailWords = 2;  // a message is up to this many values
+// The wait before an exchange's first poll, in clock cycles: its steps down and up, and its range.
+constexpr int kDelayDown = 8, kDelayUp = 128, kDelayLeast = 300, kDelayMost = 4000;
 // Words of the mailbox of `blocks` blocks: two halves, used by turns (a block sends message k + 2 only after it has
 // message k + 1 of every block, and hence after every block has read its message k).
-__host__ __device__ constexpr size_t mailWords(size_t blocks) { return 2 * static_cast<size_t>(kMailReplicas) * blocks * kMailWords; }
+__host__ __device__ constexpr size_t mailWords(size_t blocks) { return 2 * blocks * kMailWords; }
 
 // 16-byte loads and stores that are one access each.
 __device__ __forceinline__ void storeWord(MailWord* p, double value, unsigned long long tag) {
@@ -94,59 +98,54 @@ struct BoundedWait {
 
 // One exchange, run by one whole warp of every block: `mine` (the same in all lanes) is added over the `size` blocks in
 // a fixed order, and every lane of every block gets the same totals. `seq` is the exchange's number, one more than the
-// last one's. `delay`: clock cycles before the first poll. Returns false when the wait gave up.
+// last one's. `delay`: clock cycles before the first poll, adapted. Returns false when the wait gave up.
 template <int K>
 __device__ inline bool mailSum(MailWord* box, Control* ctl, unsigned long long limitNs, uint32_t rank, uint32_t size,
-                               unsigned long long seq, const double (&mine)[K], double (&total)[K], int delay = 0) {
-  static_assert(K >= 1 && K <= static_cast<int>(kMailWords), "mailSum: a message is one slot");
-  constexpr int kLoads = 5;  // slots a lane waits for at a time (160 blocks a round: one round for one block per SM)
+                               unsigned long long seq, const double (&mine)[K], double (&total)[K], int& delay) {
+  static_assert(K >= 1 && K <= static_cast<int>(kMailWords), "mailSum: a message is at most kMailWords values");
+  constexpr int kLoads = 5;  // words a lane waits for at a time (160 blocks a round: one round for one block per SM)
   const uint32_t lane = threadIdx.x & 31u;
   MailWord* half = box + (seq & 1ull) * (mailWords(size) / 2);
-  if (lane < kMailReplicas)
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-      storeWord(half + (static_cast<size_t>(lane) * size + rank) * kMailWords + k, mine[k], seq);
-  const MailWord* copy = half + static_cast<size_t>(rank % kMailReplicas) * size * kMailWords;
   double t[K];
 #pragma unroll
   for (int k = 0; k < K; ++k) t[k] = 0.0;
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    if (lane == 0) storeWord(half + static_cast<size_t>(k) * size + rank, mine[k], seq);
   BoundedWait wait;
   for (const long long start = clock64(); clock64() - start < delay;) {
   }
+  bool first = true;
   for (uint32_t b0 = 0; b0 < size; b0 += 32 * kLoads) {
     double x[kLoads][K];
-    bool have[kLoads];
-#pragma unroll
-    for (int j = 0; j < kLoads; ++j) {
-      have[j] = b0 + 32 * j + lane >= size;
-#pragma unroll
-      for (int k = 0; k < K; ++k) x[j][k] = 0.0;
-    }
     for (;;) {
+      // All loads first (lanes past the end repeat the last block's word), then the tags.
       unsigned long long tag[kLoads][K];
 #pragma unroll
-      for (int j = 0; j < kLoads; ++j)
-        if (!have[j])
+      for (int k = 0; k < K; ++k)
 #pragma unroll
-          for (int k = 0; k < K; ++k) loadWord(copy + static_cast<size_t>(b0 + 32 * j + lane) * kMailWords + k, x[j][k], tag[j][k]);
-      bool all = true;
+        for (int j = 0; j < kLoads; ++j)
+          loadWord(half + static_cast<size_t>(k) * size + min(b0 + 32 * j + lane, size - 1), x[j][k], tag[j][k]);
+      unsigned long long differ = 0;
 #pragma unroll
-      for (int j = 0; j < kLoads; ++j)
-        if (!have[j]) {
-          bool h = true;
+      for (int k = 0; k < K; ++k)
 #pragma unroll
-          for (int k = 0; k < K; ++k) h = h && tag[j][k] == seq;
-          have[j] = h;
-          all = all && h;
-        }
-      if (__all_sync(0xffffffffu, all)) break;
+        for (int j = 0; j < kLoads; ++j) differ |= tag[j][k] ^ seq;
+      if (__all_sync(0xffffffffu, differ == 0)) break;
+      first = false;
       if (__any_sync(0xffffffffu, wait.expired(ctl, limitNs))) return false;
     }
 #pragma unroll
-    for (int k = 0; k < K; ++k) t[k] += ((x[0][k] + x[1][k]) + (x[2][k] + x[3][k])) + x[4][k];
+    for (int k = 0; k < K; ++k) {
+#pragma unroll
+      for (int j = 0; j < kLoads; ++j)
+        if (b0 + 32 * j + lane >= size) x[j][k] = 0.0;
+      t[k] += ((x[0][k] + x[1][k]) + (x[2][k] + x[3][k])) + x[4][k];
+    }
   }
 #pragma unroll
   for (int k = 0; k < K; ++k) total[k] = warpSum(t[k]);
+  delay = first ? max(delay - kDelayDown, kDelayLeast) : min(delay + kDelayUp, kDelayMost);
   return true;
 }
 

@@ -101,8 +101,8 @@ struct Params {
   int pcgVariant;       // the block-Jacobi PCG form: 0 reference order (resident rows where the scene fits), 1 pipelined,
                         // 2 Chronopoulos-Gear, 3 reference order on the 1024-thread kernel (kept in the view so that
                         // captured frame graphs are recaptured when it changes)
-  uint32_t slicedSlots; // k_solve_rows_learned: padded slots of the sliced layout a block may hold in shared memory
   uint32_t residentSlots, residentNodes;  // k_solve_rows: a block's padded slots and its rows and halo, in shared memory
+  uint32_t factorSlots; // k_solve_rows_learned: a block's padded factor slots
   uint32_t haloStride;  // entries of `halo` per solve block
   unsigned long long barrierLimitNs;
 };
@@ -133,6 +133,7 @@ struct Dev {
   const float* Lf;         // learned factor L: 9 planes of slotsPadded floats on lower slots (k_solve<true>)
   const uint32_t* tslot;   // slot of (j, i) for slot (i, j)
   const float4* LfRows;    // the factor by rows, three float4 a slot: L_ij at lower slots, L_ji at upper (i, j)
+  float4* LfSliced;        // k_solve_rows_learned: 3 * factorSlots per block where the factor does not fit shared memory
   const float4* fExt;
   const float4* pinPos;
   float* blocks;   // 9 planes of slotsPadded floats, component 3*row+col
@@ -1033,12 +1034,12 @@ __device__ inline int pcgReferenceOrder(const Dev& D, GridSync& gs, const SmemMa
 // shared memory a slot and 16 a gathered z, against 128 bytes a clock: 1.3 us), then one exchange. Fewer blocks than SMs
 // for small scenes: 2.7-2.9 us for 8 to 148 blocks at 1,600 particles, slower at 4,000 and 10k. A row's slots four at a
 // time with two slots in registers: 4.31 us at 60k; two at a time 4.39, six 4.43; four or six slots in registers spill
-// (4.30-4.32). Exchange delays of 500-900 cycles are within 3 % of each other; none costs 8-15 % on small scenes.
+// (4.30-4.32).
 constexpr int kRowThreads = 512;    // k_solve_rows block size
 constexpr int kRowWorkers = 480;    // of these, the threads that own a row each; the last warp does the exchanges
 constexpr int kResidentRows = 4;    // the solve templates' Variant value of this form
 constexpr int kRegSlots = 2;        // slots of each row kept in registers (even, so that slot parity is the same)
-constexpr int kExchangeDelay = 700; // clock cycles before an exchange's first poll
+constexpr int kExchangeDelay = 700; // clock cycles before an exchange's first poll, to begin with
 constexpr uint32_t kNoColumn = 0xFFFFu;  // localCol of a pinned column
 
 // Shared memory of one padded slot (nine floats and a 16-bit column) and of one particle's z.
@@ -1052,6 +1053,8 @@ struct ResidentMatrix {
   uint32_t base, len;      // this thread's warp: its first position and its padded slots (even)
   uint32_t rows, haloSize;
   const uint32_t* halo;    // the halo's particles
+  const float4* factor;    // the learned factor's slots (row 0; rows 1 and 2 follow): in shared memory or D.LfSliced
+  uint32_t factorBase;     // this thread's warp's first position there
   float reg[kRegSlots][9];
   uint32_t regCols[kRegSlots / 2];
 };
@@ -1062,11 +1065,15 @@ struct ResidentShared {
   float factor;  // beta, or alpha
   int code;      // 0 go on, 1 stop, 2 an exchange gave up
   int failed;    // a halo wait gave up
+  unsigned long long seq;  // the last exchange's number
 };
 
 // Copies this block's rows [r0, r1) into registers and the sliced layout (all threads; ends with a block barrier).
 // Returns false, after raising error 4, when the block does not fit what the host sized (P.residentSlots,
 // P.residentNodes; the host picks k_solve_rows only for scenes whose every block fits, so this is a guard).
+// Learned: also a second array for gathered vectors, and the factor by rows in the sliced layout: in shared memory, or
+// where it does not fit in the block's part of D.LfSliced (so that a warp's loads of it are contiguous).
+template <bool Learned>
 __device__ inline bool stageResident(const Dev& D, uint32_t rank, uint32_t r0, uint32_t r1, ResidentMatrix& A) {
   constexpr int kWarps = kRowWorkers / 32;
   // The rows' first slots relative to the block's first, bit 31 set for pinned rows (they take no product).
@@ -1111,7 +1118,16 @@ __device__ inline bool stageResident(const Dev& D, uint32_t rank, uint32_t r0, u
   float4* a = solveSmem;
   float4* b = a + cap;
   A.z = b + cap;
-  float* c = reinterpret_cast<float*>(A.z + D.P.residentNodes);
+  float4* behindZ = A.z + (Learned ? 2 : 1) * D.P.residentNodes;
+  const uint32_t factorCap = Learned ? D.P.factorSlots : 0u;
+  float4* factor = Learned && D.LfSliced ? D.LfSliced + 3 * static_cast<size_t>(factorCap) * rank : behindZ;
+  A.factor = factor;
+  A.factorBase = w < kWarps ? warpBase[w] + 32u * kRegSlots * w : 0u;  // every slot has a place here
+  if (Learned && total + 32u * kRegSlots * kWarps > factorCap) {
+    if (t == 0) atomicExch(&D.ctl->error, 4);
+    return false;
+  }
+  float* c = reinterpret_cast<float*>(Learned && !D.LfSliced ? behindZ + 3 * factorCap : behindZ);
   uint16_t* cols = reinterpret_cast<uint16_t*>(c + cap);
   A.a = a;
   A.b = b;
@@ -1120,7 +1136,7 @@ __device__ inline bool stageResident(const Dev& D, uint32_t rank, uint32_t r0, u
   A.base = w < kWarps ? warpBase[w] : 0u;
   A.len = w < kWarps ? warpLen[w] : 0u;
   const uint32_t SP = D.P.slotsPadded, zeroNode = D.P.residentNodes - 1;
-  if (t == 0) A.z[zeroNode] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (t < (Learned ? 2u : 1u)) A.z[zeroNode + t * D.P.residentNodes] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   // The row's first slots, and the padding of its lane.
   uint32_t rc[kRegSlots];
 #pragma unroll
@@ -1150,6 +1166,13 @@ __device__ inline bool stageResident(const Dev& D, uint32_t rank, uint32_t r0, u
     }
     if (off[lo] & kPinnedBit) continue;  // a pinned row's slot
     const uint32_t j = k - off[lo];
+    if (Learned) {
+      const float4* row = D.LfRows + 3 * static_cast<size_t>(first + k);
+      float4* f = factor + warpBase[lo >> 5] + 32u * kRegSlots * (lo >> 5) + 32u * j + (lo & 31u);
+      f[0] = __ldg(row);
+      f[factorCap] = __ldg(row + 1);
+      f[2 * factorCap] = __ldg(row + 2);
+    }
     if (j < kRegSlots) continue;
     const uint32_t pos = warpBase[lo >> 5] + 32u * (j - kRegSlots) + (lo & 31u);
     const uint32_t s = first + k;
@@ -1168,7 +1191,7 @@ __device__ inline bool stageResident(const Dev& D, uint32_t rank, uint32_t r0, u
 
 // U of this thread's slots (U even) from slot k on: all their loads are issued before the first product.
 template <int U>
-__device__ __forceinline__ void residentSlots(const ResidentMatrix& A, uint32_t k, float3 (&acc)[2]) {
+__device__ __forceinline__ void residentSlots(const ResidentMatrix& A, const float4* z, uint32_t k, float3 (&acc)[2]) {
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t cc[U / 2];
   float4 a[U], b[U], x[U];
@@ -1183,7 +1206,7 @@ __device__ __forceinline__ void residentSlots(const ResidentMatrix& A, uint32_t 
     c[u] = A.c[pos];
   }
 #pragma unroll
-  for (int u = 0; u < U; ++u) x[u] = A.z[(u & 1) ? cc[u / 2] >> 16 : cc[u / 2] & 0xFFFFu];
+  for (int u = 0; u < U; ++u) x[u] = z[(u & 1) ? cc[u / 2] >> 16 : cc[u / 2] & 0xFFFFu];
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const float m[9] = {a[u].x, a[u].y, a[u].z, a[u].w, b[u].x, b[u].y, b[u].z, b[u].w, c[u]};
@@ -1194,24 +1217,25 @@ __device__ __forceinline__ void residentSlots(const ResidentMatrix& A, uint32_t 
 // y_i (unfiltered) = sum over the row's unpinned columns j of A_ij z_j, for this thread's row, in pcgReferenceOrder<2>'s
 // order: slot k of the row into sum k mod 2, each sum in slot order, the odd sum added to the even one last. Pinned
 // columns and padding hold zero blocks and name the zero particle: they add +0 to a sum that is never -0.
-__device__ __forceinline__ float3 residentProduct(const ResidentMatrix& A) {
+__device__ __forceinline__ float3 residentProduct(const ResidentMatrix& A, const float4* z) {
   float3 acc[2] = {mk(0, 0, 0), mk(0, 0, 0)};
   {
     float4 x[kRegSlots];
 #pragma unroll
-    for (int k = 0; k < kRegSlots; ++k) x[k] = A.z[(k & 1) ? A.regCols[k / 2] >> 16 : A.regCols[k / 2] & 0xFFFFu];
+    for (int k = 0; k < kRegSlots; ++k) x[k] = z[(k & 1) ? A.regCols[k / 2] >> 16 : A.regCols[k / 2] & 0xFFFFu];
 #pragma unroll
     for (int k = 0; k < kRegSlots; ++k) blockMulAddRn(acc[k & 1], A.reg[k], xyz(x[k]));
   }
   uint32_t k = 0;
-  for (; k + 4 <= A.len; k += 4) residentSlots<4>(A, k, acc);
-  if (k < A.len) residentSlots<2>(A, k, acc);
+  for (; k + 4 <= A.len; k += 4) residentSlots<4>(A, z, k, acc);
+  if (k < A.len) residentSlots<2>(A, z, k, acc);
   return mk(__fadd_rn(acc[0].x, acc[1].x), __fadd_rn(acc[0].y, acc[1].y), __fadd_rn(acc[0].z, acc[1].z));
 }
 
-// This iteration's z of the halo into shared memory, each particle's as soon as it carries `tag`. Returns false when a
-// wait gave up.
-__device__ __forceinline__ bool takeHalo(const Dev& D, const ResidentMatrix& A, const float4* global, uint32_t tag) {
+// The halo's entries of `global` into shared memory (behind the block's own in `z`), each particle's as soon as it carries
+// `tag`. Returns false when a wait gave up.
+__device__ __forceinline__ bool takeHalo(const Dev& D, const ResidentMatrix& A, float4* z, const float4* global,
+                                         uint32_t tag) {
   constexpr uint32_t kStep = kRowWorkers;
   bool ok = true;
   BoundedWait wait;
@@ -1228,38 +1252,40 @@ __device__ __forceinline__ bool takeHalo(const Dev& D, const ResidentMatrix& A, 
         break;
       }
     }
-    A.z[A.rows + h] = f4(v0);
-    if (two) A.z[A.rows + h + kStep] = f4(v1);
+    z[A.rows + h] = f4(v0);
+    if (two) z[A.rows + h + kStep] = f4(v1);
   }
   return ok;
 }
 
 // The reference-order PCG of pcgReferenceOrder (same recurrences, same stopping tests) over resident rows. Writes
-// step and resid of the block's rows; returns the iteration count, or -1 when an exchange gave up.
+// step and resid of the block's rows; returns the iteration count, or -1 when an exchange gave up. `seq` is the last
+// exchange's number, advanced by the exchanges done.
 //
 // Barriers: 1 hands the row warps' sums to the exchange warp (they only arrive), 3 its scalars to the row warps (it only
 // arrives), 2 is the row warps' own, between the z in shared memory and the product. The exchange warp evaluates every
 // stopping test, so all warps leave after the same exchange; a row warp whose halo wait gave up says so through `failed`
 // and leaves like the others.
-__device__ inline int pcgResident(const Dev& D, GridSync& gs, ResidentMatrix& A) {
+__device__ inline int pcgResident(const Dev& D, GridSync& gs, ResidentMatrix& A, unsigned long long& seq) {
   constexpr int kWarps = kRowWorkers / 32;
   __shared__ ResidentShared sh;
   const int maxCg = D.P.maxCg;
   const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
-  const unsigned long long base = __ldcg(D.mailSeq);
+  const unsigned long long base = seq;
   if (threadIdx.x == 0) sh.failed = 0;
   __syncthreads();
   int it = 0, code = 0;
   if (w == kWarps) {  // the exchange warp
     double rz = 0.0, r0 = 0.0;
-    unsigned long long seq = base;
+    unsigned long long num = base;
+    int delayA = kExchangeDelay, delayB = kExchangeDelay;
     while (it < maxCg) {
       namedSync<1>(kRowThreads);
       double part[2], sum[2];
 #pragma unroll
       for (int k = 0; k < 2; ++k) part[k] = warpSum(lane < kWarps ? sh.red[k][lane] : 0.0);
       float factor = 0.0f;
-      if (!mailSum<2>(D.mail, D.ctl, D.P.barrierLimitNs, gs.rank, gs.size, ++seq, part, sum, kExchangeDelay)) {
+      if (!mailSum<2>(D.mail, D.ctl, D.P.barrierLimitNs, gs.rank, gs.size, ++num, part, sum, delayB)) {
         code = 2;
       } else if (it == 0) {
         r0 = sqrt(sum[0]);
@@ -1277,7 +1303,7 @@ __device__ inline int pcgResident(const Dev& D, GridSync& gs, ResidentMatrix& A)
       if (code) break;
       namedSync<1>(kRowThreads);
       double pap[1] = {warpSum(lane < kWarps ? sh.red[0][lane] : 0.0)}, pAp[1];
-      if (sh.failed || !mailSum<1>(D.mail, D.ctl, D.P.barrierLimitNs, gs.rank, gs.size, ++seq, pap, pAp, kExchangeDelay))
+      if (sh.failed || !mailSum<1>(D.mail, D.ctl, D.P.barrierLimitNs, gs.rank, gs.size, ++num, pap, pAp, delayA))
         code = 2;
       else
         code = pAp[0] > 0.0 ? 0 : 1;
@@ -1289,7 +1315,7 @@ __device__ inline int pcgResident(const Dev& D, GridSync& gs, ResidentMatrix& A)
       if (code) break;
       ++it;
     }
-    if (gs.rank == 0 && lane == 0) *D.mailSeq = seq;  // every block has sent a message, so has read the number
+    if (lane == 0) sh.seq = num;
   } else {
     uint32_t r0i, r1i;
     blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
@@ -1322,9 +1348,9 @@ __device__ inline int pcgResident(const Dev& D, GridSync& gs, ResidentMatrix& A)
         }
       }
       namedArrive<1>(kRowThreads);
-      if (!takeHalo(D, A, D.z, tag)) sh.failed = 1;
+      if (!takeHalo(D, A, A.z, D.z, tag)) sh.failed = 1;
       namedSync<2>(kRowWorkers);
-      const float3 az = busy ? residentProduct(A) : mk(0, 0, 0);
+      const float3 az = busy ? residentProduct(A, A.z) : mk(0, 0, 0);
       namedSync<3>(kRowThreads);
       code = sh.code;
       if (code) break;
@@ -1355,351 +1381,264 @@ __device__ inline int pcgResident(const Dev& D, GridSync& gs, ResidentMatrix& A)
     }
   }
   __syncthreads();
+  seq = sh.seq;
+  __syncthreads();
   return code == 2 ? -1 : it;
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// The learned PCG's resident rows: the matrix in a sliced layout in shared memory (nine planes, then the columns; padding
-// holds kPinnedBit), the vectors' gathers from global memory.
-constexpr int kSlicedDepth = 12;     // gathers a row thread has in flight (even, so k0 + k has the parity of k)
+// The learned PCG over resident rows (k_solve_rows_learned): pcgLearned's recurrences, stopping tests and breakdown rules
+// with the matrix, the rows and the exchanges of pcgResident, and the factor by rows in the sliced layout (three float4 a
+// slot): in shared memory where a block has the room (up to about 28k particles), else in the L2.
+//
+// An iteration is three products, A z, y = L^T r and z = L y, each of which needs its operand from the neighbours, and
+// three sums. The operands are published with tags and taken as they come; r.r travels during the two factor products
+// and r.z during A z, so only p.Ap is waited for. Two arrays in shared memory hold the operands by turns: an operand is
+// written only after the barrier that follows every read of the array's last one.
+//
+// Measured (us per PCG iteration, one B200, against four counter barriers an iteration and the operands gathered from the
+// L2): 10k particles 7.0 (was 13.7), 60k 12.7 (25.1). What bounds it: at 10k the way of r, y and z to the neighbours, one
+// after the other, and the exchange of p.Ap (about 4 us); at 60k also the factor's 42 MB from the L2. At 60k the factor
+// read by rows (each lane its own row) took 18.7-19.7, since every 16-byte load was its own L2 sector; 2, 3 or 4 slots in
+// flight 13.2, 12.7 and 14.0 (four spill).
+constexpr int kLearnedDepth = 3;  // slots whose factor blocks a row thread has in flight
 
-struct SlicedMatrix {
-  const float* planes;   // 9 planes of `stride` floats
-  const uint32_t* cols;  // `stride` column indices (bit 31: pinned column or padding)
-  uint32_t stride;       // padded slots of the block
-  uint32_t base, len;    // this thread's warp: its first position and its padded row length
-};
-
-// Copies this block's rows [r0, r1) into the sliced layout (all threads; ends with a block barrier). Returns false,
-// after raising error 4, when the padded slots exceed P.slicedSlots (the host picks k_solve_rows only for scenes whose
-// every block fits, so this is a guard).
-__device__ inline bool stageSliced(const Dev& D, uint32_t r0, uint32_t r1, SlicedMatrix& A) {
-  constexpr int kWarps = kRowThreads / 32;
-  // The rows' first slots relative to the block's first, bit 31 set for pinned rows (they take no product).
-  __shared__ uint32_t off[kRowThreads + 1];
-  __shared__ uint32_t warpLen[kWarps], warpBase[kWarps + 1];
-  const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5;
-  const uint32_t R = r1 - r0;
-  if (R > static_cast<uint32_t>(kRowThreads) || blockDim.x != static_cast<unsigned>(kRowThreads)) {
-    if (t == 0) atomicExch(&D.ctl->error, 4);
-    return false;
-  }
-  const uint32_t first = __ldg(D.rowStart + r0);  // r0 <= n: rowStart has n + 1 entries
-  uint32_t c = 0;
-  if (t < R) {
-    const uint32_t rs = __ldg(D.rowStart + r0 + t);
-    const bool pinned = D.particle[r0 + t].pinned != 0u;
-    off[t] = (rs - first) | (pinned ? kPinnedBit : 0u);
-    if (!pinned) c = __ldg(D.rowStart + r0 + t + 1) - rs;
-  }
-  if (t == 0) off[R] = __ldg(D.rowStart + r1) - first;
-  const uint32_t len = __reduce_max_sync(0xffffffffu, c);
-  if (lane == 0) warpLen[w] = len;
-  __syncthreads();
-  if (t == 0) {
-    uint32_t acc = 0;
-    for (int k = 0; k < kWarps; ++k) {
-      warpBase[k] = acc;
-      acc += 32u * warpLen[k];
-    }
-    warpBase[kWarps] = acc;
-  }
-  __syncthreads();
-  const uint32_t total = warpBase[kWarps];
-  if (total > D.P.slicedSlots) {
-    if (t == 0) atomicExch(&D.ctl->error, 4);
-    return false;
-  }
-  float* planes = reinterpret_cast<float*>(solveSmem);
-  uint32_t* cols = reinterpret_cast<uint32_t*>(planes + 9 * total);
-  A.planes = planes;
-  A.cols = cols;
-  A.stride = total;
-  A.base = warpBase[w];
-  A.len = warpLen[w];
-  // Padding of this thread's row: positions [c, len) of its lane.
-  for (uint32_t k = c; k < len; ++k) cols[A.base + 32u * k + lane] = kPinnedBit;
-  // The slots, read in slot order (coalesced); each finds its row by bisection over off[].
-  const uint32_t S = off[R];
-  const uint32_t SP = D.P.slotsPadded;
-  for (uint32_t k = t; k < S; k += blockDim.x) {
-    uint32_t lo = 0, hi = R;  // row lo's first slot <= k < row hi's first slot
-    while (hi - lo > 1) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if ((off[mid] & ~kPinnedBit) <= k) lo = mid; else hi = mid;
-    }
-    if (off[lo] & kPinnedBit) continue;  // a pinned row's slot
-    const uint32_t j = k - off[lo];
-    const uint32_t pos = warpBase[lo >> 5] + 32u * j + (lo & 31u);
-    const uint32_t s = first + k;
-#pragma unroll
-    for (int q = 0; q < 9; ++q) planes[q * total + pos] = __ldg(D.blocks + q * SP + s);
-    cols[pos] = __ldg(D.colIndex + s);
-  }
-  __syncthreads();
-  return true;
+// acc += B x (Upper: B^T x) for this thread's row over its slots [k0, k1) (slot k is global slot rs + k; the columns are
+// sorted, so the lower part j <= i is [0, kd] and the upper part j >= i is [kd, end) with kd the diagonal's position).
+// The learned PCG's dot product and contact filter, with every rounding written out, so that its iterates do not depend
+// on how the compiler contracts the code around them (the first two products' sum fused into the first).
+__device__ __forceinline__ float dotYRn(float a0, float a1, float a2, float3 b) {
+  return __fmaf_rn(a2, b.z, __fmaf_rn(a0, b.x, __fmul_rn(a1, b.y)));
+}
+__device__ __forceinline__ float3 filterYRn(const Contact& c, float3 v) {
+  if (c.active == 0u) return v;
+  const float3 n = xyz(c.normal);
+  return axpyRn(n, -dotYRn(n.x, n.y, n.z, v), v);
 }
 
-// y_i (unfiltered) = sum over the row's unpinned columns j of A_ij x_j, for this thread's row, in pcgReferenceOrder<2>'s
-// order: slot k of the row into sum k mod 2, each sum in slot order, the odd sum added to the even one last.
-__device__ __forceinline__ float3 slicedProduct(const SlicedMatrix& A, const float4* x) {
-  float3 acc0 = mk(0, 0, 0), acc1 = mk(0, 0, 0);
-  const uint32_t lane = threadIdx.x & 31u;
-  for (uint32_t k0 = 0; k0 < A.len; k0 += kSlicedDepth) {
-    uint32_t col[kSlicedDepth];
-#pragma unroll
-    for (int k = 0; k < kSlicedDepth; ++k)
-      col[k] = k0 + k < A.len ? A.cols[A.base + 32u * (k0 + k) + lane] : kPinnedBit;
-    float3 v[kSlicedDepth];
-#pragma unroll
-    for (int k = 0; k < kSlicedDepth; ++k) v[k] = (col[k] & kPinnedBit) ? mk(0, 0, 0) : ld3(x, col[k]);
-#pragma unroll
-    for (int k = 0; k < kSlicedDepth; ++k) {
-      if (col[k] & kPinnedBit) continue;
-      const uint32_t pos = A.base + 32u * (k0 + k) + lane;
-      float a[9];
-#pragma unroll
-      for (int q = 0; q < 9; ++q) a[q] = A.planes[q * A.stride + pos];
-      blockMulAddRn((k & 1) ? acc1 : acc0, a, v[k]);
-    }
-  }
-  return mk(__fadd_rn(acc0.x, acc1.x), __fadd_rn(acc0.y, acc1.y), __fadd_rn(acc0.z, acc1.z));
-}
-
-// The reference-order PCG of pcgReferenceOrder (same recurrences, same stopping tests) over resident rows. Writes
-// step, resid, r and z of the block's rows; returns the iteration count, or -1 when a grid barrier gave up.
-__device__ inline int pcgResidentRows(const Dev& D, GridSync& gs, const SlicedMatrix& A) {
-  uint32_t r0i, r1i;
-  blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
-  const uint32_t i = r0i + threadIdx.x;
-  const bool own = i < r1i;
-  Contact c{};
-  M3 M{};
-  float3 step = mk(0, 0, 0), resid = mk(0, 0, 0), r = mk(0, 0, 0), z = mk(0, 0, 0);
-  float3 p = mk(0, 0, 0), apFull = mk(0, 0, 0), ap = mk(0, 0, 0);
-  // CG init (kernels.h:252-268): step = 0, resid = -grad, r = filter(resid), z = filter(M r).
-  double tot[2];
-  {
-    double v[2] = {0.0, 0.0};
-    if (own) {
-      c = D.contact[i];
-      M = loadPrecond(D, i);
-      resid = -ld3(D.grad, i);
-      r = filterRn(c, resid);
-      z = filterRn(c, mulRn(M, r));
-      D.z[i] = f4(z);
-      v[0] += dotd3(r, z);
-      v[1] += dotd3(r, r);
-    }
-    if (!gridReduce<2>(D, gs, v, tot)) return -1;
-  }
-  double rz = tot[0];
-  const double r0 = sqrt(tot[1]);
-  double beta = 0.0;
-  int it = 0;
-  const int maxCg = D.P.maxCg;
-  if (r0 > 0.0) {
-    while (it < maxCg) {
-      // A p = A z + beta A pPrev, p = z + beta pPrev (the direction update folded into the product).
-      const float fb = static_cast<float>(beta);
-      const bool firstIt = it == 0;
-      double vpap[1] = {0.0};
-      const float3 az = slicedProduct(A, D.z);
-      if (own) {
-        p = firstIt ? z : axpyRn(p, fb, z);
-        const float3 acc = firstIt ? az : axpyRn(apFull, fb, az);
-        ap = filterRn(c, acc);
-        apFull = acc;
-        vpap[0] += dotd3(p, ap);
-      }
-      double pAp[1];
-      if (!gridReduce<1, false, true>(D, gs, vpap, pAp)) return -1;
-      if (!(pAp[0] > 0.0)) break;
-      const double alpha = rz / pAp[0];
-      const float fa = static_cast<float>(alpha);
-      ++it;
-      // Update (kernels.h:304-315) fused with the preconditioner apply (kernels.h:324-332).
-      double v[2] = {0.0, 0.0};
-      if (own) {
-        step = axpyRn(p, fa, step);
-        r = axpyRn(ap, -fa, r);
-        resid = axpyRn(apFull, -fa, resid);
-        z = filterRn(c, mulRn(M, r));
-        D.z[i] = f4(z);
-        v[0] += dotd3(r, r);
-        v[1] += dotd3(r, z);
-      }
-      double t2[2];
-      if (!gridReduce<2>(D, gs, v, t2)) return -1;
-      if (sqrt(t2[0]) <= D.P.cgTolerance * r0) break;
-      beta = t2[1] / rz;
-      rz = t2[1];
-    }
-  }
-  if (own) {
-    D.step[i] = f4(step);
-    D.resid[i] = f4(resid);
-    D.r[i] = f4(r);
-  }
-  return it;
-}
-
-constexpr int kLearnedDepth = 4;  // slots whose factor rows and gathered vector a row thread has in flight
-
-// acc += B x (Upper: B^T x) for this thread's row over its slots [k0, k1) of the block's sliced column layout (slot k
-// is global slot rs + k; the columns are sorted, so the lower part j <= i is [0, kd] and the upper part j >= i is
-// [kd, end) with kd the diagonal's position), the blocks from the factor by rows (D.LfRows); padding and pinned columns
-// carry bit 31 and are skipped. kLearnedDepth slots' loads are issued before their first FMA.
-template <bool Upper>
-__device__ __forceinline__ float3 factorProduct(const Dev& D, const SlicedMatrix& A, uint32_t rs, uint32_t kBegin,
-                                                uint32_t kEnd, const float4* x) {
-  const uint32_t lane = threadIdx.x & 31u;
+// InSmem: the factor is in shared memory. kLearnedDepth slots' loads are issued before their first product (past the
+// range's end the last slot's again, unused).
+template <bool Upper, bool InSmem>
+__device__ __forceinline__ float3 factorProduct(const Dev& D, const ResidentMatrix& A, const float4* x,
+                                                uint32_t kBegin, uint32_t kEnd) {
+  const uint32_t lane = threadIdx.x & 31u, zeroNode = D.P.residentNodes - 1;
+  const uint16_t* cols = reinterpret_cast<const uint16_t*>(A.cols);
   float3 acc = mk(0, 0, 0);
   for (uint32_t k0 = kBegin; k0 < kEnd; k0 += kLearnedDepth) {
-    bool use[kLearnedDepth];
-    float3 v[kLearnedDepth];
-    float4 m[kLearnedDepth][3];
+    uint32_t col[kLearnedDepth];
+    float4 m[kLearnedDepth][3], v[kLearnedDepth];
 #pragma unroll
     for (int u = 0; u < kLearnedDepth; ++u) {
-      const uint32_t k = k0 + u;
-      const uint32_t col = k < kEnd ? A.cols[A.base + 32u * k + lane] : kPinnedBit;
-      use[u] = !(col & kPinnedBit);
-      v[u] = mk(0, 0, 0);
-      m[u][0] = m[u][1] = m[u][2] = make_float4(0, 0, 0, 0);
-      if (use[u]) {
-        v[u] = ld3(x, col);
-        const float4* row = D.LfRows + 3 * static_cast<size_t>(rs + k);
-        m[u][0] = __ldg(row);
-        m[u][1] = __ldg(row + 1);
-        m[u][2] = __ldg(row + 2);
-      }
+      const uint32_t k = min(k0 + u, kEnd - 1), j = max(k, static_cast<uint32_t>(kRegSlots)) - kRegSlots;
+      static_assert(kRegSlots == 2, "the register slots' columns are one word");
+      const uint32_t inRegs = k == 0 ? A.regCols[0] & 0xFFFFu : A.regCols[0] >> 16;
+      const uint32_t inSmem = cols[A.base + (32u * (j >> 1) + lane) * 2u + (j & 1u)];
+      col[u] = k < static_cast<uint32_t>(kRegSlots) ? inRegs : inSmem;
+      if (k0 + u >= kEnd) col[u] = zeroNode;
     }
 #pragma unroll
     for (int u = 0; u < kLearnedDepth; ++u) {
-      if (!use[u]) continue;
+      const uint32_t k = min(k0 + u, kEnd - 1);
+      const float4* f = A.factor + A.factorBase + 32u * k + lane;
+#pragma unroll
+      for (int q = 0; q < 3; ++q) m[u][q] = InSmem ? f[q * D.P.factorSlots] : __ldcg(f + q * D.P.factorSlots);
+      v[u] = x[col[u]];
+    }
+#pragma unroll
+    for (int u = 0; u < kLearnedDepth; ++u) {
+      if (col[u] == zeroNode) continue;  // pinned columns and the end of the range
       const float4 a = m[u][0], b = m[u][1], c = m[u][2];
-      const float3 w = v[u];
+      const float3 w = xyz(v[u]);
       if (Upper) {  // L_ji^T x_j
-        acc.x += a.x * w.x + b.x * w.y + c.x * w.z;
-        acc.y += a.y * w.x + b.y * w.y + c.y * w.z;
-        acc.z += a.z * w.x + b.z * w.y + c.z * w.z;
+        acc.x = __fadd_rn(acc.x, dotYRn(a.x, b.x, c.x, w));
+        acc.y = __fadd_rn(acc.y, dotYRn(a.y, b.y, c.y, w));
+        acc.z = __fadd_rn(acc.z, dotYRn(a.z, b.z, c.z, w));
       } else {  // L_ij x_j
-        acc.x += a.x * w.x + a.y * w.y + a.z * w.z;
-        acc.y += b.x * w.x + b.y * w.y + b.z * w.z;
-        acc.z += c.x * w.x + c.y * w.y + c.z * w.z;
+        acc.x = __fadd_rn(acc.x, dotYRn(a.x, a.y, a.z, w));
+        acc.y = __fadd_rn(acc.y, dotYRn(b.x, b.y, b.z, w));
+        acc.z = __fadd_rn(acc.z, dotYRn(c.x, c.y, c.z, w));
       }
     }
   }
   return acc;
 }
 
-// z_i = F(L L^T r)_i for this thread's row over resident rows (pcgLearnedResident). y = L^T r goes through D.ap (r was
-// published by the caller's reduction; a grid barrier publishes y); returns false when the barrier gave up.
-__device__ inline bool applyLearnedResident(const Dev& D, GridSync& gs, const SlicedMatrix& A, uint32_t i, bool own,
-                                            uint32_t rs, uint32_t kd, uint32_t len, const Contact& c, float3& z) {
-  // y_i = sum over the row's slots (i, j), j >= i, of L_(j, i)^T r_j.
-  if (own) D.ap[i] = f4(factorProduct<true>(D, A, rs, kd, len, D.r));  // pinned rows: kd = len = 0
-  if (!gs.sync()) return false;
-  // z_i = F(sum over the row's slots (i, j), j <= i, of L_(i, j) y_j).
-  if (own) {
-    z = filterContact(c, factorProduct<false>(D, A, rs, 0, min(kd + 1, len), D.ap));
-    D.z[i] = f4(z);
-  }
-  return true;
-}
-
-// The learned-preconditioner PCG of pcgLearned (M^-1 = L L^T, contact-filtered, the same stopping tests and breakdown
-// rules) over resident rows: each thread keeps its row's step, resid, r, z, p, A p and its filtered copy in registers;
-// the matrix is the block's sliced shared-memory copy; r and z are published for the neighbours' gathers. Four grid
-// exchanges an iteration (p.Ap; r.r, which publishes r; y = L^T r; r.z, which publishes z), as in pcgLearned. Returns
-// the iteration count, -1 when a barrier gave up, or -2 - iterations on a breakdown (the caller then solves with
-// block-Jacobi).
-__device__ inline int pcgLearnedResident(const Dev& D, GridSync& gs, const SlicedMatrix& A) {
-  uint32_t r0i, r1i;
-  blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
-  const uint32_t i = r0i + threadIdx.x;
-  const bool own = i < r1i;
-  const uint32_t rs = own ? __ldg(D.rowStart + i) : 0u;
-  // The row's length and its diagonal's position (the factor's lower part is [0, kd], the upper [kd, len)); a pinned
-  // row has no slots in the sliced layout (its L is zero) and takes none, and no range passes the warp's length.
-  const bool live = own && D.particle[i].pinned == 0u;
-  const uint32_t len = live ? min(__ldg(D.rowStart + i + 1) - rs, A.len) : 0u;
-  const uint32_t kd = live ? min(__ldg(D.diagSlot + i) - rs, len) : 0u;
-  Contact c{};
-  float3 step = mk(0, 0, 0), resid = mk(0, 0, 0), r = mk(0, 0, 0), z = mk(0, 0, 0);
-  float3 p = mk(0, 0, 0), ap = mk(0, 0, 0), apFull = mk(0, 0, 0);
-  auto writeBack = [&] {
-    if (own) {
-      D.step[i] = f4(step);
-      D.resid[i] = f4(resid);
-      D.r[i] = f4(r);
+// Returns the iteration count, -1 when a wait gave up, or -2 - iterations on a breakdown (the caller then solves with
+// block-Jacobi). `seq` is the last exchange's number, advanced by the exchanges done.
+__device__ inline int pcgLearnedResident(const Dev& D, GridSync& gs, ResidentMatrix& A, unsigned long long& seq) {
+  constexpr int kWarps = kRowWorkers / 32;
+  __shared__ ResidentShared sh;
+  const int maxCg = D.P.maxCg;
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  const unsigned long long base = seq;
+  if (threadIdx.x == 0) sh.failed = 0;
+  __syncthreads();
+  int it = 0, code = 0;
+  if (w == kWarps) {  // the exchange warp
+    double rz = 0.0, r0 = 0.0, rr0 = 0.0, total = 0.0;
+    unsigned long long num = base;
+    // One sum: waits for the row warps' part, adds it up over the blocks; false when a wait gave up.
+    int delays[3] = {kExchangeDelay, kExchangeDelay, kExchangeDelay};  // p.Ap, r.r, r.z
+    auto sum = [&](int& delay) {
+      namedSync<1>(kRowThreads);
+      const double part[1] = {warpSum(lane < kWarps ? sh.red[0][lane] : 0.0)};
+      double t[1] = {0.0};
+      const bool ok = !sh.failed && mailSum<1>(D.mail, D.ctl, D.P.barrierLimitNs, gs.rank, gs.size, ++num, part, t,
+                                               delay);
+      total = t[0];
+      return ok;
+    };
+    auto tell = [&](float factor) {
+      if (lane == 0) {
+        sh.code = code;
+        sh.factor = factor;
+        sh.seq = num;
+      }
+      namedArrive<3>(kRowThreads);
+      return code == 0;
+    };
+    // |r0|, then r.z.
+    if (!sum(delays[1])) {
+      code = 2;
+    } else {
+      rr0 = total;
+      r0 = sqrt(rr0);
+      code = r0 > 0.0 && rr0 > 0.0 ? 0 : 1;
     }
-  };
-  double rr0;
-  {
-    double v[1] = {0.0}, t[1];
+    if (tell(0.0f)) {
+      if (!sum(delays[2])) code = 2;
+      else code = isfinite(total) ? 0 : 3;
+      rz = total;
+      if (tell(0.0f)) {
+        while (it < maxCg) {
+          if (!sum(delays[0])) code = 2;  // p.Ap
+          else code = !isfinite(total) ? 3 : total > 0.0 ? 0 : 1;
+          if (!tell(code ? 0.0f : static_cast<float>(rz / total))) break;
+          ++it;
+          if (!sum(delays[1])) code = 2;  // r.r
+          else code = !isfinite(total) ? 3 : sqrt(total) <= D.P.cgTolerance * r0 ? 1 : total > 1e6 * rr0 ? 3 : 0;
+          if (!tell(0.0f)) break;
+          if (!sum(delays[2])) code = 2;  // r.z
+          else code = isfinite(total) ? 0 : 3;
+          const float beta = static_cast<float>(total / rz);
+          rz = total;
+          if (!tell(beta)) break;
+        }
+      }
+    }
+  } else {
+    uint32_t r0i, r1i;
+    blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
+    const uint32_t i = r0i + threadIdx.x;
+    const bool own = i < r1i, busy = 32u * w < r1i - r0i;
+    // The row's length and its diagonal's position (the factor's lower part is [0, kd], the upper [kd, len)); a pinned
+    // row takes none (its L is zero), and no range passes the slots staged.
+    const uint32_t rs = own ? __ldg(D.rowStart + i) : 0u;
+    const bool live = own && D.particle[i].pinned == 0u;
+    const uint32_t len = live ? min(__ldg(D.rowStart + i + 1) - rs, A.len + kRegSlots) : 0u;
+    const uint32_t kd = live ? min(__ldg(D.diagSlot + i) - rs, len) : 0u;
+    Contact c{};
+    float3 step = mk(0, 0, 0), resid = mk(0, 0, 0), r = mk(0, 0, 0), z = mk(0, 0, 0);
+    float3 p = mk(0, 0, 0), ap = mk(0, 0, 0), apFull = mk(0, 0, 0);
     if (own) {
       c = D.contact[i];
       resid = -ld3(D.grad, i);
-      r = filterContact(c, resid);
-      D.r[i] = f4(r);
-      v[0] = dotd3(r, r);
+      r = filterRn(c, resid);
     }
-    if (!gridReduce<1>(D, gs, v, t)) return -1;
-    rr0 = t[0];
-  }
-  const double r0 = sqrt(rr0);
-  if (!(r0 > 0.0) || !(rr0 > 0.0)) {
-    writeBack();
-    return 0;
-  }
-  double rz;
-  {
-    if (!applyLearnedResident(D, gs, A, i, own, rs, kd, len, c, z)) return -1;
-    double v[1] = {own ? dotd3(r, z) : 0.0}, t[1];
-    if (!gridReduce<1>(D, gs, v, t)) return -1;
-    rz = t[0];
-  }
-  if (!isfinite(rz)) return -2;
-  double beta = 0.0;
-  int it = 0;
-  while (it < D.P.maxCg) {
-    // A p = A z + beta A pPrev, p = z + beta pPrev.
-    const float fb = static_cast<float>(beta);
-    const float3 az = slicedProduct(A, D.z);
-    double vpap[1] = {0.0}, pAp[1];
+    if (!busy && lane == 0) sh.red[0][w] = 0.0;
+    float4* cur = A.z;                        // the operand being used
+    float4* other = A.z + D.P.residentNodes;  // and the next one's place
+    unsigned long long num = base;
+    // The row's sum on its way to the exchange warp.
+    auto send = [&](float3 x, float3 y) {
+      if (busy) {
+        const double v = warpSum(dotd3(x, y));  // zero where no row is owned
+        if (lane == 0) sh.red[0][w] = v;
+      }
+      namedArrive<1>(kRowThreads);
+    };
+    auto hear = [&] {
+      namedSync<3>(kRowThreads);
+      code = sh.code;
+      return code == 0;
+    };
+    const uint32_t high = 0x80000000u;
+    auto publish = [&](float4* global, float3 v, uint32_t tag) {
+      if (own) {
+        storeTagged(global + i, v, tag);
+        cur[threadIdx.x] = f4(v);
+      }
+    };
+    auto take = [&](const float4* global, uint32_t tag) {
+      if (!takeHalo(D, A, cur, global, tag)) sh.failed = 1;
+      namedSync<2>(kRowWorkers);
+    };
+    auto turn = [&] {
+      float4* t = cur;
+      cur = other;
+      other = t;
+    };
+    // z = F(L L^T r), r.r on its way meanwhile; then r.z on its way. Returns false when r.r ends the solve.
+    auto apply = [&] {
+      const uint32_t tag = static_cast<uint32_t>(++num) | high;
+      publish(D.r, r, tag);
+      send(r, r);
+      take(D.r, tag);
+      float3 y = mk(0, 0, 0);
+      if (busy) y = D.LfSliced ? factorProduct<true, false>(D, A, cur, kd, len)
+                               : factorProduct<true, true>(D, A, cur, kd, len);
+      turn();
+      publish(D.ap, y, tag);
+      take(D.ap, tag);
+      if (busy) z = filterYRn(c, D.LfSliced ? factorProduct<false, false>(D, A, cur, 0, min(kd + 1, len))
+                                            : factorProduct<false, true>(D, A, cur, 0, min(kd + 1, len)));
+      turn();
+      if (!hear()) return false;
+      const uint32_t tagZ = static_cast<uint32_t>(++num) | high;
+      publish(D.z, z, tagZ);
+      send(r, z);
+      return true;
+    };
+    // A z, r.z arriving meanwhile. Returns false when r.z ends the solve.
+    float3 az = mk(0, 0, 0);
+    auto product = [&] {
+      take(D.z, static_cast<uint32_t>(num) | high);
+      if (busy) az = residentProduct(A, cur);
+      turn();
+      return hear();
+    };
+    if (apply() && product()) {
+      float fb = 0.0f;
+      while (it < maxCg) {
+        // A p = A z + beta A pPrev, p = z + beta pPrev.
+        if (own) {
+          p = it == 0 ? z : axpyRn(p, fb, z);
+          apFull = it == 0 ? az : axpyRn(apFull, fb, az);
+          ap = filterYRn(c, apFull);
+        }
+        ++num;
+        send(p, ap);
+        if (!hear()) break;
+        const float fa = sh.factor;
+        ++it;
+        if (own) {
+          step = axpyRn(p, fa, step);
+          r = axpyRn(ap, -fa, r);
+          resid = axpyRn(apFull, -fa, resid);
+        }
+        if (!apply() || !product()) break;
+        fb = sh.factor;
+      }
+    }
     if (own) {
-      p = it == 0 ? z : z + p * fb;
-      apFull = it == 0 ? az : az + apFull * fb;
-      ap = filterContact(c, apFull);
-      vpap[0] = dotd3(p, ap);
+      D.step[i] = f4(step);
+      D.resid[i] = f4(resid);
     }
-    if (!gridReduce<1>(D, gs, vpap, pAp)) return -1;
-    if (!isfinite(pAp[0])) return -2 - it;
-    if (!(pAp[0] > 0.0)) break;
-    const float fa = static_cast<float>(rz / pAp[0]);
-    ++it;
-    double v[1] = {0.0}, rr[1];
-    if (own) {
-      step = step + p * fa;
-      r = r - ap * fa;
-      resid = resid - apFull * fa;
-      D.r[i] = f4(r);
-      v[0] = dotd3(r, r);
-    }
-    if (!gridReduce<1>(D, gs, v, rr)) return -1;
-    if (!isfinite(rr[0])) return -2 - it;
-    if (sqrt(rr[0]) <= D.P.cgTolerance * r0) break;
-    if (rr[0] > 1e6 * rr0) return -2 - it;
-    if (!applyLearnedResident(D, gs, A, i, own, rs, kd, len, c, z)) return -1;
-    double vz[1] = {own ? dotd3(r, z) : 0.0}, rzNew[1];
-    if (!gridReduce<1>(D, gs, vz, rzNew)) return -1;
-    if (!isfinite(rzNew[0])) return -2 - it;
-    beta = rzNew[0] / rz;
-    rz = rzNew[0];
   }
-  writeBack();
-  return it;
+  __syncthreads();
+  seq = sh.seq;
+  __syncthreads();
+  return code == 2 ? -1 : code == 3 ? -2 - it : it;
 }
 
 // Pipelined contact-filtered block-Jacobi PCG (Ghysels and Vanroose, "Hiding global synchronization latency in the
@@ -2031,30 +1970,30 @@ template <bool Learned, int PL, int Variant = 0>
 __device__ inline int pcgSolve(const Dev& D, GridSync& gs) {
   uint32_t r0i, r1i;
   blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
-  if constexpr (Variant == kResidentRows && !Learned) {
+  if constexpr (Variant == kResidentRows) {
     ResidentMatrix A;
-    if (!stageResident(D, gs.rank, r0i, r1i, A)) return -1;
+    if (!stageResident<Learned>(D, gs.rank, r0i, r1i, A)) return -1;
     const unsigned long long t0 = globalTimerNs();
-    const int it = pcgResident(D, gs, A);
-    if (gs.rank == 0 && threadIdx.x == 0) D.ctl->pcgNs += static_cast<long long>(globalTimerNs() - t0);
-    return it;
-  } else if constexpr (Variant == kResidentRows) {
-    SlicedMatrix A;
-    if (!stageSliced(D, r0i, r1i, A)) return -1;
-    const unsigned long long t0 = globalTimerNs();
+    unsigned long long seq = __ldcg(D.mailSeq);
     int it;
-    {
+    if constexpr (Learned) {
       // The learned schedule without block-Jacobi iterations first (the host picks this kernel only then): a learned
       // solve that breaks down is followed by a full block-Jacobi solve, as in pcgSolveStaged.
-      it = pcgLearnedResident(D, gs, A);
+      it = pcgLearnedResident(D, gs, A, seq);
       if (gs.rank == 0 && threadIdx.x == 0) D.ctl->learnedSolves += 1;
       if (it < -1) {
         if (gs.rank == 0 && threadIdx.x == 0) D.ctl->precondFallbacks += 1;
-        const int jac = pcgResidentRows(D, gs, A);
+        const int jac = pcgResident(D, gs, A, seq);
         it = jac < 0 ? jac : jac + (-2 - it);
       }
+    } else {
+      it = pcgResident(D, gs, A, seq);
     }
-    if (gs.rank == 0 && threadIdx.x == 0) D.ctl->pcgNs += static_cast<long long>(globalTimerNs() - t0);
+    // Every block has sent a message by now (or none has), so every block has read the number.
+    if (gs.rank == 0 && threadIdx.x == 0) {
+      *D.mailSeq = seq;
+      D.ctl->pcgNs += static_cast<long long>(globalTimerNs() - t0);
+    }
     return it;
   } else {
     const SmemMatrix A = stageMatrix(D, r0i, r1i);

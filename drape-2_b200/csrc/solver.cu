@@ -74,27 +74,6 @@ static uint32_t maxResidentSlots(const uint32_t* rowStart, const uint8_t* pinned
   return most;
 }
 
-// Padded slots of the sliced layout k_solve_rows_learned stages for its largest block (the rows in warps of 32, each warp's
-// rows padded to its longest unpinned row; pinned rows take no slots), or UINT32_MAX when a block has more rows than
-// it has threads.
-static uint32_t maxSlicedSlots(const uint32_t* rowStart, const uint8_t* pinned, uint32_t n, int grid) {
-  const uint32_t per = (n + static_cast<uint32_t>(grid) - 1) / static_cast<uint32_t>(grid);
-  if (per > static_cast<uint32_t>(dcu::kRowThreads)) return UINT32_MAX;
-  uint32_t most = 0;
-  for (int b = 0; b < grid; ++b) {
-    const uint32_t r0 = std::min<uint32_t>(n, static_cast<uint32_t>(b) * per), r1 = std::min<uint32_t>(n, r0 + per);
-    uint32_t total = 0;
-    for (uint32_t w0 = r0; w0 < r1; w0 += 32) {
-      uint32_t len = 0;
-      for (uint32_t i = w0; i < std::min(r1, w0 + 32); ++i)
-        if (!pinned[i]) len = std::max(len, rowStart[i + 1] - rowStart[i]);
-      total += 32 * len;
-    }
-    most = std::max(most, total);
-  }
-  return most;
-}
-
 struct drape_solver {
   int device = 0;
   int numSMs = 0;
@@ -107,8 +86,7 @@ struct drape_solver {
   int failAfter = -1;
   static constexpr int kFrameSlots = 32;  // most frames one advanceFrames call runs before its host wait
   uint32_t solveSmemCap = 0;       // block slots one solve block can keep in shared memory
-  uint32_t rowsSmemCap = 0;        // padded slots one k_solve_rows_learned block can keep in shared memory
-  size_t residentSmemCap = 0;      // dynamic shared memory a k_solve_rows block can have
+  size_t residentSmemCap = 0, learnedSmemCap = 0;  // dynamic shared memory a k_solve_rows(_learned) block can have
   // Learned preconditioner: the solver's own copy of the network and its workspace on this solver's CSR.
   std::unique_ptr<net::Network> net;
   net::GraphHandle netGraph;
@@ -118,8 +96,9 @@ struct drape_solver {
   int pcgVariant = 0;               // block-Jacobi PCG form (drape_cuda_set_pcg_variant)
   uint64_t netNewtonCounter = 0;
   size_t solveSmemBytes = 0;       // dynamic shared memory of the solve launch for the built scene
-  size_t rowsSmemBytes = 0;        // k_solve_rows_learned's, when the built scene fits it (0: it does not)
-  size_t residentSmemBytes = 0;    // k_solve_rows's, likewise
+  size_t residentSmemBytes = 0;    // k_solve_rows's, when the built scene fits it (0: it does not)
+  size_t learnedSmemBytes = 0;     // k_solve_rows_learned's, likewise
+  bool learnedFactorOnChip = false;  // the learned factor is part of them
 
   DBuf<dcu::Particle> particle;
   DBuf<dcu::Fabric> fabric;
@@ -134,10 +113,11 @@ struct drape_solver {
   DBuf<float4> stretchDer, hingeDer;
   DBuf<dcu::Contact> contact;
   DBuf<double> partials, statsPartials;
-  DBuf<uint16_t> localCol;  // k_solve_rows: each slot's column among its block's rows and halo
-  DBuf<uint32_t> halo, haloCount;
-  DBuf<dcu::MailWord> mail;
-  DBuf<unsigned long long> mailSeq;
+  // k_solve_rows: each block's halo, then each slot's 16-bit column among its block's rows and halo (one allocation, like
+  // the mailbox with its number: device allocations are what a build waits for).
+  DBuf<uint32_t> residentIndex, haloCount;
+  DBuf<float4> factorSliced;  // k_solve_rows_learned: the factor in the sliced layout, where shared memory has no room
+  DBuf<dcu::MailWord> mail;  // its last word's tag is the number of the last exchange
   DBuf<dcu::Control> ctl;
   DBuf<dcu::StatsOut> statsOut;
   DBuf<unsigned int> statsDone;
@@ -239,8 +219,7 @@ struct drape_solver {
         if (perSM < 1) throw std::runtime_error("cuda: the resident-row solve kernel does not fit on an SM");
         return most;
       };
-      rowsSmemCap = static_cast<uint32_t>(allow(reinterpret_cast<const void*>(dcu::k_solve_rows_learned)) /
-                                          dcu::kSmemSlotBytes);
+      learnedSmemCap = allow(reinterpret_cast<const void*>(dcu::k_solve_rows_learned));
       residentSmemCap = allow(reinterpret_cast<const void*>(dcu::k_solve_rows));
     }
     solveGrid = numSMs;  // one 1024-thread block per SM: fewest barrier arrivals
@@ -250,8 +229,9 @@ struct drape_solver {
     hStats.alloc(kFrameSlots);
     ctl.alloc(1);
     partials.alloc(2 * static_cast<size_t>(solveGrid) * dcu::kPartialStride);  // two halves, alternating
-    mail.alloc(dcu::mailWords(static_cast<size_t>(solveGrid)));
-    mailSeq.alloc(1);  // the zeroed mailbox carries no number an exchange waits for: the first is 1
+    // Zeroed, the mailbox carries no number an exchange waits for: the first is 1.
+    mail.alloc(dcu::mailWords(static_cast<size_t>(solveGrid)) + 1);
+    haloCount.alloc(solveGrid);
     statsPartials.alloc(static_cast<size_t>(statsGrid) * 8);
     statsOut.alloc(kFrameSlots);
     statsDone.alloc(1);
@@ -274,6 +254,8 @@ struct drape_solver {
   }
 
   void use() const { CK(cudaSetDevice(device)); }
+
+  unsigned long long* mailSeq() const { return &mail.p[mail.n - 1].tag; }
 
   std::vector<dcu::Particle> particleData() const { return dmodel::particles(m); }
   std::vector<dcu::Fabric> fabricData() const { return dmodel::fabrics(m); }
@@ -334,12 +316,6 @@ struct drape_solver {
     dmodel::params(m, SP, barrierLimitNs, d);
     d.P.smemSlots = std::min(solveSmemCap, maxBlockSlots(m.rowStart.data(), n, solveGrid));
     solveSmemBytes = static_cast<size_t>(d.P.smemSlots) * dcu::kSmemSlotBytes;
-    {
-      const uint32_t sliced = maxSlicedSlots(m.rowStart.data(), m.pinned.data(), n, solveGrid);
-      const bool fits = sliced <= rowsSmemCap;
-      d.P.slicedSlots = fits ? std::max<uint32_t>(sliced, 1u) : 0u;
-      rowsSmemBytes = fits ? static_cast<size_t>(d.P.slicedSlots) * dcu::kSmemSlotBytes : 0;
-    }
     localize(n, B, d);
     d.fieldValues = fieldValues.p;
     d.particle = particle.p;
@@ -383,7 +359,7 @@ struct drape_solver {
     d.contact = contact.p;
     d.partials = partials.p;
     d.mail = mail.p;
-    d.mailSeq = mailSeq.p;
+    d.mailSeq = mailSeq();
     d.ctl = ctl.p;
     d.cgLog = cgLog.p;
     dev = d;
@@ -401,12 +377,11 @@ struct drape_solver {
   // Whether every solve block fits k_solve_rows (its padded slots, its rows and its halo in shared memory), and if so the
   // columns as indices into a block's rows and halo.
   void localize(uint32_t n, uint32_t B, dcu::Dev& d) {
-    residentSmemBytes = 0;
+    residentSmemBytes = learnedSmemBytes = 0;
     const uint32_t slots = maxResidentSlots(m.rowStart.data(), m.pinned.data(), n, solveGrid);
     if (n == 0 || slots == UINT32_MAX) return;
     const uint32_t words = (n + 31u) / 32u;  // n <= kRowWorkers * solveGrid: at most 18 KB of bitmap and counts
     const size_t bitmapBytes = 2 * sizeof(uint32_t) * static_cast<size_t>(words);
-    haloCount.alloc(solveGrid);
     dcu::k_localize<<<solveGrid, 512, bitmapBytes, stream>>>(n, solveGrid, rowStart.p, colIndex.p, words, haloCount.p, 0,
                                                              nullptr, nullptr);
     CK(cudaGetLastError());
@@ -421,18 +396,27 @@ struct drape_solver {
                          static_cast<size_t>(nodes) * dcu::kResidentNodeBytes;
     if (nodes >= dcu::kNoColumn || bytes > residentSmemCap) return;
     const uint32_t stride = std::max<uint32_t>(most, 1u);
-    halo.alloc(static_cast<size_t>(stride) * solveGrid);
-    localCol.alloc(B);
+    const size_t haloEntries = static_cast<size_t>(stride) * solveGrid;
+    residentIndex.alloc(haloEntries + (static_cast<size_t>(B) + 1) / 2);
+    uint16_t* localCol = reinterpret_cast<uint16_t*>(residentIndex.p + haloEntries);
     dcu::k_localize<<<solveGrid, 512, bitmapBytes, stream>>>(n, solveGrid, rowStart.p, colIndex.p, words, haloCount.p,
-                                                             stride, halo.p, localCol.p);
+                                                             stride, residentIndex.p, localCol);
     CK(cudaGetLastError());
     d.P.residentSlots = slots;
     d.P.residentNodes = nodes;
     d.P.haloStride = stride;
-    d.halo = halo.p;
+    d.halo = residentIndex.p;
     d.haloCount = haloCount.p;
-    d.localCol = localCol.p;
+    d.localCol = localCol;
     residentSmemBytes = bytes;
+    // The learned kernel: a second array of gathered vectors, and the factor where there is room.
+    const size_t more = bytes + static_cast<size_t>(nodes) * dcu::kResidentNodeBytes;
+    if (more > learnedSmemCap) return;
+    const uint32_t factorSlots = slots + dcu::kRegSlots * dcu::kRowWorkers;
+    const size_t factorBytes = 3 * sizeof(float4) * static_cast<size_t>(factorSlots);
+    d.P.factorSlots = factorSlots;
+    learnedFactorOnChip = more + factorBytes <= learnedSmemCap;
+    learnedSmemBytes = more + (learnedFactorOnChip ? factorBytes : 0);
   }
 
   // The network's workspace on this solver's CSR; the learned factor and transposed-slot map go into the device view.
@@ -447,6 +431,11 @@ struct drape_solver {
     dev.Lf = net->graphOf(*netGraph).L;
     dev.tslot = net->graphOf(*netGraph).tslot;
     dev.LfRows = net->graphOf(*netGraph).LF;
+    dev.LfSliced = nullptr;
+    if (learnedSmemBytes > 0 && !learnedFactorOnChip) {
+      factorSliced.alloc(3 * static_cast<size_t>(dev.P.factorSlots) * solveGrid);
+      dev.LfSliced = factorSliced.p;
+    }
     netNewtonCounter = 0;
   }
 
@@ -457,6 +446,7 @@ struct drape_solver {
       dev.Lf = nullptr;
       dev.tslot = nullptr;
       dev.LfRows = nullptr;
+      dev.LfSliced = nullptr;
       return;
     }
     if (!p->net) throw std::invalid_argument("null preconditioner handle");
@@ -531,9 +521,9 @@ struct drape_solver {
     // Blocks may have left an abandoned solve after different exchanges: go on with numbers none of them reached (nor
     // any tag, a number's low bits).
     unsigned long long seq = 0;
-    CK(cudaMemcpy(&seq, mailSeq.p, sizeof(seq), cudaMemcpyDeviceToHost));
+    CK(cudaMemcpy(&seq, mailSeq(), sizeof(seq), cudaMemcpyDeviceToHost));
     seq += 1ull << 24;
-    CK(cudaMemcpy(mailSeq.p, &seq, sizeof(seq), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(mailSeq(), &seq, sizeof(seq), cudaMemcpyHostToDevice));
   }
 
   // The reference-order PCG runs over resident rows (k_solve_rows) where the built scene fits it; bit-identical to
@@ -541,7 +531,7 @@ struct drape_solver {
   // (k_solve_rows_learned) unless block-Jacobi iterations come first (precondSwitch) or variant 3 forces k_solve<true>.
   bool usesResidentRows(const dcu::Dev& d) const {
     if (d.P.pcgVariant != 0) return false;
-    return learnedOn && netGraph ? rowsSmemBytes > 0 && precondSwitch == 0 : residentSmemBytes > 0;
+    return learnedOn && netGraph ? learnedSmemBytes > 0 && precondSwitch == 0 : residentSmemBytes > 0;
   }
 
   void launchSolve(const dcu::Dev& d) {
@@ -549,7 +539,7 @@ struct drape_solver {
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(solveGrid);
     cfg.blockDim = dim3(rows ? dcu::kRowThreads : dcu::kSolveThreads);
-    cfg.dynamicSmemBytes = !rows ? solveSmemBytes : learnedOn && netGraph ? rowsSmemBytes : residentSmemBytes;
+    cfg.dynamicSmemBytes = !rows ? solveSmemBytes : learnedOn && netGraph ? learnedSmemBytes : residentSmemBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;  // co-resident blocks for the grid barrier; capturable in a graph

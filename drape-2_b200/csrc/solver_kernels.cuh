@@ -338,7 +338,8 @@ __global__ void k_barrier_probe(Control* ctl, unsigned long long limitNs, int* o
 __global__ void k_mail_probe(Control* ctl, MailWord* mail, unsigned long long limitNs, int* out) {
   const double mine[1] = {1.0};
   double total[1];
-  const bool released = mailSum<1>(mail, ctl, limitNs, blockIdx.x, gridDim.x + 1, 1, mine, total);
+  int delay = 0;
+  const bool released = mailSum<1>(mail, ctl, limitNs, blockIdx.x, gridDim.x + 1, 1, mine, total, delay);
   if (threadIdx.x == 0 && blockIdx.x == 0) *out = released ? 0 : ctl->error;
 }
 

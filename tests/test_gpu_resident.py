@@ -62,3 +62,23 @@ def test_resident_rows_match_the_1024_thread_kernel(gpu, name):
     assert np.isfinite(x0).all()
     assert np.array_equal(h0, h3), (h0, h3)
     assert np.array_equal(x0, x3) and np.array_equal(v0, v3), np.abs(x0 - x3).max()
+
+
+@pytest.mark.parametrize("name", ["sheet_13x13", "pinned_37x37", "shuffled_60x60", "tube_60k"])
+def test_resident_learned_pcg_with_a_zero_output_layer_is_block_jacobi(gpu, name):
+    """With the initial network (zero output layer) the factor is exactly block-Jacobi's Cholesky factor, so the learned
+    resident kernel (the factor on chip for the small scenes, in the L2 for the 60k tube) follows the block-Jacobi one:
+    the same PCG counts in the first frame and positions that differ by the roundings of L L^T r against M^-1 r."""
+    from drape_b200 import learned
+    make = CASES.get(name, lambda: S.seamed_tube(154, 195, field_n=64, field_cell=0.012))
+    xj, _, hj, _ = _run(gpu, make(), 0, frames=1)
+    s = gpu.CudaSolver(0)
+    s.set_precond(learned.LearnedPreconditioner(0))
+    s.build(make())
+    assert s.solve_threads() == 512
+    s.step(1.0 / 60.0, 1, 2)
+    x, h, c = s.positions(), s.cg_history(), s.counters()
+    s.close()
+    assert c.learned_solves == c.newton_iterations == 2 and c.precond_fallbacks == 0
+    assert np.abs(np.asarray(h) - np.asarray(hj)).max() <= 1, (h, hj)
+    assert np.abs(x.astype(np.float64) - xj).max() < 1e-4
