@@ -104,6 +104,8 @@ struct Params {
   uint32_t residentSlots, residentNodes;  // k_solve_rows: a block's padded slots and its rows and halo, in shared memory
   uint32_t factorSlots; // k_solve_rows_learned: a block's padded factor slots
   uint32_t haloStride;  // entries of `halo` per solve block
+  // k_solve_rows_multi: slots of each row kept in shared memory (even), a block's rows, and its padded slots in the L2.
+  uint32_t multiKept, multiRows, spillSlots;
   unsigned long long barrierLimitNs;
 };
 
@@ -142,6 +144,7 @@ struct Dev {
   const uint16_t* localCol;   // per slot: its column among its solve block's rows and halo (k_localize)
   const uint32_t *halo, *haloCount;
   double* partials;
+  uint8_t* spill;             // k_solve_rows_multi: kResidentSlotBytes * spillSlots per block
   struct MailWord* mail;      // the solve grid's mailbox and the number of the last exchange (exchange.cuh)
   unsigned long long* mailSeq;
   Control* ctl;
@@ -1037,7 +1040,7 @@ __device__ inline int pcgReferenceOrder(const Dev& D, GridSync& gs, const SmemMa
 // (4.30-4.32).
 constexpr int kRowThreads = 512;    // k_solve_rows block size
 constexpr int kRowWorkers = 480;    // of these, the threads that own a row each; the last warp does the exchanges
-constexpr int kResidentRows = 4;    // the solve templates' Variant value of this form
+constexpr int kResidentRows = 4;    // the solve templates' Variant value of this form; 4 + m: m + 1 rows a thread
 constexpr int kRegSlots = 2;        // slots of each row kept in registers (even, so that slot parity is the same)
 constexpr int kExchangeDelay = 700; // clock cycles before an exchange's first poll, to begin with
 constexpr uint32_t kNoColumn = 0xFFFFu;  // localCol of a pinned column
@@ -1234,7 +1237,8 @@ __device__ __forceinline__ float3 residentProduct(const ResidentMatrix& A, const
 
 // The halo's entries of `global` into shared memory (behind the block's own in `z`), each particle's as soon as it carries
 // `tag`. Returns false when a wait gave up.
-__device__ __forceinline__ bool takeHalo(const Dev& D, const ResidentMatrix& A, float4* z, const float4* global,
+template <class Matrix>
+__device__ __forceinline__ bool takeHalo(const Dev& D, const Matrix& A, float4* z, const float4* global,
                                          uint32_t tag) {
   constexpr uint32_t kStep = kRowWorkers;
   bool ok = true;
@@ -1258,6 +1262,57 @@ __device__ __forceinline__ bool takeHalo(const Dev& D, const ResidentMatrix& A, 
   return ok;
 }
 
+// The exchange warp of pcgResident and pcgResidentMulti: every iteration's two sums, the scalars and the stopping tests.
+// Returns the iteration count; `code` as in ResidentShared.
+__device__ inline int residentExchanges(const Dev& D, const GridSync& gs, ResidentShared& sh, unsigned long long base,
+                                        int& code) {
+  constexpr int kWarps = kRowWorkers / 32;
+  const uint32_t lane = threadIdx.x & 31u;
+  const int maxCg = D.P.maxCg;
+  int it = 0;
+  double rz = 0.0, r0 = 0.0;
+  unsigned long long num = base;
+  int delayA = kExchangeDelay, delayB = kExchangeDelay;
+  while (it < maxCg) {
+    namedSync<1>(kRowThreads);
+    double part[2], sum[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) part[k] = warpSum(lane < kWarps ? sh.red[k][lane] : 0.0);
+    float factor = 0.0f;
+    if (!mailSum<2>(D.mail, D.ctl, D.P.barrierLimitNs, gs.rank, gs.size, ++num, part, sum, delayB)) {
+      code = 2;
+    } else if (it == 0) {
+      r0 = sqrt(sum[0]);
+      code = r0 > 0.0 ? 0 : 1;
+    } else {
+      code = sqrt(sum[0]) <= D.P.cgTolerance * r0 ? 1 : 0;
+      factor = static_cast<float>(sum[1] / rz);
+    }
+    rz = sum[1];
+    if (lane == 0) {
+      sh.code = code;
+      sh.factor = factor;
+    }
+    namedArrive<3>(kRowThreads);
+    if (code) break;
+    namedSync<1>(kRowThreads);
+    double pap[1] = {warpSum(lane < kWarps ? sh.red[0][lane] : 0.0)}, pAp[1];
+    if (sh.failed || !mailSum<1>(D.mail, D.ctl, D.P.barrierLimitNs, gs.rank, gs.size, ++num, pap, pAp, delayA))
+      code = 2;
+    else
+      code = pAp[0] > 0.0 ? 0 : 1;
+    if (lane == 0) {
+      sh.code = code;
+      sh.factor = code ? 0.0f : static_cast<float>(rz / pAp[0]);
+    }
+    namedArrive<3>(kRowThreads);
+    if (code) break;
+    ++it;
+  }
+  if (lane == 0) sh.seq = num;
+  return it;
+}
+
 // The reference-order PCG of pcgReferenceOrder (same recurrences, same stopping tests) over resident rows. Writes
 // step and resid of the block's rows; returns the iteration count, or -1 when an exchange gave up. `seq` is the last
 // exchange's number, advanced by the exchanges done.
@@ -1275,47 +1330,8 @@ __device__ inline int pcgResident(const Dev& D, GridSync& gs, ResidentMatrix& A,
   if (threadIdx.x == 0) sh.failed = 0;
   __syncthreads();
   int it = 0, code = 0;
-  if (w == kWarps) {  // the exchange warp
-    double rz = 0.0, r0 = 0.0;
-    unsigned long long num = base;
-    int delayA = kExchangeDelay, delayB = kExchangeDelay;
-    while (it < maxCg) {
-      namedSync<1>(kRowThreads);
-      double part[2], sum[2];
-#pragma unroll
-      for (int k = 0; k < 2; ++k) part[k] = warpSum(lane < kWarps ? sh.red[k][lane] : 0.0);
-      float factor = 0.0f;
-      if (!mailSum<2>(D.mail, D.ctl, D.P.barrierLimitNs, gs.rank, gs.size, ++num, part, sum, delayB)) {
-        code = 2;
-      } else if (it == 0) {
-        r0 = sqrt(sum[0]);
-        code = r0 > 0.0 ? 0 : 1;
-      } else {
-        code = sqrt(sum[0]) <= D.P.cgTolerance * r0 ? 1 : 0;
-        factor = static_cast<float>(sum[1] / rz);
-      }
-      rz = sum[1];
-      if (lane == 0) {
-        sh.code = code;
-        sh.factor = factor;
-      }
-      namedArrive<3>(kRowThreads);
-      if (code) break;
-      namedSync<1>(kRowThreads);
-      double pap[1] = {warpSum(lane < kWarps ? sh.red[0][lane] : 0.0)}, pAp[1];
-      if (sh.failed || !mailSum<1>(D.mail, D.ctl, D.P.barrierLimitNs, gs.rank, gs.size, ++num, pap, pAp, delayA))
-        code = 2;
-      else
-        code = pAp[0] > 0.0 ? 0 : 1;
-      if (lane == 0) {
-        sh.code = code;
-        sh.factor = code ? 0.0f : static_cast<float>(rz / pAp[0]);
-      }
-      namedArrive<3>(kRowThreads);
-      if (code) break;
-      ++it;
-    }
-    if (lane == 0) sh.seq = num;
+  if (w == kWarps) {
+    it = residentExchanges(D, gs, sh, base, code);
   } else {
     uint32_t r0i, r1i;
     blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
@@ -1379,6 +1395,300 @@ __device__ inline int pcgResident(const Dev& D, GridSync& gs, ResidentMatrix& A,
       D.step[i] = f4(step);
       D.resid[i] = f4(resid);
     }
+  }
+  __syncthreads();
+  seq = sh.seq;
+  __syncthreads();
+  return code == 2 ? -1 : it;
+}
+
+// ---------------------------------------------------------------------------------------------------------------
+// The same PCG for scenes with more rows than k_solve_rows has threads for, or more matrix than its shared memory holds
+// (k_solve_rows_multi): each row thread owns Rows rows of its block (rows 32 (w + 15 m) + lane for m < Rows, so slice
+// w + 15 m of 32 rows is warp w's), keeps their p, A p, r, resid and step in registers and the contact planes in shared
+// memory. The first P.multiKept slots of each row sit in shared memory; the others are copied at the start of the launch
+// into the block's part of D.spill, in the sliced layout, and read from the L2 in every product. The preconditioner
+// blocks are read from the L2. Exchanges, tags and stopping tests are pcgResident's; beta arrives during the first
+// slice's product, so each row's p and A p are formed as soon as its product is.
+//
+// What bounds it: the bytes an SM reads from the L2 in an iteration, 38 a slot that is not kept and 48 a row. Measured (us per PCG iteration
+// on one B200, against the 1024-thread kernel, which reads every row vector and most of the matrix from the L2 and takes
+// two counter barriers): 72k particles 7.1 (11.9), 102k 8.4 (18.4), 141k 9.8 (25.5), 150k 10.7 (27.9), 199k 21.6 (45.5).
+// Three rows a thread take the block to 213k particles; the state of a fourth would not fit the registers.
+struct MultiMatrix {
+  const float4 *a, *b;   // kept slots, as in ResidentMatrix
+  const float* c;
+  const uint32_t* cols;
+  const float4 *sa, *sb;  // slots in the L2
+  const float* sc;
+  const uint32_t* scols;
+  float4* z;
+  float4* plane;  // the rows' contact planes: normal, and in w whether the contact is active
+  uint32_t rows, haloSize;
+  const uint32_t* halo;
+};
+
+constexpr int kMultiMost = 3;  // rows a thread may own
+
+struct MultiSlices {  // per slice: its first kept slot, its kept slots, its first slot in the L2, and its slots there
+  uint32_t kept[kMultiMost * kRowWorkers / 32 + 1], keptLen[kMultiMost * kRowWorkers / 32];
+  uint32_t spill[kMultiMost * kRowWorkers / 32 + 1], spillLen[kMultiMost * kRowWorkers / 32];
+};
+
+__device__ __forceinline__ float3 filterRn(float4 plane, float3 v) {
+  if (plane.w == 0.0f) return v;
+  return axpyRn(xyz(plane), -dotRn(plane.x, plane.y, plane.z, v), v);
+}
+
+template <int Rows>
+__device__ inline bool stageMulti(const Dev& D, uint32_t rank, uint32_t r0, uint32_t r1, MultiMatrix& A,
+                                  MultiSlices& sl) {
+  constexpr uint32_t kMost = Rows * kRowWorkers;
+  __shared__ uint32_t off[kMost + 1];
+  const uint32_t t = threadIdx.x, lane = t & 31u;
+  const uint32_t R = r1 - r0, slices = (R + 31u) / 32u, q = D.P.multiKept;
+  A.rows = R;
+  A.haloSize = __ldg(D.haloCount + rank);
+  A.halo = D.halo + static_cast<size_t>(rank) * D.P.haloStride;
+  if (R > kMost || blockDim.x != static_cast<unsigned>(kRowThreads) || R + A.haloSize >= D.P.residentNodes) {
+    if (t == 0) atomicExch(&D.ctl->error, 4);
+    return false;
+  }
+  const uint32_t first = __ldg(D.rowStart + r0);
+  for (uint32_t r = t; r < 32u * slices; r += blockDim.x) {
+    uint32_t count = 0;
+    if (r < R) {
+      const uint32_t rs = __ldg(D.rowStart + r0 + r);
+      const bool pinned = D.particle[r0 + r].pinned != 0u;
+      off[r] = (rs - first) | (pinned ? kPinnedBit : 0u);
+      if (!pinned) count = __ldg(D.rowStart + r0 + r + 1) - rs;
+    }
+    const uint32_t len = (__reduce_max_sync(0xffffffffu, count) + 1u) & ~1u;
+    if (lane == 0) {
+      sl.keptLen[r / 32] = min(len, q);
+      sl.spillLen[r / 32] = len - min(len, q);
+    }
+  }
+  if (t == 0) off[R] = __ldg(D.rowStart + r1) - first;
+  __syncthreads();
+  if (t == 0) {
+    uint32_t k = 0, x = 0;
+    for (uint32_t i = 0; i < slices; ++i) {
+      sl.kept[i] = k;
+      sl.spill[i] = x;
+      k += 32u * sl.keptLen[i];
+      x += 32u * sl.spillLen[i];
+    }
+    sl.kept[slices] = k;
+    sl.spill[slices] = x;
+  }
+  __syncthreads();
+  const uint32_t cap = D.P.residentSlots, spillCap = D.P.spillSlots, zeroNode = D.P.residentNodes - 1;
+  if (sl.kept[slices] > cap || sl.spill[slices] > spillCap) {
+    if (t == 0) atomicExch(&D.ctl->error, 4);
+    return false;
+  }
+  float4* a = solveSmem;
+  float4* b = a + cap;
+  A.z = b + cap;
+  A.plane = A.z + D.P.residentNodes;
+  float* c = reinterpret_cast<float*>(A.plane + D.P.multiRows);
+  uint16_t* cols = reinterpret_cast<uint16_t*>(c + cap);
+  float4* sa = reinterpret_cast<float4*>(D.spill + static_cast<size_t>(rank) * spillCap * kResidentSlotBytes);
+  float4* sb = sa + spillCap;
+  float* sc = reinterpret_cast<float*>(sb + spillCap);
+  uint16_t* scols = reinterpret_cast<uint16_t*>(sc + spillCap);
+  A.a = a;
+  A.b = b;
+  A.c = c;
+  A.cols = reinterpret_cast<const uint32_t*>(cols);
+  A.sa = sa;
+  A.sb = sb;
+  A.sc = sc;
+  A.scols = reinterpret_cast<const uint32_t*>(scols);
+  if (t == 0) A.z[zeroNode] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  for (uint32_t r = t; r < R; r += blockDim.x) {
+    const Contact ct = D.contact[r0 + r];
+    A.plane[r] = f4(xyz(ct.normal));
+    A.plane[r].w = ct.active != 0u ? 1.0f : 0.0f;
+  }
+  auto colAt = [](uint32_t base, uint32_t j, uint32_t l) { return base + (32u * (j >> 1) + l) * 2u + (j & 1u); };
+  auto put = [&](uint32_t slice, uint32_t j, uint32_t l, const float (&m)[9], uint32_t col) {
+    const float4 x = make_float4(m[0], m[1], m[2], m[3]), y = make_float4(m[4], m[5], m[6], m[7]);
+    const uint16_t cl = static_cast<uint16_t>(col == kNoColumn ? zeroNode : col);
+    if (j < q) {
+      const uint32_t pos = sl.kept[slice] + 32u * j + l;
+      a[pos] = x;
+      b[pos] = y;
+      c[pos] = m[8];
+      cols[colAt(sl.kept[slice], j, l)] = cl;
+    } else {
+      const uint32_t pos = sl.spill[slice] + 32u * (j - q) + l;
+      sa[pos] = x;
+      sb[pos] = y;
+      sc[pos] = m[8];
+      scols[colAt(sl.spill[slice], j - q, l)] = cl;
+    }
+  };
+  // Padding: each row's positions past its own slots (past its pinned rows' none).
+  const float zero[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+  for (uint32_t r = t; r < 32u * slices; r += blockDim.x) {
+    const uint32_t count = r < R && !(off[r] & kPinnedBit) ? (off[r + 1] & ~kPinnedBit) - off[r] : 0u;
+    for (uint32_t j = count; j < sl.keptLen[r / 32] + sl.spillLen[r / 32]; ++j) put(r / 32, j, r & 31u, zero, kNoColumn);
+  }
+  const uint32_t S = off[R], SP = D.P.slotsPadded;
+  for (uint32_t k = t; k < S; k += blockDim.x) {
+    uint32_t lo = 0, hi = R;  // row lo's first slot <= k < row hi's first slot
+    while (hi - lo > 1) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if ((off[mid] & ~kPinnedBit) <= k) lo = mid; else hi = mid;
+    }
+    if (off[lo] & kPinnedBit) continue;  // a pinned row's slot
+    const uint32_t s = first + k, col = __ldg(D.localCol + s);
+    float m[9];
+#pragma unroll
+    for (int e = 0; e < 9; ++e) m[e] = col == kNoColumn ? 0.0f : __ldg(D.blocks + e * SP + s);
+    put(lo >> 5, k - off[lo], lo & 31u, m, col);
+  }
+  __syncthreads();
+  return true;
+}
+
+// U slots (U even) of a slice from slot k on, kept (shared memory) or not (L2): all their loads before the first product.
+template <int U, bool Kept>
+__device__ __forceinline__ void multiSlots(const MultiMatrix& A, uint32_t base, uint32_t k, float3 (&acc)[2]) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t cc[U / 2];
+  float4 a[U], b[U], x[U];
+  float c[U];
+#pragma unroll
+  for (int u = 0; u < U / 2; ++u) {
+    const uint32_t at = base / 2 + 16u * k + 32u * u + lane;
+    cc[u] = Kept ? A.cols[at] : __ldcg(A.scols + at);
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const uint32_t pos = base + 32u * (k + u) + lane;
+    a[u] = Kept ? A.a[pos] : __ldcg(A.sa + pos);
+    b[u] = Kept ? A.b[pos] : __ldcg(A.sb + pos);
+    c[u] = Kept ? A.c[pos] : __ldcg(A.sc + pos);
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u) x[u] = A.z[(u & 1) ? cc[u / 2] >> 16 : cc[u / 2] & 0xFFFFu];
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const float m[9] = {a[u].x, a[u].y, a[u].z, a[u].w, b[u].x, b[u].y, b[u].z, b[u].w, c[u]};
+    blockMulAddRn(acc[u & 1], m, xyz(x[u]));
+  }
+}
+
+// A z for this thread's row of a slice, in residentProduct's order (multiKept is even, so slot parity is kept).
+__device__ __forceinline__ float3 multiProduct(const MultiMatrix& A, const MultiSlices& sl, uint32_t slice) {
+  float3 acc[2] = {mk(0, 0, 0), mk(0, 0, 0)};
+  const uint32_t kept = sl.keptLen[slice], spill = sl.spillLen[slice];
+  uint32_t k = 0;
+  for (; k + 4 <= kept; k += 4) multiSlots<4, true>(A, sl.kept[slice], k, acc);
+  if (k < kept) multiSlots<2, true>(A, sl.kept[slice], k, acc);
+  k = 0;
+  for (; k + 4 <= spill; k += 4) multiSlots<4, false>(A, sl.spill[slice], k, acc);
+  if (k < spill) multiSlots<2, false>(A, sl.spill[slice], k, acc);
+  return mk(__fadd_rn(acc[0].x, acc[1].x), __fadd_rn(acc[0].y, acc[1].y), __fadd_rn(acc[0].z, acc[1].z));
+}
+
+template <int Rows>
+__device__ inline int pcgResidentMulti(const Dev& D, GridSync& gs, const MultiMatrix& A, const MultiSlices& sl,
+                                       unsigned long long& seq) {
+  constexpr int kWarps = kRowWorkers / 32;
+  __shared__ ResidentShared sh;
+  const int maxCg = D.P.maxCg;
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  const unsigned long long base = seq;
+  if (threadIdx.x == 0) sh.failed = 0;
+  __syncthreads();
+  int it = 0, code = 0;
+  if (w == kWarps) {
+    it = residentExchanges(D, gs, sh, base, code);
+  } else {
+    uint32_t r0i, r1i;
+    blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
+    const uint32_t R = r1i - r0i;
+    uint32_t row[Rows];  // in the block
+    bool own[Rows];
+    float3 step[Rows], resid[Rows], r[Rows], p[Rows], apFull[Rows];
+#pragma unroll
+    for (int m = 0; m < Rows; ++m) {
+      row[m] = 32u * (w + kWarps * m) + lane;
+      own[m] = row[m] < R;
+      step[m] = resid[m] = r[m] = p[m] = apFull[m] = mk(0, 0, 0);
+      if (own[m]) {
+        resid[m] = -ld3(D.grad, r0i + row[m]);
+        r[m] = filterRn(A.plane[row[m]], resid[m]);
+      }
+    }
+    while (it < maxCg) {
+      const uint32_t tag = static_cast<uint32_t>(base + 1 + 2 * static_cast<unsigned long long>(it)) | 0x80000000u;
+      double rr = 0.0, rz = 0.0;
+#pragma unroll
+      for (int m = 0; m < Rows; ++m)
+        if (own[m]) {
+          const uint32_t i = r0i + row[m];
+          const float3 z = filterRn(A.plane[row[m]], mulRn(loadPrecond(D, i), r[m]));
+          storeTagged(D.z + i, z, tag);
+          A.z[row[m]] = f4(z);
+          rr += dotd3(r[m], r[m]);
+          rz += dotd3(r[m], z);
+        }
+      rr = warpSum(rr);
+      rz = warpSum(rz);
+      if (lane == 0) {
+        sh.red[0][w] = rr;
+        sh.red[1][w] = rz;
+      }
+      namedArrive<1>(kRowThreads);
+      if (!takeHalo(D, A, A.z, D.z, tag)) sh.failed = 1;
+      namedSync<2>(kRowWorkers);
+      double pap = 0.0;
+      float fb = 0.0f;
+#pragma unroll
+      for (int m = 0; m < Rows; ++m) {
+        const bool busy = 32u * (w + kWarps * m) < R;
+        const float3 az = busy ? multiProduct(A, sl, w + kWarps * m) : mk(0, 0, 0);
+        if (m == 0) {
+          namedSync<3>(kRowThreads);
+          code = sh.code;
+          if (code) break;
+          fb = sh.factor;
+        }
+        if (own[m]) {
+          const float3 z = xyz(A.z[row[m]]);
+          p[m] = it == 0 ? z : axpyRn(p[m], fb, z);
+          apFull[m] = it == 0 ? az : axpyRn(apFull[m], fb, az);
+          pap += dotd3(p[m], filterRn(A.plane[row[m]], apFull[m]));
+        }
+      }
+      if (code) break;
+      pap = warpSum(pap);
+      if (lane == 0) sh.red[0][w] = pap;
+      namedArrive<1>(kRowThreads);
+      namedSync<3>(kRowThreads);
+      code = sh.code;
+      if (code) break;
+      const float fa = sh.factor;
+      ++it;
+#pragma unroll
+      for (int m = 0; m < Rows; ++m)
+        if (own[m]) {
+          step[m] = axpyRn(p[m], fa, step[m]);
+          r[m] = axpyRn(filterRn(A.plane[row[m]], apFull[m]), -fa, r[m]);
+          resid[m] = axpyRn(apFull[m], -fa, resid[m]);
+        }
+    }
+#pragma unroll
+    for (int m = 0; m < Rows; ++m)
+      if (own[m]) {
+        D.step[r0i + row[m]] = f4(step[m]);
+        D.resid[r0i + row[m]] = f4(resid[m]);
+      }
   }
   __syncthreads();
   seq = sh.seq;
@@ -1970,7 +2280,20 @@ template <bool Learned, int PL, int Variant = 0>
 __device__ inline int pcgSolve(const Dev& D, GridSync& gs) {
   uint32_t r0i, r1i;
   blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
-  if constexpr (Variant == kResidentRows) {
+  if constexpr (Variant > kResidentRows) {
+    constexpr int kRows = Variant - kResidentRows + 1;
+    __shared__ MultiSlices sl;
+    MultiMatrix A;
+    if (!stageMulti<kRows>(D, gs.rank, r0i, r1i, A, sl)) return -1;
+    const unsigned long long t0 = globalTimerNs();
+    unsigned long long seq = __ldcg(D.mailSeq);
+    const int it = pcgResidentMulti<kRows>(D, gs, A, sl, seq);
+    if (gs.rank == 0 && threadIdx.x == 0) {
+      *D.mailSeq = seq;
+      D.ctl->pcgNs += static_cast<long long>(globalTimerNs() - t0);
+    }
+    return it;
+  } else if constexpr (Variant == kResidentRows) {
     ResidentMatrix A;
     if (!stageResident<Learned>(D, gs.rank, r0i, r1i, A)) return -1;
     const unsigned long long t0 = globalTimerNs();
@@ -2053,7 +2376,7 @@ __device__ inline void solveGroup(const Dev& D, GridSync& gs) {
   // The resident-row kernel's 512-thread blocks stand for the reference-order kernel's 1024-thread ones: its energies
   // are summed as two virtual threads per thread, in that kernel's order, so both kernels take the same line-search
   // decisions (its rows, at most 512 per block, already sit on the same threads).
-  constexpr bool kVirtual = Variant == kResidentRows;
+  constexpr bool kVirtual = Variant >= kResidentRows;
   // Contact normal force from the residual (kernels.h:391-396), Newton slope grad . step and E(0), in FP64.
   double se[2];
   {

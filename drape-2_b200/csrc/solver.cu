@@ -53,26 +53,36 @@ static uint32_t maxBlockSlots(const uint32_t* rowStart, uint32_t n, int grid) {
   return most;
 }
 
-// Padded shared-memory slots of k_solve_rows's largest block (the rows in warps of 32, each warp's rows padded to its
-// longest unpinned row, whose first kRegSlots slots sit in registers), or UINT32_MAX when a block has more rows than
-// k_solve_rows has row threads.
-static uint32_t maxResidentSlots(const uint32_t* rowStart, const uint8_t* pinned, uint32_t n, int grid) {
-  const uint32_t per = (n + static_cast<uint32_t>(grid) - 1) / static_cast<uint32_t>(grid);
-  if (per > static_cast<uint32_t>(dcu::kRowWorkers)) return UINT32_MAX;
-  uint32_t most = 0;
-  for (int b = 0; b < grid; ++b) {
-    const uint32_t r0 = std::min<uint32_t>(n, static_cast<uint32_t>(b) * per), r1 = std::min<uint32_t>(n, r0 + per);
-    uint32_t total = 0;
-    for (uint32_t w0 = r0; w0 < r1; w0 += 32) {
-      uint32_t len = 0;
-      for (uint32_t i = w0; i < std::min(r1, w0 + 32); ++i)
-        if (!pinned[i]) len = std::max(len, rowStart[i + 1] - rowStart[i]);
-      total += len > dcu::kRegSlots ? 32 * ((len - dcu::kRegSlots + 1) & ~1u) : 0u;
+// The resident-row kernels' layout of a scene: for each solve block its rows in warps of 32, and for each warp the slots of
+// its longest unpinned row, to which they are padded (every block has the same number of entries).
+struct WarpLengths {
+  uint32_t perBlock = 0;
+  std::vector<uint32_t> len;
+  WarpLengths(const Model& m, int grid) {
+    const uint32_t n = static_cast<uint32_t>(m.x.size());
+    const uint32_t per = (n + static_cast<uint32_t>(grid) - 1) / static_cast<uint32_t>(grid);
+    perBlock = (per + 31) / 32;
+    len.assign(static_cast<size_t>(perBlock) * grid, 0);
+    for (int b = 0; b < grid; ++b) {
+      const uint32_t r0 = std::min<uint32_t>(n, static_cast<uint32_t>(b) * per), r1 = std::min<uint32_t>(n, r0 + per);
+      for (uint32_t i = r0; i < r1; ++i) {
+        uint32_t& l = len[static_cast<size_t>(b) * perBlock + (i - r0) / 32];
+        if (!m.pinned[i]) l = std::max(l, m.rowStart[i + 1] - m.rowStart[i]);
+      }
     }
-    most = std::max(most, total);
   }
-  return most;
-}
+  // The most padded slots of a block beyond the first `skip` of each row and within the first `keep` of the rest.
+  uint32_t most(uint32_t skip, uint32_t keep) const {
+    uint32_t out = 0;
+    for (size_t b = 0; b < len.size(); b += perBlock) {
+      uint32_t total = 0;
+      for (uint32_t k = 0; k < perBlock; ++k)
+        if (len[b + k] > skip) total += 32 * std::min(keep, (len[b + k] - skip + 1) & ~1u);
+      out = std::max(out, total);
+    }
+    return out;
+  }
+};
 
 struct drape_solver {
   int device = 0;
@@ -86,7 +96,8 @@ struct drape_solver {
   int failAfter = -1;
   static constexpr int kFrameSlots = 32;  // most frames one advanceFrames call runs before its host wait
   uint32_t solveSmemCap = 0;       // block slots one solve block can keep in shared memory
-  size_t residentSmemCap = 0, learnedSmemCap = 0;  // dynamic shared memory a k_solve_rows(_learned) block can have
+  // Dynamic shared memory a block of k_solve_rows, k_solve_rows_multi<2>, <3> and k_solve_rows_learned can have.
+  size_t residentSmemCap[dcu::kMultiMost] = {}, learnedSmemCap = 0;
   // Learned preconditioner: the solver's own copy of the network and its workspace on this solver's CSR.
   std::unique_ptr<net::Network> net;
   net::GraphHandle netGraph;
@@ -97,6 +108,7 @@ struct drape_solver {
   uint64_t netNewtonCounter = 0;
   size_t solveSmemBytes = 0;       // dynamic shared memory of the solve launch for the built scene
   size_t residentSmemBytes = 0;    // k_solve_rows's, when the built scene fits it (0: it does not)
+  int residentRowsPerThread = 1;   // 1: k_solve_rows; more: k_solve_rows_multi
   size_t learnedSmemBytes = 0;     // k_solve_rows_learned's, likewise
   bool learnedFactorOnChip = false;  // the learned factor is part of them
 
@@ -116,6 +128,7 @@ struct drape_solver {
   // k_solve_rows: each block's halo, then each slot's 16-bit column among its block's rows and halo (one allocation, like
   // the mailbox with its number: device allocations are what a build waits for).
   DBuf<uint32_t> residentIndex, haloCount;
+  DBuf<uint8_t> spill;  // k_solve_rows_multi: the slots that shared memory has no room for
   DBuf<float4> factorSliced;  // k_solve_rows_learned: the factor in the sliced layout, where shared memory has no room
   DBuf<dcu::MailWord> mail;  // its last word's tag is the number of the last exchange
   DBuf<dcu::Control> ctl;
@@ -220,7 +233,9 @@ struct drape_solver {
         return most;
       };
       learnedSmemCap = allow(reinterpret_cast<const void*>(dcu::k_solve_rows_learned));
-      residentSmemCap = allow(reinterpret_cast<const void*>(dcu::k_solve_rows));
+      residentSmemCap[0] = allow(reinterpret_cast<const void*>(dcu::k_solve_rows));
+      residentSmemCap[1] = allow(reinterpret_cast<const void*>(dcu::k_solve_rows_multi<2>));
+      residentSmemCap[2] = allow(reinterpret_cast<const void*>(dcu::k_solve_rows_multi<3>));
     }
     solveGrid = numSMs;  // one 1024-thread block per SM: fewest barrier arrivals
     pointGrid = numSMs * 8;
@@ -374,27 +389,64 @@ struct drape_solver {
     built = true;
   }
 
-  // Whether every solve block fits k_solve_rows (its padded slots, its rows and its halo in shared memory), and if so the
-  // columns as indices into a block's rows and halo.
+  // Picks the resident-row kernel that every solve block fits, if one does, and builds its index arrays: the halos, and
+  // the columns as indices into a block's rows and halo. One row a thread with the whole matrix on chip is the fastest
+  // form; else the fewest rows a thread, with the matrix partly in the L2.
   void localize(uint32_t n, uint32_t B, dcu::Dev& d) {
     residentSmemBytes = learnedSmemBytes = 0;
-    const uint32_t slots = maxResidentSlots(m.rowStart.data(), m.pinned.data(), n, solveGrid);
-    if (n == 0 || slots == UINT32_MAX) return;
-    const uint32_t words = (n + 31u) / 32u;  // n <= kRowWorkers * solveGrid: at most 18 KB of bitmap and counts
+    const uint32_t per = (n + static_cast<uint32_t>(solveGrid) - 1) / static_cast<uint32_t>(solveGrid);
+    if (n == 0 || per > static_cast<uint32_t>(dcu::kMultiMost * dcu::kRowWorkers)) return;
+    const uint32_t words = (n + 31u) / 32u;  // at most 54 KB of bitmap and counts
     const size_t bitmapBytes = 2 * sizeof(uint32_t) * static_cast<size_t>(words);
+    CK(cudaFuncSetAttribute(dcu::k_localize, cudaFuncAttributeMaxDynamicSharedMemorySize, 64 << 10));
     dcu::k_localize<<<solveGrid, 512, bitmapBytes, stream>>>(n, solveGrid, rowStart.p, colIndex.p, words, haloCount.p, 0,
                                                              nullptr, nullptr);
     CK(cudaGetLastError());
     std::vector<uint32_t> counts(solveGrid);
     CK(cudaMemcpyAsync(counts.data(), haloCount.p, sizeof(uint32_t) * counts.size(), cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    const uint32_t per = (n + static_cast<uint32_t>(solveGrid) - 1) / static_cast<uint32_t>(solveGrid);
     uint32_t most = 0;
     for (uint32_t c : counts) most = std::max(most, c);
     const uint32_t nodes = per + most + 1;  // and the zero particle
-    const size_t bytes = (static_cast<size_t>(slots) * dcu::kResidentSlotBytes + 15) / 16 * 16 +
-                         static_cast<size_t>(nodes) * dcu::kResidentNodeBytes;
-    if (nodes >= dcu::kNoColumn || bytes > residentSmemCap) return;
+    if (nodes >= dcu::kNoColumn) return;
+    const size_t nodeBytes = static_cast<size_t>(nodes) * dcu::kResidentNodeBytes;
+    auto slotBytes = [](uint32_t slots) {
+      return (static_cast<size_t>(slots) * dcu::kResidentSlotBytes + 15) / 16 * 16;
+    };
+    const WarpLengths lengths(m, solveGrid);
+    const uint32_t whole = lengths.most(dcu::kRegSlots, UINT32_MAX);
+    if (per <= static_cast<uint32_t>(dcu::kRowWorkers) && slotBytes(whole) + nodeBytes <= residentSmemCap[0]) {
+      residentRowsPerThread = 1;
+      d.P.residentSlots = whole;
+      residentSmemBytes = slotBytes(whole) + nodeBytes;
+      // The learned kernel: a second array of gathered vectors, and the factor where there is room.
+      const size_t more = residentSmemBytes + nodeBytes;
+      if (more <= learnedSmemCap) {
+        const uint32_t factorSlots = whole + dcu::kRegSlots * dcu::kRowWorkers;
+        const size_t factorBytes = 3 * sizeof(float4) * static_cast<size_t>(factorSlots);
+        d.P.factorSlots = factorSlots;
+        learnedFactorOnChip = more + factorBytes <= learnedSmemCap;
+        learnedSmemBytes = more + (learnedFactorOnChip ? factorBytes : 0);
+      }
+    } else {
+      residentRowsPerThread = per <= static_cast<uint32_t>(2 * dcu::kRowWorkers) ? 2 : 3;
+      const size_t cap = residentSmemCap[residentRowsPerThread - 1];
+      const size_t fixed = nodeBytes + sizeof(float4) * static_cast<size_t>(per);
+      if (fixed > cap) return;
+      // The most slots a row can keep: every block's padded slots within that many have to fit.
+      uint32_t kept = 0;
+      for (uint32_t k = 2; k <= 64; k += 2) {
+        if (fixed + slotBytes(lengths.most(0, k)) > cap) break;
+        kept = k;
+      }
+      d.P.multiKept = kept;
+      d.P.multiRows = per;
+      d.P.residentSlots = lengths.most(0, kept);
+      d.P.spillSlots = lengths.most(kept, UINT32_MAX);
+      residentSmemBytes = fixed + slotBytes(d.P.residentSlots);
+      spill.alloc(static_cast<size_t>(d.P.spillSlots) * dcu::kResidentSlotBytes * solveGrid);
+      d.spill = spill.p;
+    }
     const uint32_t stride = std::max<uint32_t>(most, 1u);
     const size_t haloEntries = static_cast<size_t>(stride) * solveGrid;
     residentIndex.alloc(haloEntries + (static_cast<size_t>(B) + 1) / 2);
@@ -402,21 +454,11 @@ struct drape_solver {
     dcu::k_localize<<<solveGrid, 512, bitmapBytes, stream>>>(n, solveGrid, rowStart.p, colIndex.p, words, haloCount.p,
                                                              stride, residentIndex.p, localCol);
     CK(cudaGetLastError());
-    d.P.residentSlots = slots;
     d.P.residentNodes = nodes;
     d.P.haloStride = stride;
     d.halo = residentIndex.p;
     d.haloCount = haloCount.p;
     d.localCol = localCol;
-    residentSmemBytes = bytes;
-    // The learned kernel: a second array of gathered vectors, and the factor where there is room.
-    const size_t more = bytes + static_cast<size_t>(nodes) * dcu::kResidentNodeBytes;
-    if (more > learnedSmemCap) return;
-    const uint32_t factorSlots = slots + dcu::kRegSlots * dcu::kRowWorkers;
-    const size_t factorBytes = 3 * sizeof(float4) * static_cast<size_t>(factorSlots);
-    d.P.factorSlots = factorSlots;
-    learnedFactorOnChip = more + factorBytes <= learnedSmemCap;
-    learnedSmemBytes = more + (learnedFactorOnChip ? factorBytes : 0);
   }
 
   // The network's workspace on this solver's CSR; the learned factor and transposed-slot map go into the device view.
@@ -551,8 +593,10 @@ struct drape_solver {
         CK(cudaLaunchKernelEx(&cfg, dcu::k_solve_rows_learned, d));
       else
         CK(cudaLaunchKernelEx(&cfg, dcu::k_solve<true, 0>, d));
-    } else if (rows) {
+    } else if (rows && residentRowsPerThread == 1) {
       CK(cudaLaunchKernelEx(&cfg, dcu::k_solve_rows, d));
+    } else if (rows) {
+      CK(cudaLaunchKernelEx(&cfg, residentRowsPerThread == 2 ? dcu::k_solve_rows_multi<2> : dcu::k_solve_rows_multi<3>, d));
     } else if (d.P.pcgVariant == 1) {
       CK(cudaLaunchKernelEx(&cfg, dcu::k_solve<false, 1>, d));
     } else if (d.P.pcgVariant == 2) {

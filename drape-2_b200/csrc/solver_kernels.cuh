@@ -117,6 +117,15 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_solve_rows(Dev D) {
   solveGroup<false, kRowLanes, kResidentRows>(D, gs);
 }
 
+// The same for larger scenes: Rows rows a thread, the matrix partly in the L2 (pcgResidentMulti).
+template <int Rows>
+__global__ void __launch_bounds__(kRowThreads, 1) k_solve_rows_multi(Dev D) {
+  if (D.ctl->newtonDone) return;
+  GridSync gs;
+  gs.init(D.ctl, D.P.barrierLimitNs);
+  solveGroup<false, kRowLanes, kResidentRows + Rows - 1>(D, gs);
+}
+
 // The same with the learned preconditioner (pcgLearnedResident; block-Jacobi after a breakdown), for scenes that fit
 // resident rows and solves that start with the learned preconditioner.
 __global__ void __launch_bounds__(kRowThreads, 1) k_solve_rows_learned(Dev D) {

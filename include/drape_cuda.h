@@ -230,7 +230,8 @@ int drape_cuda_set_host_wait(drape_solver* s, uint32_t spin_microseconds);
    stopping tests, cpu_solver.cpp:169-213): 0 (the default) the reference's order, two grid-wide reductions per
    iteration, run over resident rows (one 512-thread block per SM, each row's PCG state in its thread's registers, the
    block's matrix in a sliced layout in shared memory) where every block has at most 480 rows and its sliced matrix, its
-   rows' z and its neighbours' fit in shared memory, else on one 1024-thread block per SM: the two kernels give bit-identical results; 1 pipelined
+   rows' z and its neighbours' fit in shared memory, else up to three rows a thread with the matrix partly in the L2
+   (at most 1440 rows a block), else on one 1024-thread block per SM: the two kernels give bit-identical results; 1 pipelined
    (Ghysels and Vanroose 2014), one reduction per iteration and three more work vectors, its FP32 recurrences drifting
    further from the products they stand for; 2 Chronopoulos-Gear, one reduction and one plain barrier per iteration
    with the reference order's recurrences; 3 the reference's order on the 1024-thread kernel whatever the scene (for
@@ -238,7 +239,7 @@ int drape_cuda_set_host_wait(drape_solver* s, uint32_t spin_microseconds);
    always runs its own PCG. */
 int drape_cuda_set_pcg_variant(drape_solver* s, int variant);
 /* Threads per block of the built scene's solve kernel under the current settings: 512 when the reference-order PCG runs
-   over resident rows, else 1024 (the grid has one block per SM either way). */
+   over resident rows (one or several a thread), else 1024 (the grid has one block per SM either way). */
 int drape_cuda_solve_threads(const drape_solver* s, int* threads);
 
 /* The bounded wait of the device grid barrier, in nanoseconds (0 restores the default of 2 s). A kernel whose barrier

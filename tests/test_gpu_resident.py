@@ -39,6 +39,10 @@ CASES = {
     "pinned_37x37": lambda: _hanging(37),
     "shuffled_60x60": lambda: _shuffled(60, 3),
     "tube_66k": lambda: S.seamed_tube(161, 205, field_n=64, field_cell=0.012),
+    # Several rows a thread, the matrix partly in the L2: the smallest and largest of two rows, and three rows.
+    "tube_72k": lambda: S.seamed_tube(169, 213, field_n=64, field_cell=0.012),
+    "tube_141k": lambda: S.seamed_tube(236, 299, field_n=64, field_cell=0.012),
+    "tube_150k": lambda: S.seamed_tube(243, 309, field_n=64, field_cell=0.012),
 }
 
 
