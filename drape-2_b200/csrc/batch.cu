@@ -28,6 +28,7 @@
 #include "kernels.cuh"
 #include "learned.hpp"
 #include "model.hpp"
+#include "packed_read.cuh"
 
 using drape_b200::Model;
 using dbuf::check;
@@ -482,6 +483,7 @@ struct drape_batch {
   HostPinned<unsigned char> hControl;
   HostPinned<bcu::StatsOut> hStats;
   HostPinned<dcu::Control> hCtl;
+  packed::Reader reader;
   bcu::View view{};
 
   // Learned preconditioner over the whole batch graph (global indices), the factor read per garment.
@@ -519,6 +521,7 @@ struct drape_batch {
     BCK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     hStats.alloc(1);
     hCtl.alloc(1);
+    reader.init();
   }
 
   ~drape_batch() {
@@ -1504,17 +1507,7 @@ int drape_batch_read_positions(const drape_batch* cb, uint32_t index, float* out
     const size_t n = b->models[index].x.size();
     if (count != n || !out) throw std::invalid_argument("readPositions: span size must equal the garment's particle count");
     b->use();
-    std::vector<float4> tmp(n);
-    if (n) {
-      BCK(cudaMemcpyAsync(tmp.data(), b->x.p + b->pBase[index], sizeof(float4) * n, cudaMemcpyDeviceToHost,
-                          b->stream));
-      BCK(cudaStreamSynchronize(b->stream));
-    }
-    for (size_t i = 0; i < n; ++i) {
-      out[3 * i] = tmp[i].x;
-      out[3 * i + 1] = tmp[i].y;
-      out[3 * i + 2] = tmp[i].z;
-    }
+    if (n) b->reader.read(b->x.p + b->pBase[index], n, out, b->stream);
   });
 }
 

@@ -146,7 +146,7 @@ class BatchSolver:
 
     def positions(self, index: int) -> np.ndarray:
         n = self.particle_count(index)
-        out = np.zeros((n, 3), np.float32)
+        out = np.empty((n, 3), np.float32)
         self._check(self.L.drape_batch_read_positions(self.h, index, out.ctypes.data_as(_P(_f)), n))
         return out
 

@@ -14,7 +14,7 @@ LIB = os.path.join(LIB_DIR, "libdrape_cuda.so")
 OBJ_DIR = os.path.join(LIB_DIR, "obj")
 
 SOURCES = ["solver.cu", "batch.cu", "learned.cu", "bake.cu", "model.cpp", "mesher.cpp"]
-HEADERS = ["kernels.cuh", "exchange.cuh", "device_math.cuh", "model.hpp", "learned.hpp", "umma.cuh", "device_model.hpp",
+HEADERS = ["kernels.cuh", "exchange.cuh", "packed_read.cuh", "device_math.cuh", "model.hpp", "learned.hpp", "umma.cuh", "device_model.hpp",
            "device_buffer.hpp", "solver_kernels.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")

@@ -185,7 +185,7 @@ class CudaSolver:
 
     def positions(self) -> np.ndarray:
         n = self.particle_count()
-        out = np.zeros((n, 3), np.float32)
+        out = np.empty((n, 3), np.float32)
         self._check(self.L.drape_cuda_read_positions(self.h, _p(out, _f), n))
         return out
 
@@ -196,7 +196,7 @@ class CudaSolver:
 
     def velocities(self) -> np.ndarray:
         n = self.particle_count()
-        out = np.zeros((n, 3), np.float32)
+        out = np.empty((n, 3), np.float32)
         self._check(self.L.drape_cuda_read_velocities(self.h, _p(out, _f), n))
         return out
 

@@ -86,3 +86,15 @@ def test_resident_learned_pcg_with_a_zero_output_layer_is_block_jacobi(gpu, name
     assert c.learned_solves == c.newton_iterations == 2 and c.precond_fallbacks == 0
     assert np.abs(np.asarray(h) - np.asarray(hj)).max() <= 1, (h, hj)
     assert np.abs(x.astype(np.float64) - xj).max() < 1e-4
+
+
+@pytest.mark.parametrize("side", [3, 128, 129])
+def test_reads_in_chunks_equal_the_snapshot(gpu, side):
+    """Positions and velocities are read through a 16,384-particle staging buffer: below, at and past one chunk they
+    equal the snapshot's, which copies the padded vectors."""
+    s = gpu.CudaSolver(0)
+    s.build(S.sheet_on_sphere(n=side, height=0.16, cg_tolerance=1e-2, max_cg=50))
+    s.step(1.0 / 60.0, 1, 2)
+    snap = s.snapshot()
+    assert np.array_equal(s.positions(), snap["positions"]) and np.array_equal(s.velocities(), snap["velocities"])
+    s.close()
