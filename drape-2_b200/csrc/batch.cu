@@ -45,7 +45,10 @@ struct SegRun {
   int32_t substeps;   // substeps of this frame; 0: the garment does not advance
   int32_t action;     // kActRestore | kActSettle | kActAssemble | kActSave, applied before the substeps
   uint32_t smemSlots; // block slots a solve block of this garment keeps in shared memory
-  uint32_t pad;
+  // The resident-row solve (k_solve_batch_resident): as in dcu::Params, and where the garment's blocks' parts of the
+  // spilled slots (bytes) and halos (entries) begin.
+  uint32_t kept, rows, slots, nodes, spillSlots, haloStride, pad;
+  uint64_t spillAt, haloAt;
 };
 constexpr int32_t kActRestore = 1, kActSettle = 2, kActAssemble = 4, kActSave = 8;
 
@@ -66,6 +69,9 @@ struct View {
   dcu::Garment* snapG;
   float* snapGap;
   StatsOut* stats;              // G
+  uint8_t* spill;               // the resident-row solve's arrays (localCol and mailSeq are in the segment views)
+  uint32_t *halo, *haloCount;
+  dcu::MailWord* mail;
   uint32_t G;
 };
 
@@ -233,6 +239,59 @@ __global__ void __launch_bounds__(Threads, 1024 / Threads) k_solve_batch(View V)
   dcu::GridSync gs;
   gs.init(sD.ctl, sD.P.barrierLimitNs, rank, size);
   dcu::solveGroup<Learned, RL>(sD, gs);
+}
+
+// The same with the reference-order PCG over resident rows (dcu::pcgResidentMulti, the slot-parallel scheme's order of
+// sums): one 512-thread block per SM, a garment's group sized by its rows, up to Rows rows a thread. Against the
+// slot-parallel kernel it reads no row vector and only part of the matrix from the L2 (or HBM), and the garment's sums
+// are exchanged by messages instead of counter barriers.
+template <int Rows>
+__global__ void __launch_bounds__(dcu::kRowThreads, 1) k_solve_batch_resident(View V) {
+  __shared__ dcu::Dev sD;
+  __shared__ uint32_t g, rank, size;
+  if (threadIdx.x == 0) {
+    g = segmentOf(V.solveStart, V.G, blockIdx.x);
+    rank = blockIdx.x - V.solveStart[g];
+    size = V.solveStart[g + 1] - V.solveStart[g];
+  }
+  __syncthreads();
+  if (rank >= size || V.segs[g].ctl->newtonDone) return;  // blocks past the last garment's have none
+  loadSegment(V, g, sD);
+  if (threadIdx.x == 0) {
+    const SegRun& r = V.run[g];
+    const uint32_t first = V.solveStart[g];
+    sD.partials = V.partials + 2ull * first * dcu::kPartialStride;
+    sD.P.multiKept = r.kept;
+    sD.P.multiRows = r.rows;
+    sD.P.residentSlots = r.slots;
+    sD.P.residentNodes = r.nodes;
+    sD.P.spillSlots = r.spillSlots;
+    sD.P.haloStride = r.haloStride;
+    sD.spill = V.spill + r.spillAt;
+    sD.halo = V.halo + r.haloAt;
+    sD.haloCount = V.haloCount + first;
+    sD.mail = V.mail + dcu::mailWords(first);
+  }
+  __syncthreads();
+  dcu::GridSync gs;
+  gs.init(sD.ctl, sD.P.barrierLimitNs, rank, size);
+  dcu::solveGroup<false, 0, dcu::kResidentRows + Rows>(sD, gs);
+}
+
+// The index arrays of every resident-row solve block for the partition in the frame control; Fill false: the halos' sizes
+// only.
+template <bool Fill>
+__global__ void __launch_bounds__(512) k_localize_batch(View V) {
+  __shared__ uint32_t g;
+  if (threadIdx.x == 0) g = segmentOf(V.solveStart, V.G, blockIdx.x);
+  __syncthreads();
+  const uint32_t rank = blockIdx.x - V.solveStart[g], size = V.solveStart[g + 1] - V.solveStart[g];
+  if (rank >= size) return;
+  const dcu::Dev& D = V.segs[g];
+  const SegRun& r = V.run[g];
+  dcu::localizeBlock(D.P.n, rank, size, D.rowStart, D.colIndex, (D.P.n + 31u) / 32u, V.haloCount + blockIdx.x,
+                     Fill ? V.halo + r.haloAt + static_cast<size_t>(rank) * r.haloStride : nullptr,
+                     const_cast<uint16_t*>(D.localCol));
 }
 
 // Assembly clocks of the garments that took substep s.
@@ -479,7 +538,7 @@ struct drape_batch {
   DBuf<bcu::StatsOut> stats;
   DBuf<double> statsPart;         // 8 doubles per point-kernel block
   DBuf<unsigned int> statsDone;   // per garment: blocks of k_stats_batch finished
-  DBuf<unsigned char> control;  // frame control: G SegRun, then G + 1 solve-block starts
+  DBuf<unsigned char> control;  // frame control (controlBytes)
   HostPinned<unsigned char> hControl;
   HostPinned<bcu::StatsOut> hStats;
   HostPinned<dcu::Control> hCtl;
@@ -499,8 +558,24 @@ struct drape_batch {
   std::vector<uint32_t> solveCount;  // current solve partition
   bool tunedByHand = false;
 
+  // The resident-row solve of the default variant's scheme, where the advancing garments fit it (planResident).
+  bool residentOn = false;
+  static constexpr size_t kWaves = 8;   // launches a Newton iteration's solve may take
+  int residentRows = 0, residentWaves = 0;  // rows a thread; launches
+  size_t residentSmem = 0, residentSmemCap = 0;
+  std::vector<uint32_t> residentLive;   // the garments its arrays are built for
+  std::vector<uint32_t> residentStart;  // the waves' block starts, G + 1 each
+  bool residentFits = false;
+  std::vector<bcu::SegRun> residentRun;  // its per-garment fields
+  DBuf<uint16_t> localCol;
+  DBuf<uint32_t> halo, haloCount;
+  DBuf<uint8_t> spill;
+  DBuf<dcu::MailWord> mail;
+  DBuf<unsigned long long> mailSeq;
+
   cudaGraphExec_t graphExec = nullptr;
-  int graphSubsteps = -1, graphIterations = -1, graphVariant = -1, graphLearned = -1;
+  int graphSubsteps = -1, graphIterations = -1, graphVariant = -1, graphLearned = -1, graphRows = -1, graphWaves = -1;
+  size_t graphSmem = 0;
   bool graphUsable = true;
 
   bool profiling = false;
@@ -548,6 +623,8 @@ struct drape_batch {
   }
 
   bcu::SegRun* runs() { return reinterpret_cast<bcu::SegRun*>(hControl.p); }
+  // The frame control: G SegRun, then kWaves times G + 1 solve-block starts (one wave's, except for the resident solve).
+  size_t controlBytes() const { return sizeof(bcu::SegRun) * G + sizeof(uint32_t) * kWaves * (G + 1); }
   uint32_t* solveStartHost() { return reinterpret_cast<uint32_t*>(hControl.p + sizeof(bcu::SegRun) * G); }
 
   void add(const drape_scene_desc& scene) {
@@ -724,9 +801,19 @@ struct drape_batch {
       d.tslot = tslot.p + sBase[g];
       d.cgLog = nullptr;
     }
+    localCol.alloc(B);
+    mailSeq.alloc(G);
+    mail.alloc(kWaves * dcu::mailWords(static_cast<size_t>(numSMs)));
+    haloCount.alloc(kWaves * numSMs);
+    for (uint32_t g = 0; g < G; ++g) {
+      views[g].localCol = localCol.p + sBase[g];
+      views[g].mailSeq = mailSeq.p + g;
+    }
+    view.mail = mail.p;
+    view.haloCount = haloCount.p;
     segs.upload(views, s);
-    control.alloc(sizeof(bcu::SegRun) * G + sizeof(uint32_t) * (G + 1));
-    hControl.alloc(sizeof(bcu::SegRun) * G + sizeof(uint32_t) * (G + 1));
+    control.alloc(controlBytes());
+    hControl.alloc(controlBytes());
     view.segs = segs.p;
     view.run = reinterpret_cast<const bcu::SegRun*>(control.p);
     view.solveStart = reinterpret_cast<const uint32_t*>(control.p + sizeof(bcu::SegRun) * G);
@@ -743,9 +830,24 @@ struct drape_batch {
     view.stats = stats.p;
     view.G = G;
     BCK(cudaStreamSynchronize(s));
+    residentSmemCap = SIZE_MAX;
+    int optin = 0;
+    BCK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+    for (int rows = 1; rows <= dcu::kMultiMost; ++rows) {
+      const void* k = reinterpret_cast<const void*>(residentKernel(rows));
+      cudaFuncAttributes fa{};
+      BCK(cudaFuncGetAttributes(&fa, k));
+      const size_t most = (static_cast<size_t>(optin) - fa.sharedSizeBytes) & ~static_cast<size_t>(15);
+      BCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)));
+      residentSmemCap = std::min(residentSmemCap, most);
+    }
+    for (SolveKernel k : {bcu::k_localize_batch<false>, bcu::k_localize_batch<true>})
+      BCK(cudaFuncSetAttribute(reinterpret_cast<const void*>(k), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               kLocalizeSmem));
     built = true;
     setVariant(variant);
     if (learnedOn) bindNet();
+    planResident(std::vector<int>(G, 1));  // the usual first frame's partition: every garment advances
   }
 
   // ---- solve variant and partition ----
@@ -776,9 +878,173 @@ struct drape_batch {
     solveCount.clear();
   }
 
+  static constexpr int kLocalizeSmem = 64 << 10;
+  static SolveKernel residentKernel(int rows) {
+    return rows == 1 ? bcu::k_solve_batch_resident<1>
+                     : rows == 2 ? bcu::k_solve_batch_resident<2> : bcu::k_solve_batch_resident<3>;
+  }
+
+  // Whether the advancing garments fit the resident-row solve: waves of garments, one launch each, with one block per SM,
+  // at most kMultiMost rows a thread, and for each garment its rows, their contact planes and the halo in shared memory.
+  // As few waves as possible, the largest garments dealt out first; in a wave the blocks are shared out so that the most
+  // rows of any block are as few as possible. Rebuilds the index arrays when the partition changes.
+  //
+  // The rule: the default variant with block-Jacobi, whenever it fits in kWaves launches. Measured (us per Newton
+  // iteration's solve on one B200, k_solve_batch<false, 0, 256> in brackets): 2 garments of 500 particles 165 (571), 5 of
+  // 700-3,000 182 (514), 16 of 2k-40k (175k in all, one wave) 780-960 (1,740), 243k 1,075 (2,650), 394k 2,726 (4,173),
+  // 584k 4,001 (6,249); the fastest of the other variants takes 2,130, 3,403 and 5,124 for the last three.
+  bool planResident(const std::vector<int>& substeps) {
+    if (variant != 0 || (learnedOn && netGraph)) return false;
+    const uint32_t most = dcu::kMultiMost * dcu::kRowWorkers;
+    std::vector<uint32_t> live;
+    for (uint32_t g = 0; g < G; ++g)
+      if (substeps[g] > 0) live.push_back(g);
+    if (live == residentLive) return residentFits;
+    residentLive = live;
+    residentFits = false;
+    if (live.empty()) return false;
+    auto rows = [&](uint32_t g) { return static_cast<uint32_t>(models[g].x.size()); };
+    std::stable_sort(live.begin(), live.end(), [&](uint32_t a, uint32_t b) { return rows(a) > rows(b); });
+    auto blocksAt = [&](const std::vector<uint32_t>& of, uint32_t perBlock) {
+      uint64_t total = 0;
+      for (uint32_t g : of) total += (rows(g) + perBlock - 1) / perBlock;
+      return total;
+    };
+    std::vector<std::vector<uint32_t>> wave;
+    for (size_t W = 1; W <= kWaves && wave.empty(); ++W) {
+      std::vector<std::vector<uint32_t>> w(W);
+      std::vector<uint64_t> load(W, 0);
+      for (uint32_t g : live) {
+        const size_t k = std::min_element(load.begin(), load.end()) - load.begin();
+        w[k].push_back(g);
+        load[k] += rows(g);
+      }
+      bool fits = true;
+      for (const auto& of : w) fits = fits && blocksAt(of, most) <= static_cast<uint64_t>(numSMs);
+      if (fits) wave = std::move(w);
+    }
+    if (wave.empty()) return false;
+    residentWaves = static_cast<int>(wave.size());
+    residentRun.assign(G, bcu::SegRun{});
+    residentStart.assign(static_cast<size_t>(residentWaves) * (G + 1), 0);
+    std::vector<uint32_t> count(G, 0);
+    for (int k = 0; k < residentWaves; ++k) {
+      uint32_t lo = 32, hi = most;  // fewest rows a block with which the wave fits
+      while (lo < hi) {
+        const uint32_t mid = (lo + hi) / 2;
+        if (blocksAt(wave[k], mid) <= static_cast<uint64_t>(numSMs)) hi = mid; else lo = mid + 1;
+      }
+      std::vector<uint32_t> c(G, 0);
+      for (uint32_t g : wave[k]) c[g] = count[g] = (rows(g) + hi - 1) / hi;
+      const auto start = prefix(c);
+      std::copy(start.begin(), start.end(), residentStart.begin() + static_cast<size_t>(k) * (G + 1));
+    }
+    std::copy(residentStart.begin(), residentStart.end(), solveStartHost());
+    // The halos' sizes for this partition.
+    size_t words = 0;
+    for (uint32_t g = 0; g < G; ++g) words = std::max<size_t>(words, (rows(g) + 31) / 32);
+    const size_t bitmap = 2 * sizeof(uint32_t) * words;
+    if (bitmap > static_cast<size_t>(kLocalizeSmem)) return false;
+    auto uploadControl = [&] {
+      BCK(cudaMemcpyAsync(control.p, hControl.p, controlBytes(), cudaMemcpyHostToDevice, stream));
+    };
+    uploadControl();
+    for (int k = 0; k < residentWaves; ++k) bcu::k_localize_batch<false><<<numSMs, 512, bitmap, stream>>>(waveView(k));
+    BCK(cudaGetLastError());
+    std::vector<uint32_t> halos(static_cast<size_t>(numSMs) * residentWaves);
+    BCK(cudaMemcpyAsync(halos.data(), haloCount.p, sizeof(uint32_t) * halos.size(), cudaMemcpyDeviceToHost, stream));
+    BCK(cudaStreamSynchronize(stream));
+    uint64_t spillMost = 0, haloEntries = 0;
+    size_t smem = 0;
+    uint32_t mostRows = 0;
+    for (int k = 0; k < residentWaves; ++k) {
+      uint64_t spillBytes = 0;  // the waves use the spill buffer one after the other
+      for (uint32_t g : wave[k]) {
+        const Model& m = models[g];
+        bcu::SegRun& r = residentRun[g];
+        r.rows = (rows(g) + count[g] - 1) / count[g];
+        const uint32_t first = residentStart[static_cast<size_t>(k) * (G + 1) + g];
+        for (uint32_t b = first; b < first + count[g]; ++b)
+          r.haloStride = std::max(r.haloStride, halos[static_cast<size_t>(k) * numSMs + b]);
+        r.nodes = r.rows + r.haloStride + 1;
+        if (r.nodes >= dcu::kNoColumn) return false;
+        const size_t fixed =
+            static_cast<size_t>(r.nodes) * dcu::kResidentNodeBytes + sizeof(float4) * static_cast<size_t>(r.rows);
+        auto bytes = [&](uint32_t slots) {
+          return fixed + (static_cast<size_t>(slots) * dcu::kResidentSlotBytes + 15) / 16 * 16;
+        };
+        if (fixed > residentSmemCap) return false;
+        const dmodel::WarpLengths lengths(m, static_cast<int>(count[g]));
+        for (uint32_t q = 2; q <= 64 && bytes(lengths.most(0, q)) <= residentSmemCap; q += 2) r.kept = q;
+        r.slots = lengths.most(0, r.kept);
+        r.spillSlots = lengths.most(r.kept, UINT32_MAX);
+        r.spillAt = spillBytes;
+        r.haloAt = haloEntries;
+        spillBytes += static_cast<uint64_t>(r.spillSlots) * dcu::kResidentSlotBytes * count[g];
+        haloEntries += static_cast<uint64_t>(r.haloStride) * count[g];
+        smem = std::max(smem, bytes(r.slots));
+        mostRows = std::max(mostRows, r.rows);
+      }
+      spillMost = std::max(spillMost, spillBytes);
+    }
+    if (spillMost > spill.n || !spill.p) {
+      dropGraph();
+      spill.alloc(std::max<uint64_t>(spillMost, 16));
+      view.spill = spill.p;
+    }
+    if (haloEntries > halo.n || !halo.p) {
+      dropGraph();
+      halo.alloc(std::max<uint64_t>(haloEntries, 1));
+      view.halo = halo.p;
+    }
+    residentRows = static_cast<int>((mostRows + dcu::kRowWorkers - 1) / dcu::kRowWorkers);
+    residentSmem = smem;
+    writeResident();
+    uploadControl();
+    for (int k = 0; k < residentWaves; ++k) bcu::k_localize_batch<true><<<numSMs, 512, bitmap, stream>>>(waveView(k));
+    BCK(cudaGetLastError());
+    // The garments' parts of the mailbox move: no word left from another garment's exchanges may look like a message.
+    BCK(cudaMemsetAsync(mail.p, 0, sizeof(dcu::MailWord) * mail.n, stream));
+    BCK(cudaStreamSynchronize(stream));
+    residentFits = true;
+    return true;
+  }
+
+  // The view of a wave's launch: its block starts, mailbox and halo sizes.
+  bcu::View waveView(int k) const {
+    bcu::View v = view;
+    v.solveStart += static_cast<size_t>(k) * (G + 1);
+    v.mail += static_cast<size_t>(k) * dcu::mailWords(static_cast<size_t>(numSMs));
+    v.haloCount += static_cast<size_t>(k) * numSMs;
+    return v;
+  }
+
+  // The resident-row solve's part of the frame control.
+  void writeResident() {
+    std::copy(residentStart.begin(), residentStart.end(), solveStartHost());
+    for (uint32_t g = 0; g < G; ++g) {
+      bcu::SegRun& r = runs()[g];
+      const bcu::SegRun& q = residentRun[g];
+      r.smemSlots = 0;
+      r.kept = q.kept;
+      r.rows = q.rows;
+      r.slots = q.slots;
+      r.nodes = q.nodes;
+      r.spillSlots = q.spillSlots;
+      r.haloStride = q.haloStride;
+      r.spillAt = q.spillAt;
+      r.haloAt = q.haloAt;
+    }
+  }
+
   // Solve blocks for the advancing garments (substeps > 0 this frame); writes the starts and smem slot caps into the
   // frame control.
   void partition(const std::vector<int>& substeps) {
+    residentOn = planResident(substeps);
+    if (residentOn) {
+      writeResident();
+      return;
+    }
     std::vector<double> w(G, 0.0);
     for (uint32_t g = 0; g < G; ++g)
       if (substeps[g] > 0) w[g] = static_cast<double>(models[g].colIndex.size()) + 5.0 * models[g].x.size();
@@ -861,11 +1127,11 @@ struct drape_batch {
 
   void launchSolve(bool timed) {
     const Variant& V = kVariants[variant];
-    SolveKernel k = learnedOn && netGraph ? V.learned : V.jacobi;
+    SolveKernel k = residentOn ? residentKernel(residentRows) : learnedOn && netGraph ? V.learned : V.jacobi;
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(solveBlocks);
-    cfg.blockDim = dim3(V.threads);
-    cfg.dynamicSmemBytes = solveSmem;
+    cfg.gridDim = dim3(residentOn ? numSMs : solveBlocks);
+    cfg.blockDim = dim3(residentOn ? dcu::kRowThreads : V.threads);
+    cfg.dynamicSmemBytes = residentOn ? residentSmem : solveSmem;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -877,7 +1143,8 @@ struct drape_batch {
       a = takeEvent();
       BCK(cudaEventRecord(a, stream));
     }
-    BCK(cudaLaunchKernelEx(&cfg, k, view));
+    for (int w = 0; w < (residentOn ? residentWaves : 1); ++w)
+      BCK(cudaLaunchKernelEx(&cfg, k, residentOn ? waveView(w) : view));
     if (timed) {
       cudaEvent_t b = takeEvent();
       BCK(cudaEventRecord(b, stream));
@@ -888,8 +1155,7 @@ struct drape_batch {
   // Enqueues one frame: per-garment control upload, actions, substeps x (activation, assembly, [network], solve),
   // finish and clocks, statistics, control-block and statistics download. Returns the kernels it launched.
   int enqueueFrame(int maxSubsteps, int iterations, bool timed) {
-    const size_t ctlBytes = sizeof(bcu::SegRun) * G + sizeof(uint32_t) * (G + 1);
-    BCK(cudaMemcpyAsync(control.p, hControl.p, ctlBytes, cudaMemcpyHostToDevice, stream));
+    BCK(cudaMemcpyAsync(control.p, hControl.p, controlBytes(), cudaMemcpyHostToDevice, stream));
     int launches = 0;
     const uint32_t pointGrid = [&] { uint32_t t = 0; for (auto c : pointCount) t += c; return t; }();
     const uint32_t asmGrid = [&] { uint32_t t = 0; for (auto c : asmCount) t += c; return t; }();
@@ -909,7 +1175,7 @@ struct drape_batch {
           launches += 8;
         }
         launchSolve(timed);
-        ++launches;
+        launches += residentOn ? residentWaves : 1;
       }
       bcu::k_points<2><<<pointGrid, kPointThreads, 0, stream>>>(view, s);
       bcu::k_clock_batch<<<(G + 127) / 128, 128, 0, stream>>>(view, s);
@@ -939,7 +1205,10 @@ struct drape_batch {
       prof.solve_launches += maxSub * iterations;
     } else {
       if (graphUsable && (!graphExec || graphSubsteps != maxSub || graphIterations != iterations ||
-                          graphVariant != variant || graphLearned != static_cast<int>(learned))) {
+                          graphVariant != variant || graphLearned != static_cast<int>(learned) ||
+                          graphRows != (residentOn ? residentRows : 0) ||
+                          graphWaves != (residentOn ? residentWaves : 0) ||
+                          graphSmem != (residentOn ? residentSmem : 0))) {
         dropGraph();
         capture(maxSub, iterations);
       }
@@ -992,6 +1261,9 @@ struct drape_batch {
     graphIterations = iterations;
     graphVariant = variant;
     graphLearned = learnedOn && netGraph ? 1 : 0;
+    graphRows = residentOn ? residentRows : 0;
+    graphWaves = residentOn ? residentWaves : 0;
+    graphSmem = residentOn ? residentSmem : 0;
     graphLaunchesPerFrame = launches;
   }
   int graphLaunchesPerFrame = 0;
@@ -1023,6 +1295,11 @@ struct drape_batch {
       x.barrierArrivals = 0;
     }
     BCK(cudaMemcpy(ctl.p, c.data(), sizeof(dcu::Control) * G, cudaMemcpyHostToDevice));
+    // As for a single solver: go on with exchange numbers that no block of an abandoned solve reached.
+    std::vector<unsigned long long> seq(G);
+    BCK(cudaMemcpy(seq.data(), mailSeq.p, sizeof(unsigned long long) * G, cudaMemcpyDeviceToHost));
+    for (auto& q : seq) q += 1ull << 24;
+    BCK(cudaMemcpy(mailSeq.p, seq.data(), sizeof(unsigned long long) * G, cudaMemcpyHostToDevice));
   }
 
   void setRun(uint32_t g, double dt, int substeps, int32_t action) {
@@ -1219,7 +1496,7 @@ struct drape_batch {
     drape_batch_tuning t{};
     t.row_lanes = kVariants[variant].rowLanes;
     t.block_threads = kVariants[variant].threads;
-    t.blocks = solveBlocks;
+    t.blocks = residentOn ? numSMs : solveBlocks;
     return t;
   }
 

@@ -423,6 +423,10 @@ __device__ __forceinline__ float3 axpyRn(float3 x, float s, float3 y) {  // y + 
 __device__ __forceinline__ float dotRn(float a0, float a1, float a2, float3 b) {
   return __fmaf_rn(a2, b.z, __fmaf_rn(a1, b.y, __fmul_rn(a0, b.x)));
 }
+// The same three products with the first two's sum fused into the first.
+__device__ __forceinline__ float dotYRn(float a0, float a1, float a2, float3 b) {
+  return __fmaf_rn(a2, b.z, __fmaf_rn(a0, b.x, __fmul_rn(a1, b.y)));
+}
 __device__ __forceinline__ float3 mulRn(const M3& a, float3 v) {
   return mk(dotRn(a.m[0], a.m[1], a.m[2], v), dotRn(a.m[3], a.m[4], a.m[5], v), dotRn(a.m[6], a.m[7], a.m[8], v));
 }
@@ -1040,7 +1044,7 @@ __device__ inline int pcgReferenceOrder(const Dev& D, GridSync& gs, const SmemMa
 // (4.30-4.32).
 constexpr int kRowThreads = 512;    // k_solve_rows block size
 constexpr int kRowWorkers = 480;    // of these, the threads that own a row each; the last warp does the exchanges
-constexpr int kResidentRows = 4;    // the solve templates' Variant value of this form; 4 + m: m + 1 rows a thread
+constexpr int kResidentRows = 4;    // the solve templates' Variant value of this form; 4 + m: m rows a thread
 constexpr int kRegSlots = 2;        // slots of each row kept in registers (even, so that slot parity is the same)
 constexpr int kExchangeDelay = 700; // clock cycles before an exchange's first poll, to begin with
 constexpr uint32_t kNoColumn = 0xFFFFu;  // localCol of a pinned column
@@ -1402,6 +1406,70 @@ __device__ inline int pcgResident(const Dev& D, GridSync& gs, ResidentMatrix& A,
   return code == 2 ? -1 : it;
 }
 
+// Index arrays of one solve block (blocks of at most 512 threads): its halo (the particles of other blocks its unpinned rows
+// couple to, in particle order) and every slot's column as an index among the block's rows and halo (kNoColumn for pinned
+// columns). The particles met are marked in a bitmap in shared memory (`words` words, and their running counts). With
+// `halo` null only the count is written.
+__device__ inline void localizeBlock(uint32_t n, uint32_t rank, uint32_t size, const uint32_t* __restrict__ rowStart,
+                                     const uint32_t* __restrict__ colIndex, uint32_t words,
+                                     uint32_t* __restrict__ haloCount, uint32_t* __restrict__ halo,
+                                     uint16_t* __restrict__ localCol) {
+  uint32_t* bits = reinterpret_cast<uint32_t*>(solveSmem);
+  uint32_t* before = bits + words;  // bits set in the words before
+  __shared__ uint32_t warpTotal[17];
+  const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5;
+  uint32_t r0, r1;
+  blockRange(n, rank, size, r0, r1);
+  const uint32_t s0 = rowStart[r0], s1 = rowStart[r1];
+  for (uint32_t k = t; k < words; k += blockDim.x) bits[k] = 0u;
+  __syncthreads();
+  for (uint32_t s = s0 + t; s < s1; s += blockDim.x) {
+    const uint32_t c = colIndex[s];
+    if (!(c & kPinnedBit) && (c < r0 || c >= r1)) atomicOr(bits + (c >> 5), 1u << (c & 31u));
+  }
+  __syncthreads();
+  uint32_t base = 0;
+  for (uint32_t k0 = 0; k0 < words; k0 += blockDim.x) {
+    const uint32_t k = k0 + t;
+    const uint32_t mine = k < words ? __popc(bits[k]) : 0u;
+    uint32_t sum = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, sum, o);
+      if (lane >= static_cast<uint32_t>(o)) sum += y;
+    }
+    if (lane == 31) warpTotal[w] = sum;
+    __syncthreads();
+    if (t == 0) {
+      uint32_t acc = 0;
+      for (uint32_t q = 0; q < blockDim.x / 32; ++q) {
+        const uint32_t x = warpTotal[q];
+        warpTotal[q] = acc;
+        acc += x;
+      }
+      warpTotal[16] = acc;
+    }
+    __syncthreads();
+    if (k < words) before[k] = base + warpTotal[w] + sum - mine;
+    base += warpTotal[16];
+    __syncthreads();
+  }
+  if (t == 0) *haloCount = base;
+  if (!halo) return;
+  for (uint32_t k = t; k < words; k += blockDim.x) {
+    uint32_t at = before[k];
+    for (uint32_t m = bits[k]; m; m &= m - 1) halo[at++] = 32 * k + __ffs(m) - 1;
+  }
+  for (uint32_t s = s0 + t; s < s1; s += blockDim.x) {
+    const uint32_t c = colIndex[s];
+    uint32_t local = kNoColumn;
+    if (!(c & kPinnedBit))
+      local = c >= r0 && c < r1 ? c - r0
+                                : r1 - r0 + before[c >> 5] + __popc(bits[c >> 5] & ((1u << (c & 31u)) - 1u));
+    localCol[s] = static_cast<uint16_t>(local);
+  }
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // The same PCG for scenes with more rows than k_solve_rows has threads for, or more matrix than its shared memory holds
 // (k_solve_rows_multi): each row thread owns Rows rows of its block (rows 32 (w + 15 m) + lane for m < Rows, so slice
@@ -1555,7 +1623,7 @@ __device__ inline bool stageMulti(const Dev& D, uint32_t rank, uint32_t r0, uint
 }
 
 // U slots (U even) of a slice from slot k on, kept (shared memory) or not (L2): all their loads before the first product.
-template <int U, bool Kept>
+template <int U, bool Kept, bool Sequential>
 __device__ __forceinline__ void multiSlots(const MultiMatrix& A, uint32_t base, uint32_t k, float3 (&acc)[2]) {
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t cc[U / 2];
@@ -1578,24 +1646,33 @@ __device__ __forceinline__ void multiSlots(const MultiMatrix& A, uint32_t base, 
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     const float m[9] = {a[u].x, a[u].y, a[u].z, a[u].w, b[u].x, b[u].y, b[u].z, b[u].w, c[u]};
-    blockMulAddRn(acc[u & 1], m, xyz(x[u]));
+    if (Sequential) {
+      acc[0].x = __fadd_rn(acc[0].x, dotYRn(m[0], m[1], m[2], xyz(x[u])));
+      acc[0].y = __fadd_rn(acc[0].y, dotYRn(m[3], m[4], m[5], xyz(x[u])));
+      acc[0].z = __fadd_rn(acc[0].z, dotYRn(m[6], m[7], m[8], xyz(x[u])));
+    } else {
+      blockMulAddRn(acc[u & 1], m, xyz(x[u]));
+    }
   }
 }
 
-// A z for this thread's row of a slice, in residentProduct's order (multiKept is even, so slot parity is kept).
+// A z for this thread's row of a slice, in residentProduct's order (multiKept is even, so slot parity is kept), or
+// Sequential in the slot-parallel scheme's (directionProducts<0>): all slots in one sum.
+template <bool Sequential>
 __device__ __forceinline__ float3 multiProduct(const MultiMatrix& A, const MultiSlices& sl, uint32_t slice) {
   float3 acc[2] = {mk(0, 0, 0), mk(0, 0, 0)};
   const uint32_t kept = sl.keptLen[slice], spill = sl.spillLen[slice];
   uint32_t k = 0;
-  for (; k + 4 <= kept; k += 4) multiSlots<4, true>(A, sl.kept[slice], k, acc);
-  if (k < kept) multiSlots<2, true>(A, sl.kept[slice], k, acc);
+  for (; k + 4 <= kept; k += 4) multiSlots<4, true, Sequential>(A, sl.kept[slice], k, acc);
+  if (k < kept) multiSlots<2, true, Sequential>(A, sl.kept[slice], k, acc);
   k = 0;
-  for (; k + 4 <= spill; k += 4) multiSlots<4, false>(A, sl.spill[slice], k, acc);
-  if (k < spill) multiSlots<2, false>(A, sl.spill[slice], k, acc);
+  for (; k + 4 <= spill; k += 4) multiSlots<4, false, Sequential>(A, sl.spill[slice], k, acc);
+  if (k < spill) multiSlots<2, false, Sequential>(A, sl.spill[slice], k, acc);
+  if (Sequential) return acc[0];
   return mk(__fadd_rn(acc[0].x, acc[1].x), __fadd_rn(acc[0].y, acc[1].y), __fadd_rn(acc[0].z, acc[1].z));
 }
 
-template <int Rows>
+template <int Rows, bool Sequential>
 __device__ inline int pcgResidentMulti(const Dev& D, GridSync& gs, const MultiMatrix& A, const MultiSlices& sl,
                                        unsigned long long& seq) {
   constexpr int kWarps = kRowWorkers / 32;
@@ -1652,7 +1729,7 @@ __device__ inline int pcgResidentMulti(const Dev& D, GridSync& gs, const MultiMa
 #pragma unroll
       for (int m = 0; m < Rows; ++m) {
         const bool busy = 32u * (w + kWarps * m) < R;
-        const float3 az = busy ? multiProduct(A, sl, w + kWarps * m) : mk(0, 0, 0);
+        const float3 az = busy ? multiProduct<Sequential>(A, sl, w + kWarps * m) : mk(0, 0, 0);
         if (m == 0) {
           namedSync<3>(kRowThreads);
           code = sh.code;
@@ -1715,11 +1792,8 @@ constexpr int kLearnedDepth = 3;  // slots whose factor blocks a row thread has 
 
 // acc += B x (Upper: B^T x) for this thread's row over its slots [k0, k1) (slot k is global slot rs + k; the columns are
 // sorted, so the lower part j <= i is [0, kd] and the upper part j >= i is [kd, end) with kd the diagonal's position).
-// The learned PCG's dot product and contact filter, with every rounding written out, so that its iterates do not depend
-// on how the compiler contracts the code around them (the first two products' sum fused into the first).
-__device__ __forceinline__ float dotYRn(float a0, float a1, float a2, float3 b) {
-  return __fmaf_rn(a2, b.z, __fmaf_rn(a0, b.x, __fmul_rn(a1, b.y)));
-}
+// The learned PCG's contact filter, with every rounding written out, so that its iterates do not depend on how the
+// compiler contracts the code around it.
 __device__ __forceinline__ float3 filterYRn(const Contact& c, float3 v) {
   if (c.active == 0u) return v;
   const float3 n = xyz(c.normal);
@@ -2281,13 +2355,13 @@ __device__ inline int pcgSolve(const Dev& D, GridSync& gs) {
   uint32_t r0i, r1i;
   blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
   if constexpr (Variant > kResidentRows) {
-    constexpr int kRows = Variant - kResidentRows + 1;
+    constexpr int kRows = Variant - kResidentRows;
     __shared__ MultiSlices sl;
     MultiMatrix A;
     if (!stageMulti<kRows>(D, gs.rank, r0i, r1i, A, sl)) return -1;
     const unsigned long long t0 = globalTimerNs();
     unsigned long long seq = __ldcg(D.mailSeq);
-    const int it = pcgResidentMulti<kRows>(D, gs, A, sl, seq);
+    const int it = pcgResidentMulti<kRows, PL == 0>(D, gs, A, sl, seq);
     if (gs.rank == 0 && threadIdx.x == 0) {
       *D.mailSeq = seq;
       D.ctl->pcgNs += static_cast<long long>(globalTimerNs() - t0);

@@ -54,37 +54,6 @@ static uint32_t maxBlockSlots(const uint32_t* rowStart, uint32_t n, int grid) {
   return most;
 }
 
-// The resident-row kernels' layout of a scene: for each solve block its rows in warps of 32, and for each warp the slots of
-// its longest unpinned row, to which they are padded (every block has the same number of entries).
-struct WarpLengths {
-  uint32_t perBlock = 0;
-  std::vector<uint32_t> len;
-  WarpLengths(const Model& m, int grid) {
-    const uint32_t n = static_cast<uint32_t>(m.x.size());
-    const uint32_t per = (n + static_cast<uint32_t>(grid) - 1) / static_cast<uint32_t>(grid);
-    perBlock = (per + 31) / 32;
-    len.assign(static_cast<size_t>(perBlock) * grid, 0);
-    for (int b = 0; b < grid; ++b) {
-      const uint32_t r0 = std::min<uint32_t>(n, static_cast<uint32_t>(b) * per), r1 = std::min<uint32_t>(n, r0 + per);
-      for (uint32_t i = r0; i < r1; ++i) {
-        uint32_t& l = len[static_cast<size_t>(b) * perBlock + (i - r0) / 32];
-        if (!m.pinned[i]) l = std::max(l, m.rowStart[i + 1] - m.rowStart[i]);
-      }
-    }
-  }
-  // The most padded slots of a block beyond the first `skip` of each row and within the first `keep` of the rest.
-  uint32_t most(uint32_t skip, uint32_t keep) const {
-    uint32_t out = 0;
-    for (size_t b = 0; b < len.size(); b += perBlock) {
-      uint32_t total = 0;
-      for (uint32_t k = 0; k < perBlock; ++k)
-        if (len[b + k] > skip) total += 32 * std::min(keep, (len[b + k] - skip + 1) & ~1u);
-      out = std::max(out, total);
-    }
-    return out;
-  }
-};
-
 struct drape_solver {
   int device = 0;
   int numSMs = 0;
@@ -416,7 +385,7 @@ struct drape_solver {
     auto slotBytes = [](uint32_t slots) {
       return (static_cast<size_t>(slots) * dcu::kResidentSlotBytes + 15) / 16 * 16;
     };
-    const WarpLengths lengths(m, solveGrid);
+    const dmodel::WarpLengths lengths(m, solveGrid);
     const uint32_t whole = lengths.most(dcu::kRegSlots, UINT32_MAX);
     if (per <= static_cast<uint32_t>(dcu::kRowWorkers) && slotBytes(whole) + nodeBytes <= residentSmemCap[0]) {
       residentRowsPerThread = 1;

@@ -43,68 +43,13 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_solve(Dev D) {
   solveGroup<Learned, kRowLanes, Variant>(D, gs);
 }
 
-// Per build: the halo of each solve block (the particles of other blocks its unpinned rows couple to, in particle order)
-// and every slot's column as an index among the block's rows and halo (kNoColumn for pinned columns). One block per
-// solve block; the particles met are marked in a bitmap in shared memory (`words` words, and their running counts).
-// With `halo` null only the counts are written.
+// Per build, one block per solve block (localizeBlock).
 __global__ void __launch_bounds__(512) k_localize(uint32_t n, uint32_t solveBlocks, const uint32_t* __restrict__ rowStart,
                                                   const uint32_t* __restrict__ colIndex, uint32_t words,
                                                   uint32_t* __restrict__ haloCount, uint32_t haloStride,
                                                   uint32_t* __restrict__ halo, uint16_t* __restrict__ localCol) {
-  uint32_t* bits = reinterpret_cast<uint32_t*>(solveSmem);
-  uint32_t* before = bits + words;  // bits set in the words before
-  __shared__ uint32_t warpTotal[17];
-  const uint32_t t = threadIdx.x, lane = t & 31u, w = t >> 5;
-  uint32_t r0, r1;
-  blockRange(n, blockIdx.x, solveBlocks, r0, r1);
-  const uint32_t s0 = rowStart[r0], s1 = rowStart[r1];
-  for (uint32_t k = t; k < words; k += blockDim.x) bits[k] = 0u;
-  __syncthreads();
-  for (uint32_t s = s0 + t; s < s1; s += blockDim.x) {
-    const uint32_t c = colIndex[s];
-    if (!(c & kPinnedBit) && (c < r0 || c >= r1)) atomicOr(bits + (c >> 5), 1u << (c & 31u));
-  }
-  __syncthreads();
-  uint32_t base = 0;
-  for (uint32_t k0 = 0; k0 < words; k0 += blockDim.x) {
-    const uint32_t k = k0 + t;
-    const uint32_t mine = k < words ? __popc(bits[k]) : 0u;
-    uint32_t sum = mine;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const uint32_t y = __shfl_up_sync(0xffffffffu, sum, o);
-      if (lane >= static_cast<uint32_t>(o)) sum += y;
-    }
-    if (lane == 31) warpTotal[w] = sum;
-    __syncthreads();
-    if (t == 0) {
-      uint32_t acc = 0;
-      for (uint32_t q = 0; q < blockDim.x / 32; ++q) {
-        const uint32_t x = warpTotal[q];
-        warpTotal[q] = acc;
-        acc += x;
-      }
-      warpTotal[16] = acc;
-    }
-    __syncthreads();
-    if (k < words) before[k] = base + warpTotal[w] + sum - mine;
-    base += warpTotal[16];
-    __syncthreads();
-  }
-  if (t == 0) haloCount[blockIdx.x] = base;
-  if (!halo) return;
-  for (uint32_t k = t; k < words; k += blockDim.x) {
-    uint32_t at = before[k];
-    for (uint32_t m = bits[k]; m; m &= m - 1) halo[static_cast<size_t>(blockIdx.x) * haloStride + at++] = 32 * k + __ffs(m) - 1;
-  }
-  for (uint32_t s = s0 + t; s < s1; s += blockDim.x) {
-    const uint32_t c = colIndex[s];
-    uint32_t local = kNoColumn;
-    if (!(c & kPinnedBit))
-      local = c >= r0 && c < r1 ? c - r0
-                                : r1 - r0 + before[c >> 5] + __popc(bits[c >> 5] & ((1u << (c & 31u)) - 1u));
-    localCol[s] = static_cast<uint16_t>(local);
-  }
+  localizeBlock(n, blockIdx.x, solveBlocks, rowStart, colIndex, words, haloCount + blockIdx.x,
+                halo ? halo + static_cast<size_t>(blockIdx.x) * haloStride : nullptr, localCol);
 }
 
 // The same Newton iteration with the reference-order PCG over resident rows (pcgResidentRows): 512-thread blocks, so a
@@ -123,7 +68,7 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_solve_rows_multi(Dev D) {
   if (D.ctl->newtonDone) return;
   GridSync gs;
   gs.init(D.ctl, D.P.barrierLimitNs);
-  solveGroup<false, kRowLanes, kResidentRows + Rows - 1>(D, gs);
+  solveGroup<false, kRowLanes, kResidentRows + Rows>(D, gs);
 }
 
 // The same with the learned preconditioner (pcgLearnedResident; block-Jacobi after a breakdown), for scenes that fit

@@ -45,7 +45,9 @@ int drape_batch_set_precond(drape_batch* b, drape_precond* p);
 
 typedef struct drape_batch_tuning {
   int32_t row_lanes;      /* the PCG's product A p: 0 = slot-parallel (each thread a run of consecutive block
-                             slots, row sums through shared memory), or 2, 4, 8 lanes per block row (also the lanes of
+                             slots, row sums through shared memory; with block_threads 256, the default, and
+                             block-Jacobi the garments that fit run the same sums over resident rows, one 512-thread
+                             block per SM), or 2, 4, 8 lanes per block row (also the lanes of
                              the learned factor's products; 4 with slot-parallel) */
   int32_t block_threads;  /* threads per block of the solve launch: 256, 512 or 1024 (1024 / this blocks per SM) */
   int32_t blocks;         /* blocks of the solve launch */

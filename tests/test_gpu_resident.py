@@ -98,3 +98,56 @@ def test_reads_in_chunks_equal_the_snapshot(gpu, side):
     snap = s.snapshot()
     assert np.array_equal(s.positions(), snap["positions"]) and np.array_equal(s.velocities(), snap["velocities"])
     s.close()
+
+
+def _batch(gpu, sizes, tuning=None, frames=2):
+    from drape_b200 import batch
+    b = batch.BatchSolver(0)
+    for k, n in enumerate(sizes):
+        b.add(S.tube_variant(40 + k, n, field_n=32))
+    b.build()
+    if tuning:
+        b.set_tuning(*tuning)
+    for _ in range(frames):
+        b.step(1.0 / 60.0, 1, 2)
+    out = [b.positions(k) for k in range(len(sizes))], [b.counters(k).cg_iterations for k in range(len(sizes))]
+    b.close()
+    return out
+
+
+@pytest.mark.parametrize("sizes", [(64,), (300, 5000), (900, 700, 2100, 500), (30000,) * 6 + (2000,), (40000,) * 6],
+                         ids=["tiny", "two", "four", "one_wave_182k", "two_waves_240k"])
+def test_resident_batch_matches_the_slot_parallel_kernel(gpu, sizes):
+    """The batch's resident-row solve (the default variant) against the slot-parallel kernel on 512-thread blocks, whose
+    row sums it repeats in the same order: bit-identical positions and the same PCG counts, with one to three rows a
+    thread and one or two launches."""
+    xa, ca = _batch(gpu, sizes)
+    xb, cb = _batch(gpu, sizes, (0, 512))
+    assert ca == cb
+    for a, b in zip(xa, xb):
+        assert np.isfinite(a).all() and np.array_equal(a, b), np.abs(a - b).max()
+
+
+def test_resident_batch_after_the_partition_changes(gpu):
+    """Garments that end their drape leave the frame and the others' groups, halos and mailboxes move: the drape's end
+    state equals the slot-parallel kernel's."""
+    from drape_b200 import batch
+    from drape_b200.scene import drape_drape_options
+    out = []
+    for tuning in (None, (0, 512)):
+        b = batch.BatchSolver(0)
+        for k, n in enumerate((600, 3000, 1200)):
+            b.add(S.tube_variant(60 + k, n, field_n=32))
+        b.build()
+        if tuning:
+            b.set_tuning(*tuning)
+        o = drape_drape_options(substeps=1, iterations=2, frame_dt=1.0 / 60.0, max_assembly_seconds=0.05,
+                                seam_gap_done=0.001, settle_rms_speed=0.5, settle_hold_frames=3, max_sim_seconds=0.4,
+                                snapshot_every=30, max_retries=3, energy_rise_frames=60, frames_per_wait=10)
+        res, _ = b.drape_to_rest(o)
+        out.append(([b.positions(k) for k in range(3)], [int(r.frames_run) for r in res]))
+        b.close()
+    (xa, fa), (xb, fb) = out
+    assert fa == fb and len(set(fa)) > 1, fa
+    for a, b in zip(xa, xb):
+        assert np.array_equal(a, b), np.abs(a - b).max()
