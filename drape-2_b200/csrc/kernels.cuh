@@ -1409,11 +1409,11 @@ __device__ inline int pcgResident(const Dev& D, GridSync& gs, ResidentMatrix& A,
 // Index arrays of one solve block (blocks of at most 512 threads): its halo (the particles of other blocks its unpinned rows
 // couple to, in particle order) and every slot's column as an index among the block's rows and halo (kNoColumn for pinned
 // columns). The particles met are marked in a bitmap in shared memory (`words` words, and their running counts). With
-// `halo` null only the count is written.
+// `halo` null, or a halo of more than `limit`, only the count is written.
 __device__ inline void localizeBlock(uint32_t n, uint32_t rank, uint32_t size, const uint32_t* __restrict__ rowStart,
                                      const uint32_t* __restrict__ colIndex, uint32_t words,
                                      uint32_t* __restrict__ haloCount, uint32_t* __restrict__ halo,
-                                     uint16_t* __restrict__ localCol) {
+                                     uint16_t* __restrict__ localCol, uint32_t limit = UINT32_MAX) {
   uint32_t* bits = reinterpret_cast<uint32_t*>(solveSmem);
   uint32_t* before = bits + words;  // bits set in the words before
   __shared__ uint32_t warpTotal[17];
@@ -1455,7 +1455,7 @@ __device__ inline void localizeBlock(uint32_t n, uint32_t rank, uint32_t size, c
     __syncthreads();
   }
   if (t == 0) *haloCount = base;
-  if (!halo) return;
+  if (!halo || base > limit) return;
   for (uint32_t k = t; k < words; k += blockDim.x) {
     uint32_t at = before[k];
     for (uint32_t m = bits[k]; m; m &= m - 1) halo[at++] = 32 * k + __ffs(m) - 1;

@@ -1892,11 +1892,17 @@ int drape_cuda_inject_failure(drape_solver* s, int steps) {
 namespace {
 
 constexpr uint32_t kNoAllocMaxBlocks = 256;  // partials capacity (grid = one block per SM)
+constexpr uint32_t kNoAllocMaxSms = 240;     // the mailbox and the halos' sizes of as many blocks fit the partials' region
 
-// Byte layout of the scratch array (every region 256-byte aligned).
+// Byte layout of the scratch array (every region 256-byte aligned). A call uses it in one of two ways (k_noalloc_localize
+// decides): for the resident-row PCG the vectors after z hold the slots' local columns and the halos, and the partials'
+// region the mailbox and the halos' sizes; for the 1024-thread PCG they are what their names say.
 struct NoAllocLayout {
   static constexpr size_t N = DRAPE_PCG_NOALLOC_MAX_PARTICLES, B = DRAPE_PCG_NOALLOC_MAX_SLOTS;
-  static constexpr size_t vectors = 0;                                   // r, z, p0, p1, ap, apFull
+  static constexpr size_t vectors = 0;                                   // z, r, p0, p1, ap, apFull
+  static constexpr size_t localCol = vectors + sizeof(float4) * N;       // 16 bits a slot, over r and p0
+  static constexpr size_t halo = localCol + sizeof(uint16_t) * B;        // over p1, ap and apFull
+  static constexpr size_t haloEntries = 3 * sizeof(float4) * N / sizeof(uint32_t);
   static constexpr size_t precond = vectors + 6 * sizeof(float4) * N;    // 3 float4 per particle
   static constexpr size_t particle = precond + 3 * sizeof(float4) * N;
   static constexpr size_t contact = particle + sizeof(dcu::Particle) * N;
@@ -1904,9 +1910,14 @@ struct NoAllocLayout {
   static constexpr size_t cols = diag + sizeof(uint32_t) * N;
   static constexpr size_t partials = cols + sizeof(uint32_t) * B;
   static constexpr size_t control = partials + 2 * kNoAllocMaxBlocks * dcu::kPartialStride * sizeof(double);
+  static constexpr size_t mailSeq = control + 248;                       // kept from call to call
   static constexpr size_t total = control + 256;
 };
-static_assert(sizeof(dcu::Control) <= 256, "control block fits its region");
+static_assert(sizeof(dcu::Control) <= 248, "control block fits its region");
+static_assert(sizeof(uint16_t) * NoAllocLayout::B == 2 * sizeof(float4) * NoAllocLayout::N, "local columns fill r and p0");
+static_assert(dcu::mailWords(kNoAllocMaxSms) * sizeof(dcu::MailWord) + kNoAllocMaxSms * sizeof(uint32_t) <=
+                  NoAllocLayout::control - NoAllocLayout::partials,
+              "mailbox and halo sizes fit the partials' region");
 static_assert(NoAllocLayout::total == DRAPE_PCG_NOALLOC_SCRATCH_BYTES, "scratch size matches the header");
 
 // The scratch. In host code this name is a host-side stand-in, not a device address: the address a kernel may use
@@ -1916,11 +1927,14 @@ __device__ __align__(256) unsigned char g_pcgScratch[NoAllocLayout::total];
 struct NoAllocDevice {
   unsigned char* scratch = nullptr;
   int sms = 0;
+  size_t residentSmem = 0;  // dynamic shared memory of k_noalloc_rows
   bool ready = false;
 };
 constexpr int kNoAllocMaxDevices = 64;
 NoAllocDevice g_noAlloc[kNoAllocMaxDevices];
 std::mutex g_noAllocMutex;
+
+size_t noAllocRowsSmem(int device);  // sets and returns k_noalloc_rows's dynamic shared memory
 
 // The device address of the scratch array and the SM count, with `device` current. The SM count is looked up once per
 // device. The address is looked up again on every call made outside a stream capture (cudaGetSymbolAddress allocates
@@ -1939,8 +1953,9 @@ NoAllocDevice& noAllocScratch(int device, cudaStream_t stream) {
     CK(cudaGetSymbolAddress(&p, g_pcgScratch));
     if (!d.ready) {
       CK(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device));
-      if (d.sms < 1 || static_cast<uint32_t>(d.sms) > kNoAllocMaxBlocks)
+      if (d.sms < 1 || static_cast<uint32_t>(d.sms) > kNoAllocMaxSms)
         throw std::runtime_error("cuda: unsupported SM count for the no-allocation PCG");
+      d.residentSmem = noAllocRowsSmem(device);
     }
     d.scratch = static_cast<unsigned char*>(p);
     d.ready = true;
@@ -1956,10 +1971,14 @@ namespace dcu {
 // non-decreasing from 0 to `slots`, a column index >= n, or a row without its diagonal block.
 constexpr int kNoAllocBadStructure = 3;
 
-// Clears the control block and the iteration output before the structure check can raise an error in it.
-__global__ void k_noalloc_clear(Control* ctl, int* iterations) {
-  *ctl = Control{};
-  *iterations = 0;
+// Clears the control block, the iteration output and the mailbox (one block) before the structure check can raise an
+// error in it.
+__global__ void k_noalloc_clear(Control* ctl, int* iterations, MailWord* mail, uint32_t words) {
+  if (threadIdx.x == 0) {
+    *ctl = Control{};
+    *iterations = 0;
+  }
+  for (uint32_t k = threadIdx.x; k < words; k += blockDim.x) mail[k] = MailWord{0.0, 0ull};
 }
 
 // Converts the caller's flags into the solver's layouts inside the scratch (particle pinned flags, contact state,
@@ -2003,15 +2022,19 @@ __global__ void k_noalloc_prepare(uint32_t n, uint32_t slots, const uint32_t* __
   }
 }
 
-// k_pcg_precondition and k_pcg_only of the allocating entry point, skipped once the structure check has failed (every
-// block reads the same flag, written by an earlier kernel on the stream, so the cooperative launch returns as a whole).
-__global__ void k_noalloc_precondition(Dev D, const uint32_t* __restrict__ diag) {
+// Skipped, like the solves, once the structure check has failed (every block reads the same flag, written by an earlier
+// kernel on the stream, so a cooperative launch returns as a whole). One block per solve block: the block-Jacobi inverses
+// of its rows, its halo and local columns, and whether it fits the resident-row PCG's layout; a block that does not sets
+// Control::newtonDone, which sends the call to the 1024-thread PCG.
+__global__ void __launch_bounds__(512) k_noalloc_localize(Dev D, const uint32_t* __restrict__ diag) {
   if (*reinterpret_cast<volatile int*>(&D.ctl->error) != 0) return;
-  const uint32_t SP = D.P.slotsPadded;
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < D.P.n; i += gridDim.x * blockDim.x) {
+  const uint32_t SP = D.P.slotsPadded, t = threadIdx.x, lane = t & 31u, w = t >> 5;
+  uint32_t r0, r1;
+  blockRange(D.P.n, blockIdx.x, gridDim.x, r0, r1);
+  for (uint32_t i = r0 + t; i < r1; i += blockDim.x) {
     M3 A;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) A.m[k] = D.blocks[k * SP + diag[i]];
+    for (int k = 0; k < 9; ++k) A.m[k] = __ldg(D.blocks + k * SP + diag[i]);
     M3 inv;
     if (D.particle[i].pinned != 0u) {
       zero(inv);
@@ -2023,10 +2046,36 @@ __global__ void k_noalloc_precondition(Dev D, const uint32_t* __restrict__ diag)
     D.precond[3 * i + 1] = make_float4(inv.m[3], inv.m[4], inv.m[5], 0.0f);
     D.precond[3 * i + 2] = make_float4(inv.m[6], inv.m[7], inv.m[8], 0.0f);
   }
+  __shared__ uint32_t warpSlots[16];
+  uint32_t* count = const_cast<uint32_t*>(D.haloCount) + blockIdx.x;
+  localizeBlock(D.P.n, blockIdx.x, gridDim.x, D.rowStart, D.colIndex, (D.P.n + 31u) / 32u, count,
+                const_cast<uint32_t*>(D.halo) + static_cast<size_t>(blockIdx.x) * D.P.haloStride,
+                const_cast<uint16_t*>(D.localCol), D.P.haloStride);
+  const uint32_t i = r0 + t;  // at most kRowWorkers rows a block (n is at most 8192)
+  const uint32_t len = i < r1 && D.particle[i].pinned == 0u ? D.rowStart[i + 1] - D.rowStart[i] : 0u;
+  const uint32_t longest = __reduce_max_sync(0xffffffffu, len);
+  if (lane == 0) warpSlots[w] = longest > kRegSlots ? 32u * ((longest - kRegSlots + 1u) & ~1u) : 0u;
+  __syncthreads();
+  if (t == 0) {
+    uint64_t total = 0;
+    for (int k = 0; k < 16; ++k) total += warpSlots[k];
+    if (total > D.P.residentSlots || *count > D.P.haloStride || r1 - r0 > static_cast<uint32_t>(kRowWorkers))
+      D.ctl->newtonDone = 1;
+  }
+}
+
+// The resident-row PCG (pcgResident), and the 1024-thread one for systems whose rows or halos do not fit it: the same
+// iterates.
+__global__ void __launch_bounds__(kRowThreads, 1) k_noalloc_rows(Dev D) {
+  if (*reinterpret_cast<volatile int*>(&D.ctl->error) != 0 || D.ctl->newtonDone != 0) return;
+  GridSync gs;
+  gs.init(D.ctl, D.P.barrierLimitNs);
+  const int it = pcgSolve<false, kRowLanes, kResidentRows>(D, gs);
+  if (it >= 0 && blockIdx.x == 0 && threadIdx.x == 0) D.ctl->lastCg = it;
 }
 
 __global__ void __launch_bounds__(kSolveThreads, 1) k_noalloc_pcg(Dev D) {
-  if (*reinterpret_cast<volatile int*>(&D.ctl->error) != 0) return;
+  if (*reinterpret_cast<volatile int*>(&D.ctl->error) != 0 || D.ctl->newtonDone == 0) return;
   GridSync gs;
   gs.init(D.ctl, D.P.barrierLimitNs);
   const int it = pcgSolve<false, kRowLanes>(D, gs);
@@ -2034,12 +2083,28 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_noalloc_pcg(Dev D) {
 }
 
 // -2: the structure check failed; -1: a grid barrier gave up waiting; else the PCG iteration count.
-__global__ void k_noalloc_finish(const Control* ctl, int* iterations) {
+// After an abandoned solve the next call's exchanges start from a number that none of its blocks reached.
+__global__ void k_noalloc_finish(const Control* ctl, int* iterations, unsigned long long* mailSeq) {
   const int e = ctl->error;
+  if (e) *mailSeq += 1ull << 24;
   *iterations = e == kNoAllocBadStructure ? -2 : (e ? -1 : ctl->lastCg);
 }
 
 }  // namespace dcu
+
+namespace {
+
+size_t noAllocRowsSmem(int device) {
+  int optin = 0;
+  cudaFuncAttributes fa{};
+  CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  CK(cudaFuncGetAttributes(&fa, dcu::k_noalloc_rows));
+  const size_t most = (static_cast<size_t>(optin) - fa.sharedSizeBytes) & ~static_cast<size_t>(15);
+  CK(cudaFuncSetAttribute(dcu::k_noalloc_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)));
+  return most;
+}
+
+}  // namespace
 
 extern "C" int drape_cuda_pcg_noalloc(uint32_t n, uint32_t slots, const uint32_t* d_row_start,
                                       const uint32_t* d_col_index, const float* d_blocks, uint32_t slots_padded,
@@ -2075,8 +2140,8 @@ extern "C" int drape_cuda_pcg_noalloc(uint32_t n, uint32_t slots, const uint32_t
     d.P.barrierLimitNs = 2000000000ull;
     d.P.h = 1.0f;
     d.P.hD = 1.0;
-    d.r = vec;
-    d.z = vec + N;
+    d.z = vec;
+    d.r = vec + N;
     d.p0 = vec + 2 * N;
     d.p1 = vec + 3 * N;
     d.ap = vec + 4 * N;
@@ -2093,20 +2158,35 @@ extern "C" int drape_cuda_pcg_noalloc(uint32_t n, uint32_t slots, const uint32_t
     d.partials = reinterpret_cast<double*>(base + L::partials);
     d.ctl = reinterpret_cast<dcu::Control*>(base + L::control);
     auto* diag = reinterpret_cast<uint32_t*>(base + L::diag);
+    // The resident-row PCG: as much halo a block as the scratch holds, the rest of the shared memory for its slots.
+    const uint32_t sms = static_cast<uint32_t>(nd.sms), per = (n + sms - 1) / sms;
+    auto* mail = reinterpret_cast<dcu::MailWord*>(base + L::partials);
+    auto* mailSeq = reinterpret_cast<unsigned long long*>(base + L::mailSeq);
+    d.mail = mail;
+    d.mailSeq = mailSeq;
+    d.localCol = reinterpret_cast<const uint16_t*>(base + L::localCol);
+    d.halo = reinterpret_cast<const uint32_t*>(base + L::halo);
+    d.haloCount = reinterpret_cast<const uint32_t*>(mail + dcu::mailWords(sms));
+    d.P.haloStride = static_cast<uint32_t>(L::haloEntries) / sms;
+    d.P.residentNodes = per + d.P.haloStride + 1;
+    d.P.residentSlots = static_cast<uint32_t>((nd.residentSmem - d.P.residentNodes * dcu::kResidentNodeBytes) /
+                                              dcu::kResidentSlotBytes) & ~31u;
     const int pg = std::max(1, static_cast<int>((n + 255) / 256));
-    dcu::k_noalloc_clear<<<1, 1, 0, st>>>(d.ctl, d_iterations);
+    dcu::k_noalloc_clear<<<1, 256, 0, st>>>(d.ctl, d_iterations, mail, static_cast<uint32_t>(dcu::mailWords(sms)));
     CK(cudaGetLastError());
     dcu::k_noalloc_prepare<<<pg, 256, 0, st>>>(
         n, slots, d_row_start, d_col_index, d_pinned, d_active, static_cast<const float4*>(d_normals),
         reinterpret_cast<dcu::Particle*>(base + L::particle), d.contact, reinterpret_cast<uint32_t*>(base + L::cols),
         diag, d.ctl);
     CK(cudaGetLastError());
-    dcu::k_noalloc_precondition<<<pg, 256, 0, st>>>(d, diag);
+    dcu::k_noalloc_localize<<<nd.sms, 512, 2 * sizeof(uint32_t) * ((n + 31) / 32), st>>>(d, diag);
     CK(cudaGetLastError());
     void* args[] = {&d};
+    CK(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(dcu::k_noalloc_rows), dim3(nd.sms), dim3(dcu::kRowThreads),
+                                   args, nd.residentSmem, st));
     CK(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(dcu::k_noalloc_pcg), dim3(nd.sms),
                                    dim3(dcu::kSolveThreads), args, 0, st));
-    dcu::k_noalloc_finish<<<1, 1, 0, st>>>(d.ctl, d_iterations);
+    dcu::k_noalloc_finish<<<1, 1, 0, st>>>(d.ctl, d_iterations, mailSeq);
     CK(cudaGetLastError());
   });
 }

@@ -151,3 +151,51 @@ def test_resident_batch_after_the_partition_changes(gpu):
     assert fa == fb and len(set(fa)) > 1, fa
     for a, b in zip(xa, xb):
         assert np.array_equal(a, b), np.abs(a - b).max()
+
+
+def _system(n, degree, seed, local):
+    """A seeded SPD block-CSR system: a diagonal block and about `degree` symmetric neighbours a row, near the diagonal
+    (`local`) or anywhere; some rows pinned, some with an active contact."""
+    rng = np.random.default_rng(seed)
+    m = n * degree // 2
+    a = rng.integers(0, n, m)
+    b = (a + rng.integers(1, max(2, degree), m)) % n if local else rng.integers(0, n, m)
+    pairs = np.unique(np.sort(np.stack([a, b], 1)[a != b], 1), axis=0)
+    d = rng.standard_normal((len(pairs), 3))
+    block = (d[:, :, None] * d[:, None, :] + 0.1 * np.eye(3)).astype(np.float32)
+    diag = np.tile(0.5 * np.eye(3, dtype=np.float32), (n, 1, 1))
+    for k in (0, 1):
+        np.add.at(diag, pairs[:, k], block)
+    row = np.concatenate([np.arange(n), pairs[:, 0], pairs[:, 1]])
+    col = np.concatenate([np.arange(n), pairs[:, 1], pairs[:, 0]])
+    blocks = np.concatenate([diag, -block, -block])
+    order = np.lexsort((col, row))
+    start = np.zeros(n + 1, np.uint32)
+    start[1:] = np.cumsum(np.bincount(row, minlength=n))
+    normals = rng.standard_normal((n, 3)).astype(np.float32)
+    normals /= np.linalg.norm(normals, axis=1, keepdims=True)
+    pinned = (rng.random(n) < 0.05).astype(np.uint8)
+    grad = (rng.standard_normal((n, 3)) * (1 - pinned)[:, None]).astype(np.float32)
+    return dict(row_start=start, col_index=col[order].astype(np.uint32), blocks=blocks[order].reshape(-1, 9),
+                pinned=pinned, active=(rng.random(n) < 0.2).astype(np.uint8), normals=normals, grad=grad)
+
+
+@pytest.mark.parametrize("n, degree, local", [(1, 0, True), (7, 4, True), (148, 12, True), (149, 12, True),
+                                              (8190, 14, True), (8192, 12, False), (3000, 40, False)])
+def test_noalloc_pcg_over_resident_rows(gpu, n, degree, local):
+    """The allocation-free PCG against the allocating entry point (the 1024-thread kernel) where its blocks' rows and
+    halos fit the resident-row form and where they do not (scattered couplings: the 1024-thread form), twice in a row in
+    either order of the two forms: the same iteration count and iterates."""
+    import torch
+    from test_zz_no_alloc import _noalloc
+    small = _system(200, 8, 1, True)
+    for k in range(2):
+        sysd = dict(_system(n, degree, 10 + n, local), max_it=60, tol=1e-5)
+        ref = gpu.pcg(sysd["row_start"], sysd["col_index"], sysd["blocks"], sysd["pinned"], sysd["active"],
+                      sysd["normals"], sysd["grad"], 60, 1e-5)
+        step, resid, its = _noalloc(gpu, sysd)
+        assert its == ref[2]
+        assert np.linalg.norm(step - ref[0]) <= 1e-6 * np.linalg.norm(ref[0])
+        assert np.linalg.norm(resid - ref[1]) <= 1e-6 * max(np.linalg.norm(ref[1]), 1e-6)
+        _noalloc(gpu, dict(small, max_it=20, tol=1e-3))
+    torch.cuda.synchronize()
