@@ -45,9 +45,6 @@ __device__ __forceinline__ float blockAt(const Graph& g, uint32_t s, int k) { re
 __device__ __forceinline__ void st16(unsigned char* tile, uint32_t r, uint32_t c, uint32_t K, uint4 v) {
   *reinterpret_cast<uint4*>(tile + umma::kmajorOffset(r, c * 8u, K)) = v;
 }
-__device__ __forceinline__ void st1(unsigned char* tile, uint32_t r, uint32_t k, uint32_t K, __nv_bfloat16 v) {
-  *reinterpret_cast<__nv_bfloat16*>(tile + umma::kmajorOffset(r, k, K)) = v;
-}
 __device__ __forceinline__ uint4 zero4() { return make_uint4(0u, 0u, 0u, 0u); }
 
 __device__ __forceinline__ uint4 packBf16(const float* v) {
@@ -69,13 +66,6 @@ __device__ __forceinline__ void unpackBf16(uint4 u, float* v) {
     v[2 * i + 1] = __high2float(p);
   }
 }
-// Scatter a 16-byte chunk (8 BF16 of features 8c..8c+7 of row q) into the transposed tile (row = feature, k = q).
-__device__ __forceinline__ void st16T(unsigned char* tile, uint32_t q, uint32_t c, uint32_t K, uint4 v) {
-  const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) st1(tile, c * 8u + i, q, K, e[i]);
-}
-
 // Shared state of a tile kernel: one mbarrier for MMA completion and a TMEM allocation held for the whole launch.
 struct TileCtx {
   uint64_t* bar;
@@ -323,13 +313,6 @@ __device__ __forceinline__ void stageWeights(unsigned char* tile, const __nv_bfl
   const int chunks = K / 8;
   for (int k = threadIdx.x; k < rows * chunks; k += blockDim.x)
     st16(tile, k / chunks, k % chunks, K, reinterpret_cast<const uint4*>(W + static_cast<size_t>(k / chunks) * K)[k % chunks]);
-}
-// Transposed weights W^T (rows = K_in of W, K = rows of W) as a K-major operand.
-__device__ __forceinline__ void stageWeightsT(unsigned char* tile, const __nv_bfloat16* W, int outRows, int inCols) {
-  for (int k = threadIdx.x; k < outRows * inCols; k += blockDim.x) {
-    const int o = k / inCols, i = k % inCols;
-    st1(tile, i, o, outRows, W[static_cast<size_t>(o) * inCols + i]);
-  }
 }
 
 __device__ __forceinline__ void tileSlotInfo(const Graph& g, const TileRows& tr, int* slotRow, int* rowFirst,
@@ -1171,9 +1154,8 @@ __global__ void k_grad_o_kaporin(Graph g, const float4* c, const float4* w, cons
 
 struct BwOutSmem {
   unsigned char a[128 * 16 * 2];    // go tile (M = 128 slots, K = 16)
-  unsigned char wt[192 * 16 * 2];   // W_o^T (N = 192, K = 16)
-  unsigned char xt[256 * 128 * 2];  // X_out^T (M = 256 features (192 used), K = 128 slots)
-  unsigned char gt[16 * 128 * 2];   // go^T (N = 16, K = 128)
+  unsigned char w[16 * 192 * 2];    // W_o (used as its transpose: N = 192, K = 16)
+  unsigned char x[128 * 192 * 2];   // X_out (used as its transpose: M = features, K = 128 slots)
   float buf[128][65];
   float gof[128][17];
   int slotRow[128];
@@ -1182,7 +1164,7 @@ struct BwOutSmem {
   uint32_t tmem;
 };
 
-__global__ void __launch_bounds__(kThreads) k_bw_output(Graph g, const __nv_bfloat16* __restrict__ Wo,
+__global__ void __launch_bounds__(kThreads, 2) k_bw_output(Graph g, const __nv_bfloat16* __restrict__ Wo,
                                                         const __nv_bfloat16* __restrict__ h,
                                                         const float* __restrict__ go, float* GH, float* GSLOT,
                                                         float* GEPS, float* partials, int* error) {
@@ -1190,8 +1172,7 @@ __global__ void __launch_bounds__(kThreads) k_bw_output(Graph g, const __nv_bflo
   TileCtx T;
   T.init(&S.bar, &S.tmem, 256, error);
   const int t = threadIdx.x;
-  stageWeightsT(S.wt, Wo, 16, 192);
-  for (int k = t; k < 64 * 128; k += kThreads) st1(S.xt, 192 + k / 128, k % 128, 128, __float2bfloat16_rn(0.0f));
+  stageWeights(S.w, Wo, 16, 192);
   float dbAcc = 0.0f;
   bool first = true, good = true;
   for (uint32_t tile = blockIdx.x; tile < g.nTiles; tile += gridDim.x) {
@@ -1216,28 +1197,35 @@ __global__ void __launch_bounds__(kThreads) k_bw_output(Graph g, const __nv_bflo
       unpackBf16(p1, rv + 8);
       st16(S.a, t, 0, 16, p0);
       st16(S.a, t, 1, 16, p1);
-      for (int k = 0; k < 16; ++k) {
-        S.gof[t][k] = rv[k];
-        st1(S.gt, k, t, 128, __float2bfloat16_rn(rv[k]));
-      }
+      for (int k = 0; k < 16; ++k) S.gof[t][k] = rv[k];
     }
-    for (int k = t; k < 128 * 24; k += kThreads) {
-      const int q = k / 24, c = k % 24;
-      uint4 v = zero4();
-      if (q < static_cast<int>(nq)) {
-        const uint32_t s = tr.s0 + q;
-        const int sr = S.slotRow[q] >= 0 ? S.slotRow[q] : -S.slotRow[q] - 2;
-        if (c < 8) v = reinterpret_cast<const uint4*>(h + 64 * static_cast<size_t>(tr.r0 + sr))[c];
-        else if (c < 16) v = reinterpret_cast<const uint4*>(h + 64 * static_cast<size_t>(colOf(g, s)))[c - 8];
-        else v = reinterpret_cast<const uint4*>(g.eps + 64 * static_cast<size_t>(s))[c - 16];
+    // Thread t: chunk c = t % 8 of slots t / 8 + 16 i of [h_i | h_j | eps_s], the gathers of a part in flight together.
+#pragma unroll
+    for (int part = 0; part < 3; ++part) {
+      const int c = t % 8;
+      uint4 v[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int q = t / 8 + 16 * i;
+        v[i] = zero4();
+        if (q < static_cast<int>(nq)) {
+          const uint32_t s = tr.s0 + q;
+          const int sr = S.slotRow[q] >= 0 ? S.slotRow[q] : -S.slotRow[q] - 2;
+          const __nv_bfloat16* row = part == 0   ? h + 64 * static_cast<size_t>(tr.r0 + sr)
+                                     : part == 1 ? h + 64 * static_cast<size_t>(colOf(g, s))
+                                                 : g.eps + 64 * static_cast<size_t>(s);
+          v[i] = reinterpret_cast<const uint4*>(row)[c];
+        }
       }
-      st16T(S.xt, q, c, 128, v);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) st16(S.x, t / 8 + 16 * i, 8 * part + c, 192, v[i]);
     }
     const bool acc = !first;
+    // dW_o^T in two blocks of 128 features: 0-127 and 64-191 (of which the last 64 are kept).
     good = T.run([&] {
-      umma::gemmIssue(T.tmem, S.a, S.wt, 128, 192, 16, false);
-      umma::gemmIssue(T.tmem + 192, S.xt, S.gt, 128, 16, 128, acc);
-      umma::gemmIssue(T.tmem + 224, S.xt + 16 * (16 * 128), S.gt, 128, 16, 128, acc);
+      umma::gemmIssueT(T.tmem, S.a, 0, S.w, 192, 128, 192, 16, false);
+      umma::gemmIssueT(T.tmem + 192, S.x, 192, S.a, 16, 128, 16, 128, acc);
+      umma::gemmIssueT(T.tmem + 224, S.x + 8 * 128, 192, S.a, 16, 128, 16, 128, acc);
     });
     if (!good) break;
     first = false;
@@ -1275,8 +1263,8 @@ __global__ void __launch_bounds__(kThreads) k_bw_output(Graph g, const __nv_bflo
     for (int blk = 0; blk < 2; ++blk) {
       float v[16];
       T.load(192 + 32 * blk, v);
-      const int m = 128 * blk + t;
-      if (m < 192)
+      const int m = 64 * blk + t;
+      if (blk == 0 || m >= 128)
         for (int o = 0; o < 16; ++o) P[o * 192 + m] = v[o];
     }
   } else {
@@ -1286,20 +1274,46 @@ __global__ void __launch_bounds__(kThreads) k_bw_output(Graph g, const __nv_bflo
   T.done();
 }
 
-// GH[j] (+)= sum over slots (j, i) of GSLOT[(i, j)]: messages (i != j, both live) or lower slots (i >= j).
+// GH[j] (+)= sum over slots (j, i) of GSLOT[(i, j)]: messages (i != j, both live) or lower slots (i >= j). One warp a row:
+// the lanes look up 32 slots at once, then the kept ones' rows are read eight at a time and added in slot order.
 __global__ void k_gather(Graph g, const float* __restrict__ GSLOT, float* GH, int messages) {
+  constexpr int kDepth = 8;
   const uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) / 32u;
   const int lane = threadIdx.x & 31;
   if (j >= g.n) return;
   const bool pj = pinnedRow(g, j);
   float a0 = GH[64 * static_cast<size_t>(j) + lane], a1 = GH[64 * static_cast<size_t>(j) + 32 + lane];
-  for (uint32_t s = __ldg(g.rowStart + j); s < __ldg(g.rowStart + j + 1); ++s) {
-    const uint32_t i = colOf(g, s);
-    const bool keep = messages ? (i != j && !pj && !pinnedRow(g, i)) : (i >= j);
-    if (!keep) continue;
-    const size_t ts = __ldg(g.tslot + s);
-    a0 += GSLOT[64 * ts + lane];
-    a1 += GSLOT[64 * ts + 32 + lane];
+  const uint32_t end = __ldg(g.rowStart + j + 1);
+  for (uint32_t s0 = __ldg(g.rowStart + j); s0 < end; s0 += 32) {
+    uint32_t ts = 0;
+    bool keep = false;
+    if (s0 + lane < end) {
+      const uint32_t i = colOf(g, s0 + lane);
+      keep = messages ? (i != j && !pj && !pinnedRow(g, i)) : (i >= j);
+      ts = __ldg(g.tslot + s0 + lane);
+    }
+    uint32_t left = __ballot_sync(0xffffffffu, keep);
+    while (left) {
+      float x0[kDepth], x1[kDepth];
+      int count = 0;
+#pragma unroll
+      for (int k = 0; k < kDepth; ++k) {
+        x0[k] = x1[k] = 0.0f;
+        const uint32_t at = __shfl_sync(0xffffffffu, ts, left ? __ffs(left) - 1 : 0);
+        if (left) {
+          x0[k] = GSLOT[64 * static_cast<size_t>(at) + lane];
+          x1[k] = GSLOT[64 * static_cast<size_t>(at) + 32 + lane];
+          left &= left - 1;
+          ++count;
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < kDepth; ++k)
+        if (k < count) {
+          a0 += x0[k];
+          a1 += x1[k];
+        }
+    }
   }
   GH[64 * static_cast<size_t>(j) + lane] = a0;
   GH[64 * static_cast<size_t>(j) + 32 + lane] = a1;
@@ -1308,16 +1322,18 @@ __global__ void k_gather(Graph g, const float* __restrict__ GSLOT, float* GH, in
 // ------------------------------------------------------------------------------------------------------------------
 // Backward, one message-passing layer (row tiles).
 
+// What bounds it: per tile four rounds of staging, MMA and epilogue one after the other, so two CTAs share an SM (98 KB of
+// shared memory and 256 TMEM columns each). The weight gradients and the products with W^T use the K-major tiles in place
+// as MN-major operands: transposed copies cost 128 two-byte stores a thread and tile with 16-way bank conflicts, 80 KB
+// more shared memory, and left one CTA of 128 threads per SM (10k particles: 247 us a layer, now 110).
 struct BwLayerSmem {
-  unsigned char x[128 * 128 * 2];   // X_upd, then X_msg (M = 128, K = 128)
-  unsigned char xt[128 * 128 * 2];  // transposed X (M = 128 features, K = 128 rows / slots)
-  unsigned char ga[128 * 64 * 2];   // gu / gv (M = 128, K = 64)
-  unsigned char gt[64 * 128 * 2];   // gu^T / gv^T (N = 64, K = 128)
-  unsigned char wu[64 * 128 * 2];   // W_u (N = 64, K = 128)
+  unsigned char x[128 * 128 * 2];   // X_upd, then X_msg (M = 128, K = 128; as its transpose for the weight gradients)
+  unsigned char wu[64 * 128 * 2];   // W_u (N = 64, K = 128; as its transpose for the input gradients)
   unsigned char wm[64 * 128 * 2];   // W_m
-  unsigned char wut[128 * 64 * 2];  // W_u^T (N = 128, K = 64)
-  unsigned char wmt[128 * 64 * 2];  // W_m^T
-  float buf[128][65];
+  union {
+    unsigned char ga[128 * 64 * 2];  // gu, then gv (M = 128, K = 64; as its transpose for the weight gradients)
+    float buf[128][65];              // between them: the aggregate's gradient
+  };
   float bu[64], bm[64];
   int slotRow[128];
   int rowFirst[129];
@@ -1325,7 +1341,12 @@ struct BwLayerSmem {
   uint32_t tmem;
 };
 
-__global__ void __launch_bounds__(kThreads) k_bw_layer(Graph g, const __nv_bfloat16* __restrict__ Wm,
+// Element (q, f) of a gradient tile (K = 64).
+__device__ __forceinline__ float gradAt(const unsigned char* tile, int q, int f) {
+  return __bfloat162float(*reinterpret_cast<const __nv_bfloat16*>(tile + umma::kmajorOffset(q, f, 64)));
+}
+
+__global__ void __launch_bounds__(kThreads, 2) k_bw_layer(Graph g, const __nv_bfloat16* __restrict__ Wm,
                                                        const __nv_bfloat16* __restrict__ Wu,
                                                        const float* __restrict__ bm, const float* __restrict__ bu,
                                                        const __nv_bfloat16* __restrict__ hl,
@@ -1334,19 +1355,17 @@ __global__ void __launch_bounds__(kThreads) k_bw_layer(Graph g, const __nv_bfloa
                                                        float* GEPS, float* partials, int* error) {
   BwLayerSmem& S = *reinterpret_cast<BwLayerSmem*>(alignSmem(netSmem));
   TileCtx T;
-  T.init(&S.bar, &S.tmem, 512, error);
+  T.init(&S.bar, &S.tmem, 256, error);
   const int t = threadIdx.x;
   stageWeights(S.wu, Wu, 64, 128);
   stageWeights(S.wm, Wm, 64, 128);
-  stageWeightsT(S.wut, Wu, 64, 128);
-  stageWeightsT(S.wmt, Wm, 64, 128);
   if (t < 64) {
     S.bu[t] = bu[t];
     S.bm[t] = bm[t];
   }
   float dbu = 0.0f, dbm = 0.0f;
   bool first = true, good = true;
-  constexpr uint32_t kU = 0, kGX = 64, kDWU = 192, kDWM = 256;
+  constexpr uint32_t kU = 0, kGX = 0, kDWU = 128, kDWM = 192;  // u and v are read before gX is formed
   for (uint32_t tile = blockIdx.x; tile < g.nTiles; tile += gridDim.x) {
     const TileRows tr = tileRows(g, tile);
     tileSlotInfo(g, tr, S.slotRow, S.rowFirst, true);
@@ -1366,10 +1385,7 @@ __global__ void __launch_bounds__(kThreads) k_bw_layer(Graph g, const __nv_bfloa
                        : reinterpret_cast<const uint4*>(agg + 64 * static_cast<size_t>(tr.r0 + r))[c - 8];
       }
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        st16(S.x, t / 16 + 8 * i, c, 128, v[i]);
-        st16T(S.xt, t / 16 + 8 * i, c, 128, v[i]);
-      }
+      for (int i = 0; i < 16; ++i) st16(S.x, t / 16 + 8 * i, c, 128, v[i]);
     }
     if (!(good = T.run([&] { umma::gemmIssue(T.tmem + kU, S.x, S.wu, 128, 64, 128, false); }))) break;
     {
@@ -1383,23 +1399,14 @@ __global__ void __launch_bounds__(kThreads) k_bw_layer(Graph g, const __nv_bfloa
           gu[f] = (t < R && u > 0.0f) ? GH[64 * static_cast<size_t>(tr.r0 + t) + f] : 0.0f;
         }
       }
-      for (int c = 0; c < 8; ++c) {
-        const uint4 p = packBf16(gu + 8 * c);
-        st16(S.ga, t, c, 64, p);
-        float rv[8];
-        unpackBf16(p, rv);
-        for (int k = 0; k < 8; ++k) {
-          S.buf[t][8 * c + k] = rv[k];
-          st1(S.gt, 8 * c + k, t, 128, reinterpret_cast<const __nv_bfloat16*>(&p)[k]);
-        }
-      }
+      for (int c = 0; c < 8; ++c) st16(S.ga, t, c, 64, packBf16(gu + 8 * c));
     }
     __syncthreads();
     if (t < 64)
-      for (int q = 0; q < R; ++q) dbu += S.buf[q][t];
+      for (int q = 0; q < R; ++q) dbu += gradAt(S.ga, q, t);
     if (!(good = T.run([&] {
-          umma::gemmIssue(T.tmem + kGX, S.ga, S.wut, 128, 128, 64, false);
-          umma::gemmIssue(T.tmem + kDWU, S.xt, S.gt, 128, 64, 128, acc);
+          umma::gemmIssueT(T.tmem + kGX, S.ga, 0, S.wu, 128, 128, 128, 64, false);
+          umma::gemmIssueT(T.tmem + kDWU, S.x, 128, S.ga, 64, 128, 64, 128, acc);
         })))
       break;
     // gh_prev = GH + gX[0:64]; ga = gX[64:128] -> buf.
@@ -1431,10 +1438,7 @@ __global__ void __launch_bounds__(kThreads) k_bw_layer(Graph g, const __nv_bfloa
         }
       }
 #pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        st16(S.x, t / 16 + 8 * i, c, 128, v[i]);
-        st16T(S.xt, t / 16 + 8 * i, c, 128, v[i]);
-      }
+      for (int i = 0; i < 16; ++i) st16(S.x, t / 16 + 8 * i, c, 128, v[i]);
     }
     if (!(good = T.run([&] { umma::gemmIssue(T.tmem + kU, S.x, S.wm, 128, 64, 128, false); }))) break;
     float gv[64];
@@ -1451,22 +1455,13 @@ __global__ void __launch_bounds__(kThreads) k_bw_layer(Graph g, const __nv_bfloa
       }
     }
     __syncthreads();  // buf (ga) fully read
-    for (int c = 0; c < 8; ++c) {
-      const uint4 p = packBf16(gv + 8 * c);
-      st16(S.ga, t, c, 64, p);
-      float rv[8];
-      unpackBf16(p, rv);
-      for (int k = 0; k < 8; ++k) {
-        S.buf[t][8 * c + k] = rv[k];
-        st1(S.gt, 8 * c + k, t, 128, reinterpret_cast<const __nv_bfloat16*>(&p)[k]);
-      }
-    }
+    for (int c = 0; c < 8; ++c) st16(S.ga, t, c, 64, packBf16(gv + 8 * c));
     __syncthreads();
     if (t < 64)
-      for (int q = 0; q < nq; ++q) dbm += S.buf[q][t];
+      for (int q = 0; q < nq; ++q) dbm += gradAt(S.ga, q, t);
     if (!(good = T.run([&] {
-          umma::gemmIssue(T.tmem + kGX, S.ga, S.wmt, 128, 128, 64, false);
-          umma::gemmIssue(T.tmem + kDWM, S.xt, S.gt, 128, 64, 128, acc);
+          umma::gemmIssueT(T.tmem + kGX, S.ga, 0, S.wm, 128, 128, 128, 64, false);
+          umma::gemmIssueT(T.tmem + kDWM, S.x, 128, S.ga, 64, 128, 64, 128, acc);
         })))
       break;
     first = false;
@@ -1479,8 +1474,11 @@ __global__ void __launch_bounds__(kThreads) k_bw_layer(Graph g, const __nv_bfloa
           float4* d = reinterpret_cast<float4*>(GSLOT + 64 * s + 16 * c);
           for (int k = 0; k < 4; ++k) d[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
         } else if (S.slotRow[t] >= 0) {
-          float* d = GEPS + 64 * s + 16 * (c - 4);
-          for (int k = 0; k < 16; ++k) d[k] += v[k];
+          float4* d = reinterpret_cast<float4*>(GEPS + 64 * s + 16 * (c - 4));
+          for (int k = 0; k < 4; ++k) {
+            const float4 o = d[k];
+            d[k] = make_float4(o.x + v[4 * k], o.y + v[4 * k + 1], o.z + v[4 * k + 2], o.w + v[4 * k + 3]);
+          }
         }
       }
     }
@@ -1515,11 +1513,9 @@ __global__ void __launch_bounds__(kThreads) k_bw_layer(Graph g, const __nv_bfloa
 // Backward of an encoder: q = X W^T + b, gq = G (q > 0); dW^T += X^T gq (X has 16 features, padded to 128 rows).
 
 struct BwEncSmem {
-  unsigned char x[128 * 16 * 2];
+  unsigned char x[128 * 128 * 2];  // X, 16 columns used (K = 16 strided; as its transpose for the weight gradient)
   unsigned char w[64 * 16 * 2];
-  unsigned char xt[128 * 128 * 2];
-  unsigned char gt[64 * 128 * 2];
-  float buf[128][65];
+  unsigned char ga[128 * 64 * 2];  // gq (used as its transpose)
   float b[64];
   uint64_t bar;
   uint32_t tmem;
@@ -1534,7 +1530,7 @@ __global__ void __launch_bounds__(kThreads) k_bw_encode(uint32_t rows, const __n
   T.init(&S.bar, &S.tmem, 128, error);
   const int t = threadIdx.x;
   for (int k = t; k < 64 * 2; k += kThreads) st16(S.w, k / 2, k % 2, 16, reinterpret_cast<const uint4*>(W)[k]);
-  for (int k = t; k < 112 * 128; k += kThreads) st1(S.xt, 16 + k / 128, k % 128, 128, __float2bfloat16_rn(0.0f));
+  for (int k = t; k < 128 * 14; k += kThreads) st16(S.x, k / 14, 2 + k % 14, 128, zero4());
   if (t < 64) S.b[t] = b[t];
   float db = 0.0f;
   bool first = true, good = true;
@@ -1544,10 +1540,9 @@ __global__ void __launch_bounds__(kThreads) k_bw_encode(uint32_t rows, const __n
     for (int k = t; k < 128 * 2; k += kThreads) {
       const uint32_t q = k / 2, c = k % 2, r = r0 + q;
       const uint4 v = r < rows ? reinterpret_cast<const uint4*>(X + 16 * static_cast<size_t>(r))[c] : zero4();
-      st16(S.x, q, c, 16, v);
-      st16T(S.xt, q, c, 128, v);
+      st16(S.x, q, c, 128, v);
     }
-    if (!(good = T.run([&] { umma::gemmIssue(T.tmem, S.x, S.w, 128, 64, 16, false); }))) break;
+    if (!(good = T.run([&] { umma::gemmIssueDesc(T.tmem, umma::smemDescSbo(S.x, 16 * 128), umma::smemDesc(S.w, 16), 128, 64, 16, false); }))) break;
     const uint32_t r = r0 + t;
     for (int c = 0; c < 4; ++c) {
       float v[16];
@@ -1557,20 +1552,14 @@ __global__ void __launch_bounds__(kThreads) k_bw_encode(uint32_t rows, const __n
         const float q = v[k] + S.b[16 * c + k];
         gq[k] = (r < rows && q > 0.0f) ? G[64 * static_cast<size_t>(r) + 16 * c + k] : 0.0f;
       }
-      const uint4 p0 = packBf16(gq), p1 = packBf16(gq + 8);
-      float rv[16];
-      unpackBf16(p0, rv);
-      unpackBf16(p1, rv + 8);
-      for (int k = 0; k < 16; ++k) {
-        S.buf[t][16 * c + k] = rv[k];
-        st1(S.gt, 16 * c + k, t, 128, __float2bfloat16_rn(rv[k]));
-      }
+      st16(S.ga, t, 2 * c, 64, packBf16(gq));
+      st16(S.ga, t, 2 * c + 1, 64, packBf16(gq + 8));
     }
     __syncthreads();
     if (t < 64)
-      for (int q = 0; q < 128; ++q) db += S.buf[q][t];
+      for (int q = 0; q < 128; ++q) db += gradAt(S.ga, q, t);
     const bool acc = !first;
-    if (!(good = T.run([&] { umma::gemmIssue(T.tmem + 64, S.xt, S.gt, 128, 64, 128, acc); }))) break;
+    if (!(good = T.run([&] { umma::gemmIssueT(T.tmem + 64, S.x, 128, S.ga, 64, 128, 64, 128, acc); }))) break;
     first = false;
   }
   float* P = partials + static_cast<size_t>(blockIdx.x) * (64 * 16 + 64);
@@ -1620,11 +1609,20 @@ __global__ void k_ratio(double* coef, int num, int den, int dst) { coef[dst] = c
 // Gradient reduction and optimiser.
 
 __global__ void k_reduce(const float* __restrict__ partials, int grid, uint32_t count, float* dst, float scale) {
-  const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= count) return;
-  float s = 0.0f;
-  for (int c = 0; c < grid; ++c) s += partials[static_cast<size_t>(c) * count + p];
-  dst[p] += scale * s;
+  constexpr int kDepth = 16;  // partials in flight, added in CTA order
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= count) return;
+  float acc = 0.0f;
+  int b = 0;
+  for (; b + kDepth <= grid; b += kDepth) {
+    float x[kDepth];
+#pragma unroll
+    for (int i = 0; i < kDepth; ++i) x[i] = __ldg(partials + static_cast<size_t>(b + i) * count + k);
+#pragma unroll
+    for (int i = 0; i < kDepth; ++i) acc += x[i];
+  }
+  for (; b < grid; ++b) acc += __ldg(partials + static_cast<size_t>(b) * count + k);
+  dst[k] += scale * acc;
 }
 
 __global__ void k_adam(float* master, float* grad, float* m, float* v, uint32_t count, float lr, float b1, float b2,
@@ -1817,7 +1815,7 @@ Network::Network(int device) : device_(device) {
   grad_ = dalloc<float>(Layout::kCount);
   adamM_ = dalloc<float>(Layout::kCount);
   adamV_ = dalloc<float>(Layout::kCount);
-  partialsCount_ = static_cast<size_t>(numSMs_) * Layout::kLayerSize;
+  partialsCount_ = 2 * static_cast<size_t>(numSMs_) * Layout::kLayerSize;
   partials_ = dalloc<float>(partialsCount_);
   error_ = dalloc<int>(1);
   scalars_ = dalloc<double>(8);
@@ -2047,7 +2045,7 @@ void Network::lossForward(GraphStore& s, int residual) {
 }
 
 void Network::reduceInto(const float* partials, int grid, size_t count, size_t offset, float scale) {
-  k_reduce<<<static_cast<int>((count + 255) / 256), 256, 0, stream_>>>(partials, grid, static_cast<uint32_t>(count),
+  k_reduce<<<static_cast<int>((count + 63) / 64), 64, 0, stream_>>>(partials, grid, static_cast<uint32_t>(count),
                                                                       grad_ + offset, scale);
   NCK(cudaGetLastError());
 }
@@ -2066,7 +2064,7 @@ void Network::backward(GraphStore& s) {
   }
   const __nv_bfloat16* W = wBf16_;
   const float* M = master_;
-  const int grid = gridFor(g.nTiles, numSMs_);
+  const int grid = gridFor(g.nTiles, 2 * numSMs_);  // two CTAs an SM
   k_bw_output<<<grid, kThreads, smemFor(sizeof(BwOutSmem)), stream_>>>(g, W + Layout::kO, g.h[kLayers], s.go, s.GH,
                                                                          s.GSLOT, s.GEPS, partials_, error_);
   reduceInto(partials_, grid, Layout::kOB - Layout::kO + kOutputs, Layout::kO, 1.0f);
@@ -2081,12 +2079,12 @@ void Network::backward(GraphStore& s) {
     k_gather<<<wb, 256, 0, stream_>>>(g, s.GSLOT, ghPrev, 1);
     std::swap(gh, ghPrev);
   }
-  const int encGridE = gridFor((g.B + 127) / 128, numSMs_);
+  const int encGridE = gridFor((g.B + 127) / 128, 2 * numSMs_);
   k_bw_encode<<<encGridE, kThreads, smemFor(sizeof(BwEncSmem)), stream_>>>(g.B, g.e, W + Layout::kEe,
                                                                             M + Layout::kEeB, s.GEPS, partials_,
                                                                             error_);
   reduceInto(partials_, encGridE, 64 * 16 + 64, Layout::kEe, 1.0f);
-  const int encGridN = gridFor((g.n + 127) / 128, numSMs_);
+  const int encGridN = gridFor((g.n + 127) / 128, 2 * numSMs_);
   k_bw_encode<<<encGridN, kThreads, smemFor(sizeof(BwEncSmem)), stream_>>>(g.n, g.f, W + Layout::kNe,
                                                                             M + Layout::kNeB, gh, partials_, error_);
   reduceInto(partials_, encGridN, 64 * 16 + 64, Layout::kNe, 1.0f);

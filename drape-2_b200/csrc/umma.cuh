@@ -140,6 +140,27 @@ __device__ __forceinline__ void gemmIssue(uint32_t dTmem, const void* a, const v
   }
 }
 
+// The transpose of a K-major R x C tile as an operand, in place (an "MN-major" operand: its M or N dimension runs along the
+// tile's columns, its K dimension along the rows). Core matrices are the same 8 x 16 bytes; those 8 columns further lie
+// 128 bytes apart (the stride-dimension offset), those 8 rows further 16 * C bytes (the leading-dimension offset), and
+// one K = 16 step is 32 * C bytes.
+__device__ __forceinline__ uint64_t smemDescT(const void* tile, uint32_t C) {
+  const uint64_t addr = smemAddr(tile);
+  return ((addr & 0x3FFFFull) >> 4) | (static_cast<uint64_t>((16u * C) >> 4) << 16) |
+         (static_cast<uint64_t>(128u >> 4) << 32) | (1ull << 46);
+}
+
+// gemmIssue with either operand transposed: A and B are K-major tiles, `aCols` / `bCols` > 0 marks one that is used as
+// its transpose (smemDescT of a tile with that many columns).
+__device__ __forceinline__ void gemmIssueT(uint32_t dTmem, const void* a, uint32_t aCols, const void* b, uint32_t bCols,
+                                           uint32_t M, uint32_t N, uint32_t K, bool accumulate) {
+  const uint32_t idesc = instrDescBf16(M, N) | (aCols ? 1u << 15 : 0u) | (bCols ? 1u << 16 : 0u);
+  const uint64_t aDesc = aCols ? smemDescT(a, aCols) : smemDesc(a, K);
+  const uint64_t bDesc = bCols ? smemDescT(b, bCols) : smemDesc(b, K);
+  const uint64_t aStep = (aCols ? 32u * aCols : 256u) >> 4, bStep = (bCols ? 32u * bCols : 256u) >> 4;
+  for (uint32_t k = 0; k < K / 16; ++k) mma(dTmem, aDesc + k * aStep, bDesc + k * bStep, idesc, accumulate || k > 0);
+}
+
 // gemmIssue with the operands' descriptors given (smemDesc / smemDescSbo).
 __device__ __forceinline__ void gemmIssueDesc(uint32_t dTmem, uint64_t aDesc, uint64_t bDesc, uint32_t M, uint32_t N,
                                               uint32_t K, bool accumulate) {
