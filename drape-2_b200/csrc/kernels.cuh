@@ -1406,6 +1406,222 @@ __device__ inline int pcgResident(const Dev& D, GridSync& gs, ResidentMatrix& A,
   return code == 2 ? -1 : it;
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// The same PCG for small scenes in one cluster of kClusterBlocks blocks (k_solve_cluster): pcgResident with its exchanges
+// in distributed shared memory. A block's exchange warp writes its sums into every block's shared memory (st.async, which
+// completes the bytes on the receiver's mbarrier), and the halo's z is read from its owners' shared memory after a cluster
+// barrier. Same rows, products and scalars, so the same iterates.
+//
+// Why: below a few thousand particles an iteration is two ways through the L2 one after the other, whatever the grid;
+// between the SMs of a GPC they are shorter. Measured (us per PCG iteration on one B200,
+// k_solve_rows on 148 blocks in brackets): 1,600 particles 2.04 (2.79), 2,600 2.25 (2.8), 4,000 2.59 (2.82), 5,000 3.1
+// (2.8); a frame of the 1,600-particle sheet 353 us (421). At 4,000 the passes after the PCG, on 16 SMs instead of 148,
+// take what the iterations save, so scenes up to 3,500 particles run it (drape_solver::kClusterParticles).
+constexpr int kClusterBlocks = 16;
+constexpr int kClusterRows = 8;  // the solve templates' Variant value of this form
+
+__device__ __forceinline__ uint32_t sharedAddress(const void* p) {
+  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
+}
+// The shared-memory address `local` of block `rank` of the cluster.
+__device__ __forceinline__ uint32_t clusterAddress(uint32_t local, uint32_t rank) {
+  uint32_t out;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(local), "r"(rank));
+  return out;
+}
+__device__ __forceinline__ void clusterArrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void clusterWait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+struct ClusterMail {
+  double value[2][kClusterBlocks][2];  // the two sums of an iteration (r.r and r.z; p.Ap), each block's
+  unsigned long long bar[2];
+};
+
+// One exchange of K values by the exchange warp; `which` alternates, so a message never meets one not yet read (mailSum's
+// argument). `phase` counts this mbarrier's uses.
+template <int K>
+__device__ inline bool clusterSum(const Dev& D, ClusterMail& mail, int which, uint32_t phase, uint32_t rank,
+                                  const double (&mine)[K], double (&total)[K]) {
+  const uint32_t lane = threadIdx.x & 31u, bar = sharedAddress(&mail.bar[which]);
+  if (lane == 0)
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
+                 "r"(static_cast<uint32_t>(kClusterBlocks * 16))
+                 : "memory");
+  __syncwarp();
+  if (lane < static_cast<uint32_t>(kClusterBlocks)) {
+    const uint32_t to = clusterAddress(sharedAddress(&mail.value[which][rank][0]), lane);
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(to),
+                 "l"(__double_as_longlong(mine[0])), "l"(__double_as_longlong(mine[K - 1])),
+                 "r"(clusterAddress(bar, lane))
+                 : "memory");
+  }
+  BoundedWait wait;
+  for (;;) {
+    uint32_t done;
+    asm volatile(
+        "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
+        : "=r"(done)
+        : "r"(bar), "r"(phase & 1u)
+        : "memory");
+    if (__all_sync(0xffffffffu, done != 0)) break;
+    if (__any_sync(0xffffffffu, wait.expired(D.ctl, D.P.barrierLimitNs))) return false;
+  }
+#pragma unroll
+  for (int k = 0; k < K; ++k)
+    total[k] = warpSum(lane < static_cast<uint32_t>(kClusterBlocks) ? mail.value[which][lane][k] : 0.0);
+  return true;
+}
+
+// As pcgResident, on the blocks of one cluster (gs.size == kClusterBlocks). All threads of the cluster pass the same
+// cluster barriers: one before the first iteration, one in each, and one at the end, before which no block leaves its
+// shared memory to others that may still read it.
+__device__ inline int pcgCluster(const Dev& D, GridSync& gs, ResidentMatrix& A, ClusterMail& mail) {
+  constexpr int kWarps = kRowWorkers / 32;
+  __shared__ ResidentShared sh;
+  const int maxCg = D.P.maxCg;
+  const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+  int it = 0, code = 0;
+  if (w == kWarps) {
+    double rz = 0.0, r0 = 0.0;
+    uint32_t phase = 0;
+    while (it < maxCg) {
+      clusterArrive();
+      namedSync<1>(kRowThreads);
+      double part[2], sum[2];
+#pragma unroll
+      for (int k = 0; k < 2; ++k) part[k] = warpSum(lane < kWarps ? sh.red[k][lane] : 0.0);
+      float factor = 0.0f;
+      if (!clusterSum<2>(D, mail, 0, phase, gs.rank, part, sum)) {
+        code = 2;
+      } else if (it == 0) {
+        r0 = sqrt(sum[0]);
+        code = r0 > 0.0 ? 0 : 1;
+      } else {
+        code = sqrt(sum[0]) <= D.P.cgTolerance * r0 ? 1 : 0;
+        factor = static_cast<float>(sum[1] / rz);
+      }
+      rz = sum[1];
+      if (lane == 0) {
+        sh.code = code;
+        sh.factor = factor;
+      }
+      namedArrive<3>(kRowThreads);
+      clusterWait();
+      if (code) break;
+      namedSync<1>(kRowThreads);
+      double pap[1] = {warpSum(lane < kWarps ? sh.red[0][lane] : 0.0)}, pAp[1];
+      if (!clusterSum<1>(D, mail, 1, phase, gs.rank, pap, pAp))
+        code = 2;
+      else
+        code = pAp[0] > 0.0 ? 0 : 1;
+      ++phase;
+      if (lane == 0) {
+        sh.code = code;
+        sh.factor = code ? 0.0f : static_cast<float>(rz / pAp[0]);
+      }
+      namedArrive<3>(kRowThreads);
+      if (code) break;
+      ++it;
+    }
+  } else {
+    uint32_t r0i, r1i;
+    blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
+    const uint32_t i = r0i + threadIdx.x, per = (D.P.n + gs.size - 1) / gs.size;
+    const bool own = i < r1i, busy = 32u * w < r1i - r0i;  // busy: a row of this warp is owned
+    // The halo entries this thread copies each iteration: where they are in the cluster's shared memory.
+    constexpr int kMine = 3;
+    uint32_t from[kMine];
+    const uint32_t zBase = sharedAddress(A.z);
+    auto owner = [&](uint32_t h) {
+      const uint32_t j = __ldg(A.halo + h);
+      return clusterAddress(zBase + 16u * (j % per), j / per);
+    };
+#pragma unroll
+    for (int k = 0; k < kMine; ++k) {
+      const uint32_t h = threadIdx.x + k * kRowWorkers;
+      from[k] = h < A.haloSize ? owner(h) : 0u;
+    }
+    auto copyFrom = [&](uint32_t address, uint32_t h) {
+      float4 v;
+      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                   : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                   : "r"(address)
+                   : "memory");
+      A.z[A.rows + h] = v;
+    };
+    Contact c{};
+    M3 M{};
+    float3 step = mk(0, 0, 0), resid = mk(0, 0, 0), r = mk(0, 0, 0), z = mk(0, 0, 0);
+    float3 p = mk(0, 0, 0), apFull = mk(0, 0, 0), ap = mk(0, 0, 0);
+    // CG init (kernels.h:252-268): step = 0, resid = -grad, r = filter(resid), z = filter(M r).
+    if (own) {
+      c = D.contact[i];
+      M = loadPrecond(D, i);
+      resid = -ld3(D.grad, i);
+      r = filterRn(c, resid);
+      z = filterRn(c, mulRn(M, r));
+    }
+    if (!busy && lane == 0) sh.red[0][w] = sh.red[1][w] = 0.0;
+    while (it < maxCg) {
+      if (own) A.z[threadIdx.x] = f4(z);
+      clusterArrive();
+      if (busy) {
+        const double rr = warpSum(dotd3(r, r)), rz = warpSum(dotd3(r, z));  // zero where no row is owned
+        if (lane == 0) {
+          sh.red[0][w] = rr;
+          sh.red[1][w] = rz;
+        }
+      }
+      namedArrive<1>(kRowThreads);
+      clusterWait();
+#pragma unroll
+      for (int k = 0; k < kMine; ++k) {
+        const uint32_t h = threadIdx.x + k * kRowWorkers;
+        if (h < A.haloSize) copyFrom(from[k], h);
+      }
+      for (uint32_t h = threadIdx.x + kMine * kRowWorkers; h < A.haloSize; h += kRowWorkers) copyFrom(owner(h), h);
+      namedSync<2>(kRowWorkers);
+      const float3 az = busy ? residentProduct(A, A.z) : mk(0, 0, 0);
+      namedSync<3>(kRowThreads);
+      code = sh.code;
+      if (code) break;
+      // A p = A z + beta A pPrev, p = z + beta pPrev (the direction update folded into the product).
+      const float fb = sh.factor;
+      if (busy) {
+        p = it == 0 ? z : axpyRn(p, fb, z);
+        apFull = it == 0 ? az : axpyRn(apFull, fb, az);
+        ap = filterRn(c, apFull);
+        const double pap = warpSum(dotd3(p, ap));
+        if (lane == 0) sh.red[0][w] = pap;
+      }
+      namedArrive<1>(kRowThreads);
+      namedSync<3>(kRowThreads);
+      code = sh.code;
+      if (code) break;
+      const float fa = sh.factor;
+      ++it;
+      // Update (kernels.h:304-315) fused with the preconditioner apply (kernels.h:324-332).
+      step = axpyRn(p, fa, step);
+      r = axpyRn(ap, -fa, r);
+      resid = axpyRn(apFull, -fa, resid);
+      z = filterRn(c, mulRn(M, r));
+    }
+    if (own) {
+      D.step[i] = f4(step);
+      D.resid[i] = f4(resid);
+    }
+  }
+  clusterArrive();
+  clusterWait();
+  return code == 2 ? -1 : it;
+}
+
 // Index arrays of one solve block (blocks of at most 512 threads): its halo (the particles of other blocks its unpinned rows
 // couple to, in particle order) and every slot's column as an index among the block's rows and halo (kNoColumn for pinned
 // columns). The particles met are marked in a bitmap in shared memory (`words` words, and their running counts). With
@@ -2354,7 +2570,23 @@ template <bool Learned, int PL, int Variant = 0>
 __device__ inline int pcgSolve(const Dev& D, GridSync& gs) {
   uint32_t r0i, r1i;
   blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
-  if constexpr (Variant > kResidentRows) {
+  if constexpr (Variant == kClusterRows) {
+    __shared__ ClusterMail mail;
+    ResidentMatrix A;
+    stageResident<false>(D, gs.rank, r0i, r1i, A);  // raises an error status where it does not fit
+    if (threadIdx.x < 2) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(sharedAddress(&mail.bar[threadIdx.x])) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __threadfence();
+    clusterArrive();
+    clusterWait();
+    if (*reinterpret_cast<volatile int*>(&D.ctl->error) != 0) return -1;  // the same for every block
+    const unsigned long long t0 = globalTimerNs();
+    const int it = pcgCluster(D, gs, A, mail);
+    if (gs.rank == 0 && threadIdx.x == 0) D.ctl->pcgNs += static_cast<long long>(globalTimerNs() - t0);
+    return it;
+  } else if constexpr (Variant > kResidentRows) {
     constexpr int kRows = Variant - kResidentRows;
     __shared__ MultiSlices sl;
     MultiMatrix A;

@@ -98,6 +98,12 @@ struct drape_solver {
   // k_solve_rows: each block's halo, then each slot's 16-bit column among its block's rows and halo (one allocation, like
   // the mailbox with its number: device allocations are what a build waits for).
   DBuf<uint32_t> residentIndex, haloCount;
+  // k_solve_cluster: whether the built scene runs it, its shared memory, and its own index arrays.
+  bool clusterOn = false, clusterSupported = false;
+  size_t clusterSmemCap = 0, clusterSmemBytes = 0;
+  uint32_t clusterSlots = 0, clusterNodes = 0, clusterStride = 0;
+  DBuf<uint32_t> clusterIndex;
+  const uint16_t* clusterLocalCol = nullptr;
   DBuf<uint8_t> spill;  // k_solve_rows_multi: the slots that shared memory has no room for
   DBuf<float4> factorSliced;  // k_solve_rows_learned: the factor in the sliced layout, where shared memory has no room
   DBuf<dcu::MailWord> mail;  // its last word's tag is the number of the last exchange
@@ -204,6 +210,15 @@ struct drape_solver {
         return most;
       };
       learnedSmemCap = allow(reinterpret_cast<const void*>(dcu::k_solve_rows_learned));
+      clusterSmemCap = allow(reinterpret_cast<const void*>(dcu::k_solve_cluster));
+      if (cudaFuncSetAttribute(dcu::k_solve_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) {
+        cudaLaunchAttribute attr[1];
+        cudaLaunchConfig_t cfg = clusterConfig(clusterSmemCap, attr);
+        int clusters = 0;
+        clusterSupported = cudaOccupancyMaxActiveClusters(&clusters, dcu::k_solve_cluster, &cfg) == cudaSuccess &&
+                           clusters > 0;
+      }
+      cudaGetLastError();
       residentSmemCap[0] = allow(reinterpret_cast<const void*>(dcu::k_solve_rows));
       residentSmemCap[1] = allow(reinterpret_cast<const void*>(dcu::k_solve_rows_multi<2>));
       residentSmemCap[2] = allow(reinterpret_cast<const void*>(dcu::k_solve_rows_multi<3>));
@@ -304,6 +319,7 @@ struct drape_solver {
     d.P.smemSlots = std::min(solveSmemCap, maxBlockSlots(m.rowStart.data(), n, solveGrid));
     solveSmemBytes = static_cast<size_t>(d.P.smemSlots) * dcu::kSmemSlotBytes;
     localize(n, B, d);
+    if (n > 0 && residentSmemBytes > 0) localizeCluster(n, B); else clusterOn = false;
     d.fieldValues = fieldValues.p;
     d.particle = particle.p;
     d.fabric = fabric.p;
@@ -359,6 +375,31 @@ struct drape_solver {
                                                                       static_cast<size_t>(numSMs) * 16)));
     CK(cudaStreamSynchronize(s));
     built = true;
+  }
+
+  // Whether the scene runs in one cluster (k_solve_cluster), and its index arrays: at most kClusterParticles particles
+  // whose rows and matrix fit kClusterBlocks blocks. Their halos are sized for every other particle. Where the line lies
+  // is measured: see pcgCluster.
+  static constexpr uint32_t kClusterParticles = 3500;
+  void localizeCluster(uint32_t n, uint32_t B) {
+    clusterOn = false;
+    const uint32_t grid = dcu::kClusterBlocks, per = (n + grid - 1) / grid;
+    if (!clusterSupported || n > kClusterParticles || per > static_cast<uint32_t>(dcu::kRowWorkers)) return;
+    clusterSlots = dmodel::WarpLengths(m, static_cast<int>(grid)).most(dcu::kRegSlots, UINT32_MAX);
+    clusterNodes = n + 1;
+    clusterStride = n;
+    clusterSmemBytes = (static_cast<size_t>(clusterSlots) * dcu::kResidentSlotBytes + 15) / 16 * 16 +
+                       static_cast<size_t>(clusterNodes) * dcu::kResidentNodeBytes;
+    if (clusterSmemBytes > clusterSmemCap) return;
+    const size_t haloEntries = static_cast<size_t>(clusterStride) * grid;
+    clusterIndex.alloc(grid + haloEntries + (static_cast<size_t>(B) + 1) / 2);
+    uint16_t* localCol = reinterpret_cast<uint16_t*>(clusterIndex.p + grid + haloEntries);
+    const uint32_t words = (n + 31u) / 32u;
+    dcu::k_localize<<<grid, 512, 2 * sizeof(uint32_t) * static_cast<size_t>(words), stream>>>(
+        n, grid, rowStart.p, colIndex.p, words, clusterIndex.p, clusterStride, clusterIndex.p + grid, localCol);
+    CK(cudaGetLastError());
+    clusterLocalCol = localCol;
+    clusterOn = true;
   }
 
   // Picks the resident-row kernel that every solve block fits, if one does, and builds its index arrays: the halos, and
@@ -548,8 +589,35 @@ struct drape_solver {
     return learnedOn && netGraph ? learnedSmemBytes > 0 && precondSwitch == 0 : residentSmemBytes > 0;
   }
 
+  cudaLaunchConfig_t clusterConfig(size_t smem, cudaLaunchAttribute* attr) const {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(dcu::kClusterBlocks);
+    cfg.blockDim = dim3(dcu::kRowThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    attr[0].id = cudaLaunchAttributeClusterDimension;  // one cluster: its blocks are co-resident
+    attr[0].val.clusterDim.x = dcu::kClusterBlocks;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cfg;
+  }
+
   void launchSolve(const dcu::Dev& d) {
     const bool rows = usesResidentRows(d);
+    if (rows && clusterOn && !(learnedOn && netGraph)) {
+      dcu::Dev c = d;
+      c.P.residentSlots = clusterSlots;
+      c.P.residentNodes = clusterNodes;
+      c.P.haloStride = clusterStride;
+      c.haloCount = clusterIndex.p;
+      c.halo = clusterIndex.p + dcu::kClusterBlocks;
+      c.localCol = clusterLocalCol;
+      cudaLaunchAttribute attr[1];
+      const cudaLaunchConfig_t cfg = clusterConfig(clusterSmemBytes, attr);
+      CK(cudaLaunchKernelEx(&cfg, dcu::k_solve_cluster, c));
+      return;
+    }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(solveGrid);
     cfg.blockDim = dim3(rows ? dcu::kRowThreads : dcu::kSolveThreads);

@@ -20,7 +20,12 @@ __global__ void k_contact_candidates(Dev D, const float4* xs, Contact* out) {
   }
 }
 
-__global__ void k_activate(Dev D) { activateRows(D, blockIdx.x, gridDim.x); }
+// Also restarts the solve's barrier counter: the solve kernels' grids differ in size, and a barrier counts its arrivals
+// from a multiple of its own.
+__global__ void k_activate(Dev D) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) D.ctl->barrierArrivals = 0ull;
+  activateRows(D, blockIdx.x, gridDim.x);
+}
 
 constexpr int kTermThreads = 256;  // k_terms block size
 
@@ -60,6 +65,14 @@ __global__ void __launch_bounds__(kRowThreads, 1) k_solve_rows(Dev D) {
   GridSync gs;
   gs.init(D.ctl, D.P.barrierLimitNs);
   solveGroup<false, kRowLanes, kResidentRows>(D, gs);
+}
+
+// The same for small scenes, on the blocks of one cluster (pcgCluster).
+__global__ void __launch_bounds__(kRowThreads, 1) k_solve_cluster(Dev D) {
+  if (D.ctl->newtonDone) return;
+  GridSync gs;
+  gs.init(D.ctl, D.P.barrierLimitNs);
+  solveGroup<false, kRowLanes, kClusterRows>(D, gs);
 }
 
 // The same for larger scenes: Rows rows a thread, the matrix partly in the L2 (pcgResidentMulti).

@@ -37,6 +37,10 @@ CASES = {
     "sheet_13x13": lambda: S.sheet_on_sphere(n=13, height=0.16, cg_tolerance=1e-2, max_cg=50),
     "sheet_70x70": lambda: S.sheet_on_sphere(n=70, height=0.16, cg_tolerance=1e-6, max_cg=200),
     "pinned_37x37": lambda: _hanging(37),
+    # One cluster up to 3,500 particles (59 x 59), the whole grid from there on.
+    "cluster_59x59": lambda: S.sheet_on_sphere(n=59, height=0.16, cg_tolerance=1e-2, max_cg=50),
+    "cluster_shuffled_50x50": lambda: _shuffled(50, 4),
+    "grid_60x60": lambda: S.sheet_on_sphere(n=60, height=0.16, cg_tolerance=1e-2, max_cg=50),
     "shuffled_60x60": lambda: _shuffled(60, 3),
     "tube_66k": lambda: S.seamed_tube(161, 205, field_n=64, field_cell=0.012),
     # Several rows a thread, the matrix partly in the L2: the smallest and largest of two rows, and three rows.
@@ -199,3 +203,27 @@ def test_noalloc_pcg_over_resident_rows(gpu, n, degree, local):
         assert np.linalg.norm(resid - ref[1]) <= 1e-6 * max(np.linalg.norm(ref[1]), 1e-6)
         _noalloc(gpu, dict(small, max_it=20, tol=1e-3))
     torch.cuda.synchronize()
+
+
+def test_solve_kernels_of_different_grids_take_turns(gpu):
+    """One solver, three frames each with the cluster kernel, the 1024-thread kernel and the learned kernel in turn: the
+    barrier counter starts anew for each, and the block-Jacobi frames equal a solver's that never changed."""
+    from drape_b200 import learned
+    net = learned.LearnedPreconditioner(0)
+    scene = CASES["cluster_59x59"]()
+    a, b = gpu.CudaSolver(0), gpu.CudaSolver(0)
+    for s in (a, b):
+        s.build(scene)
+    for k in range(3):
+        start = b.snapshot()
+        a.set_pcg_variant(3 if k == 1 else 0)
+        a.step(1.0 / 60.0, 1, 2)
+        b.step(1.0 / 60.0, 1, 2)
+        assert np.array_equal(a.positions(), b.positions())
+        a.set_precond(net)
+        a.step(1.0 / 60.0, 1, 2)
+        a.set_precond(None)
+        a.restore(b.snapshot())
+        assert np.isfinite(start["positions"]).all()
+    a.close()
+    b.close()
