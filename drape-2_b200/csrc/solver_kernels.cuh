@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(kSolveThreads, 1) k_pcg_only(Dev D) {
 // row then adds its slots' products in slot order. Configuration: 256 threads, 128 rows, 1024-slot chunks (4.36 TB/s
 // on the tiled 60k-tube system; a 128-thread, 64-row variant held to 32 registers reached 4.19 there).
 constexpr uint32_t kSpmvThreads = 256, kSpmvBlockRows = 128, kSpmvBlockChunk = 1024;
+constexpr uint32_t kSpmvPerSm = 6;  // blocks an SM holds
 
 __global__ void __launch_bounds__(kSpmvThreads) k_spmv(uint32_t n, const uint32_t* __restrict__ rowStart,
                                                            const uint32_t* __restrict__ colIndex,
@@ -288,6 +289,100 @@ __global__ void __launch_bounds__(kSpmvThreads) k_spmv(uint32_t n, const uint32_
     if (t < R) y[r0 + t] = f4(rowLive ? acc : mk(0, 0, 0));
     __syncthreads();  // rowOff is rewritten for the next row range
   }
+}
+
+// The same product where the matrix is small enough for its blocks to fill one or two waves (the launch's rule) and its
+// planes are 16-byte aligned: the block owns `rows` rows (the launch's choice) and walks their slots in chunks of
+// 4 * kSpmvThreads from a multiple of four on, each thread computing the products of four consecutive slots from one
+// 16-byte load of every block plane and of the column indices. The rows' sums are added in the same order.
+//
+// What bounds it: the latency of its loads, not their bytes. With one slot a thread and 128 rows a block, 10,080 rows make
+// 79 blocks, each with dependent rounds of 4-byte loads; four slots a thread have 40 loads in flight at once, and the rows
+// are spread over the SMs. us in a captured sequence, one slot a thread / this kernel: 1,000 rows 5.3 / 2.7; 10,080 5.4 /
+// 3.1; 40,000 10.2 / 5.4; 120,000 24.3 / 20.0. On larger systems its 64 registers (4 blocks an SM) have fewer bytes in
+// flight than the narrow kernel's 6 blocks: 200,000 28.4 / 29.9; 450,000 55.2 / 59.1. Five or six wide blocks an SM spill
+// and are slower at every size.
+constexpr uint32_t kSpmvWideChunk = 4 * kSpmvThreads;
+constexpr uint32_t kSpmvWidePerSm = 4;  // blocks an SM holds at 64 registers a thread
+
+__global__ void __launch_bounds__(kSpmvThreads) k_spmv_wide(uint32_t n, const uint32_t* __restrict__ rowStart,
+                                                            const uint32_t* __restrict__ colIndex,
+                                                            const float* __restrict__ blocks, uint32_t SP,
+                                                            const uint8_t* __restrict__ pinned,
+                                                            const float4* __restrict__ x, float4* __restrict__ y,
+                                                            uint32_t rows) {
+  __shared__ uint32_t rowEnd[kSpmvBlockRows + 1];
+  __shared__ float prod[3][kSpmvWideChunk];
+  const uint32_t t = threadIdx.x;
+  const uint32_t r0 = blockIdx.x * rows;
+  const uint32_t R = min(rows, n - r0);
+  if (t <= R) rowEnd[t] = __ldg(rowStart + r0 + t);
+  __syncthreads();
+  const uint32_t s0 = rowEnd[0], s1 = rowEnd[R];
+  float3 acc = mk(0, 0, 0);
+  const bool rowLive = t < R && pinned[r0 + t] == 0;
+  for (uint32_t c = s0 & ~3u; c < s1; c += kSpmvWideChunk) {
+    const uint32_t s = c + 4 * t;
+    if (s < s1 && s + 4 > s0) {
+      // A group of four that reaches out of [s0, s1) is read slot by slot, clamped into it: the products of slots
+      // out of the range are not used.
+      uint32_t j[4];
+      float m[9][4];
+      if (s >= s0 && s + 4 <= s1) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(colIndex + s));
+        j[0] = q.x;
+        j[1] = q.y;
+        j[2] = q.z;
+        j[3] = q.w;
+#pragma unroll
+        for (int e = 0; e < 9; ++e) {
+          const float4 v = __ldg(reinterpret_cast<const float4*>(blocks + static_cast<size_t>(e) * SP + s));
+          m[e][0] = v.x;
+          m[e][1] = v.y;
+          m[e][2] = v.z;
+          m[e][3] = v.w;
+        }
+      } else {
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const uint32_t at = min(max(s + u, s0), s1 - 1);
+          j[u] = __ldg(colIndex + at);
+#pragma unroll
+          for (int e = 0; e < 9; ++e) m[e][u] = __ldg(blocks + static_cast<size_t>(e) * SP + at);
+        }
+      }
+      float3 xj[4];
+      bool live[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        live[u] = pinned[j[u]] == 0;
+        xj[u] = xyz(__ldg(x + j[u]));
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float3 v = mk(0, 0, 0);
+        if (live[u]) {
+          v.x = m[0][u] * xj[u].x + m[1][u] * xj[u].y + m[2][u] * xj[u].z;
+          v.y = m[3][u] * xj[u].x + m[4][u] * xj[u].y + m[5][u] * xj[u].z;
+          v.z = m[6][u] * xj[u].x + m[7][u] * xj[u].y + m[8][u] * xj[u].z;
+        }
+        prod[0][4 * t + u] = v.x;
+        prod[1][4 * t + u] = v.y;
+        prod[2][4 * t + u] = v.z;
+      }
+    }
+    __syncthreads();
+    if (t < R) {
+      const uint32_t lo = max(rowEnd[t], c), hi = min(rowEnd[t + 1], c + kSpmvWideChunk);
+      for (uint32_t q = lo; q < hi; ++q) {
+        acc.x += prod[0][q - c];
+        acc.y += prod[1][q - c];
+        acc.z += prod[2][q - c];
+      }
+    }
+    __syncthreads();
+  }
+  if (t < R) y[r0 + t] = f4(rowLive ? acc : mk(0, 0, 0));
 }
 
 // A barrier that waits for one more block than the grid has: it can only end by its time limit. Used by the test of
