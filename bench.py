@@ -906,7 +906,8 @@ def main():
                "onchip_gbs": ab["pcg_iter"] / (pcg_us * 1e-6) / 1e9 if pcg_us else None,
                "note": f"floor = drape_cuda_reduction_floor on the solve's grid (one {solve_threads}-thread block per "
                        "SM), "
-                       "median of 3 x 4000 rounds; us_per_pcg_iteration = in-kernel PCG time / PCG iterations over "
+                       "median of 3 x 4000 rounds of counter-based reductions (the resident-row PCG exchanges "
+                       "by messages and runs below it); us_per_pcg_iteration = in-kernel PCG time / PCG iterations over "
                        "the timed drapes (CG init amortised); onchip_gbs = the iteration's algorithmic bytes over its "
                        "time, served from shared memory and L2"}
     roofline = {"bound": "hbm", "kernel": "k_solve", "achieved": achieved, "peak": peak, "unit": "GB/s",

@@ -74,8 +74,8 @@ struct Garment {
 // Device control block: the PCG / Newton scalars every block of k_solve recomputes identically, plus counters.
 struct Control {
   int newtonDone;   // this substep's Newton loop has stopped (slope >= 0 or max move < 1e-9)
-  int error;        // 1: a grid barrier gave up waiting; 2: a row exceeded the assembly capacity; 4: a block's sliced
-                    // matrix exceeded its shared memory (k_solve_rows)
+  int error;        // 1: a grid barrier or an exchange gave up waiting; 2: a row exceeded the assembly capacity; 4: a
+                    // block's rows or halo did not fit what the host sized (the resident-row kernels)
   unsigned long long barrierArrivals;
   long long cgIterations, newtonIterations, lineSearchHalvings, substeps, energyEvaluations;
   double lastAlpha, lastSlope, lastE0, lastMaxMove;
@@ -354,22 +354,17 @@ __device__ inline bool gridCombine(const Dev& D, GridSync& gs, int nw, double (&
   return true;
 }
 
-// HalfWarps (blocks of at most 512 threads): each half-warp is summed on its own (a 16-lane tree) into its own entry
-// of `red`, so 16 rows per entry as in a 1024-thread block whose rows sit on even lanes (pcgReferenceOrder<2>'s p.Ap
-// partials): that block's tree with zeros on its odd lanes adds the same values in the same order.
-template <int K, bool Max = false, bool HalfWarps = false>
+template <int K, bool Max = false>
 __device__ inline bool gridReduce(const Dev& D, GridSync& gs, double (&v)[K], double (&out)[K]) {
   ReduceScratch& sc = reduceScratch();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int nw = HalfWarps ? 2 * ((blockDim.x + 31) >> 5) : (blockDim.x + 31) >> 5;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
 #pragma unroll
   for (int k = 0; k < K; ++k)
 #pragma unroll
-    for (int o = HalfWarps ? 8 : 16; o > 0; o >>= 1)
-      v[k] = combine<Max>(v[k], __shfl_down_sync(0xffffffffu, v[k], o, HalfWarps ? 16 : 32));
-  if (HalfWarps ? (lane & 15) == 0 : lane == 0)
+    for (int o = 16; o > 0; o >>= 1) v[k] = combine<Max>(v[k], __shfl_down_sync(0xffffffffu, v[k], o));
+  if (lane == 0)
 #pragma unroll
-    for (int k = 0; k < K; ++k) sc.red[k][HalfWarps ? 2 * w + (lane >> 4) : w] = v[k];
+    for (int k = 0; k < K; ++k) sc.red[k][w] = v[k];
   __syncthreads();
   return gridCombine<K, Max>(D, gs, nw, out);
 }
@@ -416,7 +411,7 @@ __device__ __forceinline__ float3 filterContact(const Contact& c, float3 v) {
 
 // The PCG's FP32 arithmetic with every rounding written out (products and sums fused or rounded explicitly, nothing
 // left to the compiler's contraction), so that the reference-order kernels (pcgReferenceOrder over 1024-thread blocks,
-// pcgResidentRows over 512-thread ones) round alike in whatever code surrounds them.
+// pcgResident, pcgCluster and pcgResidentMulti over 512-thread ones) round alike in whatever code surrounds them.
 __device__ __forceinline__ float3 axpyRn(float3 x, float s, float3 y) {  // y + s x, one rounding per component
   return mk(__fmaf_rn(x.x, s, y.x), __fmaf_rn(x.y, s, y.y), __fmaf_rn(x.z, s, y.z));
 }

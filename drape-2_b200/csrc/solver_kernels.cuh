@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(512) k_localize(uint32_t n, uint32_t solveBloc
                 halo ? halo + static_cast<size_t>(blockIdx.x) * haloStride : nullptr, localCol);
 }
 
-// The same Newton iteration with the reference-order PCG over resident rows (pcgResidentRows): 512-thread blocks, so a
+// The same Newton iteration with the reference-order PCG over resident rows (pcgResident): 512-thread blocks, so a
 // row thread has the registers to keep its row's PCG state; launched only for scenes whose blocks have at most 480
 // rows and whose sliced matrix, rows and halo fit in shared memory.
 __global__ void __launch_bounds__(kRowThreads, 1) k_solve_rows(Dev D) {
