@@ -125,8 +125,8 @@ __device__ __forceinline__ D3 samplePos(const Grid& g, int x, int y, int z) {
           add(g.oz, mul(g.cell, static_cast<double>(z)))};
 }
 
-// Squared distance from p to the triangle's bounding box (the reference's cheap reject).
-__device__ __forceinline__ double boxGap2(const double* tb, D3 p) {
+// Squared distance from p to a box, lower corner then upper (the reference's cheap reject, with the triangle's bounding box).
+__device__ __forceinline__ double boxGap2(const double (&tb)[6], D3 p) {
   const double gx = fmax(fmax(dsub(tb[0], p.x), dsub(p.x, tb[3])), 0.0);
   const double gy = fmax(fmax(dsub(tb[1], p.y), dsub(p.y, tb[4])), 0.0);
   const double gz = fmax(fmax(dsub(tb[2], p.z), dsub(p.z, tb[5])), 0.0);
@@ -134,10 +134,18 @@ __device__ __forceinline__ double boxGap2(const double* tb, D3 p) {
 }
 
 constexpr int kBakeThreads = 256;
+constexpr uint32_t kNoTriangle = 0xFFFFFFFFu;  // a sample without an owner (yet)
 
 // Pass 1 (Owner = false): the smallest squared distance per sample up to the band's (atomic minimum on the double's bits;
 // non-negative doubles order like their bit patterns; it starts at the first double beyond the band's square, which stands
 // for every far sample). Pass 2 (Owner = true): the lowest triangle index reaching that minimum.
+//
+// The bounding box bounds the distance from below only in exact arithmetic: the computed closest point is a sum of two
+// rounded products and can lie out of the box by a few roundings of its coordinates (a box at 1 m with the last bits of
+// its vertices changed has such samples). Pass 1 rejects by the box as the reference does. Pass 2 has to see again every
+// triangle that pass 1 took, so its box is larger by 2^-48 of the largest coordinate, some three times those roundings:
+// the closest point lies in it, and rounded differences, squares and sums keep that order. The closest point of a
+// triangle without area can lie anywhere; a sample whose owner is not found all the same gets 0 (k_bake_combine).
 //
 // What bounds it: FP64 issue of the closest points (up to three divides each, seven diverging regions). So a sample
 // farther than the band, or than its best so far, is left by its distance from the triangle's bounding box, and a large
@@ -154,7 +162,20 @@ __global__ void __launch_bounds__(kBakeThreads) k_bake_distance(Grid g, Mesh m, 
   const int bx = r[1] - r[0] + 1, by = r[3] - r[2] + 1, bz = r[5] - r[4] + 1;
   const uint3 tri = m.t[task.tri];
   const D3 a = m.v[tri.x], b = m.v[tri.y], c = m.v[tri.z];
-  const double* tb = m.tbox + 6 * static_cast<size_t>(task.tri);
+  double tb[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) tb[k] = m.tbox[6 * static_cast<size_t>(task.tri) + k];
+  if (Owner) {
+    double most = 0.0;
+#pragma unroll
+    for (int k = 0; k < 6; ++k) most = fmax(most, fabs(tb[k]));
+    const double slack = 0x1p-48 * most;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      tb[k] = dsub(tb[k], slack);
+      tb[k + 3] = add(tb[k + 3], slack);
+    }
+  }
   const uint32_t first = task.sub * chunk, last = min(first + chunk, static_cast<uint32_t>(bx) * by * bz);
   for (uint32_t s = first + threadIdx.x; s < last; s += kBakeThreads) {
     const uint32_t row = s / bx, slab = row / by;
@@ -268,9 +289,10 @@ __global__ void k_bake_combine(Grid g, Mesh m, const Part* parts, int which, con
     const int lx = static_cast<int>(i - row * part.nx);
     const int x = part.x0 + lx, y = part.y0 + static_cast<int>(row % part.ny), z = part.z0 + static_cast<int>(row / part.ny);
     const double d2 = __longlong_as_double(static_cast<long long>(dist2[part.at + i]));
+    const bool near = d2 <= g.band2;
+    const uint32_t t = near ? owner[part.at + i] : kNoTriangle;
     double v;
-    if (d2 <= g.band2) {
-      const uint32_t t = owner[part.at + i];
+    if (t != kNoTriangle) {
       const D3 p = samplePos(g, x, y, z);
       const uint3 tri = m.t[t];
       int f;
@@ -286,6 +308,8 @@ __global__ void k_bake_combine(Grid g, Mesh m, const Part* parts, int which, con
         default: n = m.faceN[t]; break;
       }
       v = (dot(sub(p, q), n) >= 0 ? 1.0 : -1.0) * __dsqrt_rn(d2);
+    } else if (near) {
+      v = 0.0;
     } else {
       if (outside[part.word + row * part.wx + (lx >> 5)] >> (lx & 31) & 1u) continue;
       v = -g.band;
@@ -306,7 +330,7 @@ __global__ void k_reset(Grid g, unsigned long long* dist2, uint32_t* owner, size
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < count;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
     dist2[i] = static_cast<unsigned long long>(__double_as_longlong(g.band2)) + 1;  // the first double beyond
-    owner[i] = 0xFFFFFFFFu;
+    owner[i] = kNoTriangle;
   }
 }
 
