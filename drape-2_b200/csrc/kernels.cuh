@@ -2607,6 +2607,9 @@ __device__ inline int pcgSolve(const Dev& D, GridSync& gs) {
       if (gs.rank == 0 && threadIdx.x == 0) D.ctl->learnedSolves += 1;
       if (it < -1) {
         if (gs.rank == 0 && threadIdx.x == 0) D.ctl->precondFallbacks += 1;
+        // A block sends its r.z before it takes its halo of D.z, so a non-finite r.z ends the solve in a fast block while a
+        // slower one still waits for z under the old tag: no new z may be published before every block is out.
+        if (!gs.sync()) return -1;
         const int jac = pcgResident(D, gs, A, seq);
         it = jac < 0 ? jac : jac + (-2 - it);
       }
