@@ -1440,9 +1440,18 @@ struct ClusterMail {
 
 // One exchange of K values by the exchange warp; `which` alternates, so a message never meets one not yet read (mailSum's
 // argument). `phase` counts this mbarrier's uses.
+//
+// No block may leave an exchange on its own: its shared memory would go away under messages and halo reads of the others.
+// So where the wait's limit runs out, or another block has raised the error flag, `late` is set and the messages are
+// awaited all the same (they are on their way: the cluster's blocks run together and each sends before it waits); the next
+// exchange of r.r tells every block (kClusterLate), and all leave after it. The second wait has a limit too, in polls, so
+// that no pause of the whole GPU can end it. Returns false when it runs out.
+constexpr double kClusterLate = -1.0;  // in the place of a block's r.r, which is a sum of squares
+constexpr unsigned int kClusterDrainPolls = 1u << 24;
+
 template <int K>
 __device__ inline bool clusterSum(const Dev& D, ClusterMail& mail, int which, uint32_t phase, uint32_t rank,
-                                  const double (&mine)[K], double (&total)[K]) {
+                                  const double (&mine)[K], double (&total)[K], bool& late) {
   const uint32_t lane = threadIdx.x & 31u, bar = sharedAddress(&mail.bar[which]);
   if (lane == 0)
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar),
@@ -1457,7 +1466,7 @@ __device__ inline bool clusterSum(const Dev& D, ClusterMail& mail, int which, ui
                  : "memory");
   }
   BoundedWait wait;
-  for (;;) {
+  for (unsigned int drain = 0;;) {
     uint32_t done;
     asm volatile(
         "{ .reg .pred p; mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2; selp.u32 %0, 1, 0, p; }"
@@ -1465,7 +1474,11 @@ __device__ inline bool clusterSum(const Dev& D, ClusterMail& mail, int which, ui
         : "r"(bar), "r"(phase & 1u)
         : "memory");
     if (__all_sync(0xffffffffu, done != 0)) break;
-    if (__any_sync(0xffffffffu, wait.expired(D.ctl, D.P.barrierLimitNs))) return false;
+    if (late) {
+      if (++drain == kClusterDrainPolls) return false;
+    } else if (__any_sync(0xffffffffu, wait.expired(D.ctl, D.P.barrierLimitNs))) {
+      late = true;
+    }
   }
 #pragma unroll
   for (int k = 0; k < K; ++k)
@@ -1474,8 +1487,9 @@ __device__ inline bool clusterSum(const Dev& D, ClusterMail& mail, int which, ui
 }
 
 // As pcgResident, on the blocks of one cluster (gs.size == kClusterBlocks). All threads of the cluster pass the same
-// cluster barriers: one before the first iteration, one in each, and one at the end, before which no block leaves its
-// shared memory to others that may still read it.
+// cluster barriers, one in each iteration and one at the end, before which no block leaves its shared memory to others that
+// may still read it: every block learns the same sums, so all leave after the same exchange. Returns -1 in a block whose
+// wait ran out or that another told so.
 __device__ inline int pcgCluster(const Dev& D, GridSync& gs, ResidentMatrix& A, ClusterMail& mail) {
   constexpr int kWarps = kRowWorkers / 32;
   __shared__ ResidentShared sh;
@@ -1485,6 +1499,7 @@ __device__ inline int pcgCluster(const Dev& D, GridSync& gs, ResidentMatrix& A, 
   if (w == kWarps) {
     double rz = 0.0, r0 = 0.0;
     uint32_t phase = 0;
+    bool late = false;
     while (it < maxCg) {
       clusterArrive();
       namedSync<1>(kRowThreads);
@@ -1492,7 +1507,9 @@ __device__ inline int pcgCluster(const Dev& D, GridSync& gs, ResidentMatrix& A, 
 #pragma unroll
       for (int k = 0; k < 2; ++k) part[k] = warpSum(lane < kWarps ? sh.red[k][lane] : 0.0);
       float factor = 0.0f;
-      if (!clusterSum<2>(D, mail, 0, phase, gs.rank, part, sum)) {
+      if (late) part[0] = kClusterLate;
+      if (!clusterSum<2>(D, mail, 0, phase, gs.rank, part, sum, late) ||
+          __any_sync(0xffffffffu, lane < static_cast<uint32_t>(kClusterBlocks) && mail.value[0][lane][0] < 0.0)) {
         code = 2;
       } else if (it == 0) {
         r0 = sqrt(sum[0]);
@@ -1511,7 +1528,7 @@ __device__ inline int pcgCluster(const Dev& D, GridSync& gs, ResidentMatrix& A, 
       if (code) break;
       namedSync<1>(kRowThreads);
       double pap[1] = {warpSum(lane < kWarps ? sh.red[0][lane] : 0.0)}, pAp[1];
-      if (!clusterSum<1>(D, mail, 1, phase, gs.rank, pap, pAp))
+      if (!clusterSum<1>(D, mail, 1, phase, gs.rank, pap, pAp, late))
         code = 2;
       else
         code = pAp[0] > 0.0 ? 0 : 1;
@@ -1524,6 +1541,7 @@ __device__ inline int pcgCluster(const Dev& D, GridSync& gs, ResidentMatrix& A, 
       if (code) break;
       ++it;
     }
+    if (lane == 0) sh.failed = late || code == 2;
   } else {
     uint32_t r0i, r1i;
     blockRange(D.P.n, gs.rank, gs.size, r0i, r1i);
@@ -1614,7 +1632,7 @@ __device__ inline int pcgCluster(const Dev& D, GridSync& gs, ResidentMatrix& A, 
   }
   clusterArrive();
   clusterWait();
-  return code == 2 ? -1 : it;
+  return sh.failed ? -1 : it;
 }
 
 // Index arrays of one solve block (blocks of at most 512 threads): its halo (the particles of other blocks its unpinned rows
@@ -2576,7 +2594,12 @@ __device__ inline int pcgSolve(const Dev& D, GridSync& gs) {
     __threadfence();
     clusterArrive();
     clusterWait();
-    if (*reinterpret_cast<volatile int*>(&D.ctl->error) != 0) return -1;  // the same for every block
+    // An error of a kernel before, or of a block that did not fit: the same for every thread of the cluster, since none
+    // raises one between the two barriers.
+    const int error = *reinterpret_cast<volatile int*>(&D.ctl->error);
+    clusterArrive();
+    clusterWait();
+    if (error != 0) return -1;
     const unsigned long long t0 = globalTimerNs();
     const int it = pcgCluster(D, gs, A, mail);
     if (gs.rank == 0 && threadIdx.x == 0) D.ctl->pcgNs += static_cast<long long>(globalTimerNs() - t0);
