@@ -432,8 +432,9 @@ struct drape_solver {
       residentRowsPerThread = 1;
       d.P.residentSlots = whole;
       residentSmemBytes = slotBytes(whole) + nodeBytes;
-      // The learned kernel: a second array of gathered vectors, and the factor where there is room.
-      const size_t more = residentSmemBytes + nodeBytes;
+      // The learned kernel: a second array of gathered vectors, the columns read past the last, and the factor where
+      // there is room.
+      const size_t more = residentSmemBytes + nodeBytes + sizeof(uint16_t) * dcu::kColumnsRead;
       if (more <= learnedSmemCap) {
         const uint32_t factorSlots = whole + dcu::kRegSlots * dcu::kRowWorkers;
         const size_t factorBytes = 3 * sizeof(float4) * static_cast<size_t>(factorSlots);
