@@ -98,12 +98,23 @@ struct drape_solver {
   // k_solve_rows: each block's halo, then each slot's 16-bit column among its block's rows and halo (one allocation, like
   // the mailbox with its number: device allocations are what a build waits for).
   DBuf<uint32_t> residentIndex, haloCount;
-  // k_solve_cluster: whether the built scene runs it, its shared memory, and its own index arrays.
-  bool clusterOn = false, clusterSupported = false;
-  size_t clusterSmemCap = 0, clusterSmemBytes = 0;
-  uint32_t clusterSlots = 0, clusterNodes = 0, clusterStride = 0;
+  // k_solve_cluster: whether the built scene runs it (`on`), its shared memory, and its own index arrays (in clusterIndex).
+  // These are launch parameters that the device view does not hold, so frame graphs are captured anew when they change.
+  struct ClusterLayout {
+    bool on = false;
+    size_t smemBytes = 0;
+    uint32_t slots = 0, nodes = 0, stride = 0;
+    const uint32_t *haloCount = nullptr, *halo = nullptr;
+    const uint16_t* localCol = nullptr;
+    bool operator==(const ClusterLayout& o) const {
+      return on == o.on && smemBytes == o.smemBytes && slots == o.slots && nodes == o.nodes && stride == o.stride &&
+             haloCount == o.haloCount && halo == o.halo && localCol == o.localCol;
+    }
+  };
+  ClusterLayout cluster;
+  bool clusterSupported = false;
+  size_t clusterSmemCap = 0;
   DBuf<uint32_t> clusterIndex;
-  const uint16_t* clusterLocalCol = nullptr;
   DBuf<uint8_t> spill;  // k_solve_rows_multi: the slots that shared memory has no room for
   DBuf<float4> factorSliced;  // k_solve_rows_learned: the factor in the sliced layout, where shared memory has no room
   DBuf<dcu::MailWord> mail;  // its last word's tag is the number of the last exchange
@@ -319,7 +330,7 @@ struct drape_solver {
     d.P.smemSlots = std::min(solveSmemCap, maxBlockSlots(m.rowStart.data(), n, solveGrid));
     solveSmemBytes = static_cast<size_t>(d.P.smemSlots) * dcu::kSmemSlotBytes;
     localize(n, B, d);
-    if (n > 0 && residentSmemBytes > 0) localizeCluster(n, B); else clusterOn = false;
+    cluster = n > 0 && residentSmemBytes > 0 ? localizeCluster(n, B) : ClusterLayout{};
     d.fieldValues = fieldValues.p;
     d.particle = particle.p;
     d.fabric = fabric.p;
@@ -381,25 +392,28 @@ struct drape_solver {
   // whose rows and matrix fit kClusterBlocks blocks. Their halos are sized for every other particle. Where the line lies
   // is measured: see pcgCluster.
   static constexpr uint32_t kClusterParticles = 3500;
-  void localizeCluster(uint32_t n, uint32_t B) {
-    clusterOn = false;
+  ClusterLayout localizeCluster(uint32_t n, uint32_t B) {
     const uint32_t grid = dcu::kClusterBlocks, per = (n + grid - 1) / grid;
-    if (!clusterSupported || n > kClusterParticles || per > static_cast<uint32_t>(dcu::kRowWorkers)) return;
-    clusterSlots = dmodel::WarpLengths(m, static_cast<int>(grid)).most(dcu::kRegSlots, UINT32_MAX);
-    clusterNodes = n + 1;
-    clusterStride = n;
-    clusterSmemBytes = (static_cast<size_t>(clusterSlots) * dcu::kResidentSlotBytes + 15) / 16 * 16 +
-                       static_cast<size_t>(clusterNodes) * dcu::kResidentNodeBytes;
-    if (clusterSmemBytes > clusterSmemCap) return;
-    const size_t haloEntries = static_cast<size_t>(clusterStride) * grid;
+    if (!clusterSupported || n > kClusterParticles || per > static_cast<uint32_t>(dcu::kRowWorkers)) return {};
+    ClusterLayout c;
+    c.slots = dmodel::WarpLengths(m, static_cast<int>(grid)).most(dcu::kRegSlots, UINT32_MAX);
+    c.nodes = n + 1;
+    c.stride = n;
+    c.smemBytes = (static_cast<size_t>(c.slots) * dcu::kResidentSlotBytes + 15) / 16 * 16 +
+                  static_cast<size_t>(c.nodes) * dcu::kResidentNodeBytes;
+    if (c.smemBytes > clusterSmemCap) return {};
+    const size_t haloEntries = static_cast<size_t>(c.stride) * grid;
     clusterIndex.alloc(grid + haloEntries + (static_cast<size_t>(B) + 1) / 2);
     uint16_t* localCol = reinterpret_cast<uint16_t*>(clusterIndex.p + grid + haloEntries);
     const uint32_t words = (n + 31u) / 32u;
     dcu::k_localize<<<grid, 512, 2 * sizeof(uint32_t) * static_cast<size_t>(words), stream>>>(
-        n, grid, rowStart.p, colIndex.p, words, clusterIndex.p, clusterStride, clusterIndex.p + grid, localCol);
+        n, grid, rowStart.p, colIndex.p, words, clusterIndex.p, c.stride, clusterIndex.p + grid, localCol);
     CK(cudaGetLastError());
-    clusterLocalCol = localCol;
-    clusterOn = true;
+    c.haloCount = clusterIndex.p;
+    c.halo = clusterIndex.p + grid;
+    c.localCol = localCol;
+    c.on = true;
+    return c;
   }
 
   // Picks the resident-row kernel that every solve block fits, if one does, and builds its index arrays: the halos, and
@@ -606,16 +620,16 @@ struct drape_solver {
 
   void launchSolve(const dcu::Dev& d) {
     const bool rows = usesResidentRows(d);
-    if (rows && clusterOn && !(learnedOn && netGraph)) {
+    if (rows && cluster.on && !(learnedOn && netGraph)) {
       dcu::Dev c = d;
-      c.P.residentSlots = clusterSlots;
-      c.P.residentNodes = clusterNodes;
-      c.P.haloStride = clusterStride;
-      c.haloCount = clusterIndex.p;
-      c.halo = clusterIndex.p + dcu::kClusterBlocks;
-      c.localCol = clusterLocalCol;
+      c.P.residentSlots = cluster.slots;
+      c.P.residentNodes = cluster.nodes;
+      c.P.haloStride = cluster.stride;
+      c.haloCount = cluster.haloCount;
+      c.halo = cluster.halo;
+      c.localCol = cluster.localCol;
       cudaLaunchAttribute attr[1];
-      const cudaLaunchConfig_t cfg = clusterConfig(clusterSmemBytes, attr);
+      const cudaLaunchConfig_t cfg = clusterConfig(cluster.smemBytes, attr);
       CK(cudaLaunchKernelEx(&cfg, dcu::k_solve_cluster, c));
       return;
     }
@@ -653,6 +667,7 @@ struct drape_solver {
   struct FrameGraph {
     cudaGraphExec_t exec = nullptr;
     dcu::Dev dev{};
+    ClusterLayout cluster;
     double h = 0;
     int substeps = 0, iterations = 0, precondSwitch = 0;
     unsigned long long barrierLimitNs = 0;
@@ -665,7 +680,7 @@ struct drape_solver {
     FrameGraph& g = frameGraphs[slot];
     if (!g.exec || g.h != h || g.substeps != substeps || g.iterations != iterations ||
         g.precondSwitch != precondSwitch || g.barrierLimitNs != barrierLimitNs ||
-        std::memcmp(&g.dev, &dev, sizeof(dcu::Dev)) != 0) {
+        !(g.cluster == cluster) || std::memcmp(&g.dev, &dev, sizeof(dcu::Dev)) != 0) {
       if (g.exec) CK(cudaGraphExecDestroy(g.exec));
       g.exec = nullptr;
       const uint64_t bytes = d2hBytes;
@@ -693,6 +708,7 @@ struct drape_solver {
       }
       cudaGraphDestroy(graph);
       g.dev = dev;
+      g.cluster = cluster;
       g.h = h;
       g.substeps = substeps;
       g.iterations = iterations;
