@@ -884,25 +884,29 @@ struct drape_batch {
                      : rows == 2 ? bcu::k_solve_batch_resident<2> : bcu::k_solve_batch_resident<3>;
   }
 
+  // The variant whose sums the resident-row solve repeats.
+  bool residentForm() const { return variant == 0 && !(learnedOn && netGraph); }
+
   // Whether the advancing garments fit the resident-row solve: waves of garments, one launch each, with one block per SM,
   // at most kMultiMost rows a thread, and for each garment its rows, their contact planes and the halo in shared memory.
   // As few waves as possible, the largest garments dealt out first; in a wave the blocks are shared out so that the most
-  // rows of any block are as few as possible. Rebuilds the index arrays when the partition changes.
+  // rows of any block are as few as possible. Rebuilds the index arrays when the partition changes; a frame in which none
+  // advances (a phase change, statistics) leaves them as they are.
   //
   // The rule: the default variant with block-Jacobi, whenever it fits in kWaves launches. Measured (us per Newton
   // iteration's solve on one B200, k_solve_batch<false, 0, 256> in brackets): 2 garments of 500 particles 165 (571), 5 of
   // 700-3,000 182 (514), 16 of 2k-40k (175k in all, one wave) 780-960 (1,740), 243k 1,075 (2,650), 394k 2,726 (4,173),
   // 584k 4,001 (6,249); the fastest of the other variants takes 2,130, 3,403 and 5,124 for the last three.
   bool planResident(const std::vector<int>& substeps) {
-    if (variant != 0 || (learnedOn && netGraph)) return false;
+    if (!residentForm()) return false;
     const uint32_t most = dcu::kMultiMost * dcu::kRowWorkers;
     std::vector<uint32_t> live;
     for (uint32_t g = 0; g < G; ++g)
       if (substeps[g] > 0) live.push_back(g);
+    if (live.empty()) return false;  // no solve in this frame: the plan stays for the next one that has
     if (live == residentLive) return residentFits;
     residentLive = live;
     residentFits = false;
-    if (live.empty()) return false;
     auto rows = [&](uint32_t g) { return static_cast<uint32_t>(models[g].x.size()); };
     std::stable_sort(live.begin(), live.end(), [&](uint32_t a, uint32_t b) { return rows(a) > rows(b); });
     auto blocksAt = [&](const std::vector<uint32_t>& of, uint32_t perBlock) {
@@ -1492,11 +1496,13 @@ struct drape_batch {
     BCK(cudaStreamSynchronize(stream));
   }
 
+  // The variant by the names that set it, and the blocks of its launches under the last plan made (a batch is planned with
+  // every garment advancing when it is built).
   drape_batch_tuning tuning() const {
     drape_batch_tuning t{};
     t.row_lanes = kVariants[variant].rowLanes;
     t.block_threads = kVariants[variant].threads;
-    t.blocks = residentOn ? numSMs : solveBlocks;
+    t.blocks = residentForm() && residentFits ? numSMs : solveBlocks;
     return t;
   }
 

@@ -45,12 +45,13 @@ int drape_batch_set_precond(drape_batch* b, drape_precond* p);
 
 typedef struct drape_batch_tuning {
   int32_t row_lanes;      /* the PCG's product A p: 0 = slot-parallel (each thread a run of consecutive block
-                             slots, row sums through shared memory; with block_threads 256, the default, and
-                             block-Jacobi the garments that fit run the same sums over resident rows, one 512-thread
-                             block per SM), or 2, 4, 8 lanes per block row (also the lanes of
+                             slots, row sums through shared memory), or 2, 4, 8 lanes per block row (also the lanes of
                              the learned factor's products; 4 with slot-parallel) */
-  int32_t block_threads;  /* threads per block of the solve launch: 256, 512 or 1024 (1024 / this blocks per SM) */
-  int32_t blocks;         /* blocks of the solve launch */
+  int32_t block_threads;  /* threads per block of the solve launch: 256, 512 or 1024 (1024 / this blocks per SM). With
+                             row_lanes 0, block_threads 256 (the default) and block-Jacobi, garments that fit run the
+                             same sums over resident rows, in one or several launches of one 512-thread block per SM;
+                             block_threads then names the variant all the same */
+  int32_t blocks;         /* blocks of the solve launch (of each of its launches, over resident rows) */
   int32_t variants_timed; /* 0 when set by hand */
   double ms_per_newton;   /* the chosen variant's mean solve time per Newton iteration during tuning */
 } drape_batch_tuning;
@@ -92,7 +93,7 @@ int drape_batch_restore(drape_batch* b);
 typedef struct drape_batch_profile {
   int64_t frames;            /* frames run since profiling was enabled */
   int64_t graph_launches;    /* frames replayed from the captured CUDA graph */
-  int64_t solve_launches;    /* persistent solve launches (one per Newton iteration of the frame) */
+  int64_t solve_launches;    /* Newton iterations' solves, each of one launch or, over resident rows, of up to eight */
   double solve_ms;           /* device time of the solve launches */
   double frame_ms;           /* device time of whole frames */
   int64_t kernel_launches;   /* kernels launched (graph nodes included) */
