@@ -327,9 +327,12 @@ __global__ void k_fill(float* values, size_t count, float v) {
 }
 
 __global__ void k_reset(Grid g, unsigned long long* dist2, uint32_t* owner, size_t count) {
+  // The first double beyond the band's square; where that overflowed nothing lies beyond.
+  const unsigned long long start =
+      static_cast<unsigned long long>(__double_as_longlong(g.band2)) + (isinf(g.band2) ? 0ull : 1ull);
   for (size_t i = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; i < count;
        i += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    dist2[i] = static_cast<unsigned long long>(__double_as_longlong(g.band2)) + 1;  // the first double beyond
+    dist2[i] = start;
     owner[i] = kNoTriangle;
   }
 }
