@@ -1997,18 +1997,18 @@ int drape_cuda_inject_failure(drape_solver* s, int steps) {
 namespace {
 
 constexpr uint32_t kNoAllocMaxBlocks = 256;  // partials capacity (grid = one block per SM)
-constexpr uint32_t kNoAllocMaxSms = 240;     // the mailbox and the halos' sizes of as many blocks fit the partials' region
 
 // Byte layout of the scratch array (every region 256-byte aligned). A call uses it in one of two ways (k_noalloc_localize
-// decides): for the resident-row PCG the vectors after z hold the slots' local columns and the halos, and the partials'
-// region the mailbox and the halos' sizes; for the 1024-thread PCG they are what their names say.
+// decides): for the resident-row PCG the vectors after z hold the slots' local columns, the halos and their sizes, and the
+// partials' region the mailbox; for the 1024-thread PCG they are what their names say.
 struct NoAllocLayout {
   static constexpr size_t N = DRAPE_PCG_NOALLOC_MAX_PARTICLES, B = DRAPE_PCG_NOALLOC_MAX_SLOTS;
   static constexpr size_t vectors = 0;                                   // z, r, p0, p1, ap, apFull
   static constexpr size_t localCol = vectors + sizeof(float4) * N;       // 16 bits a slot, over r and p0
   static constexpr size_t halo = localCol + sizeof(uint16_t) * B;        // over p1, ap and apFull
-  static constexpr size_t haloEntries = 3 * sizeof(float4) * N / sizeof(uint32_t);
   static constexpr size_t precond = vectors + 6 * sizeof(float4) * N;    // 3 float4 per particle
+  static constexpr size_t haloCount = precond - sizeof(uint32_t) * kNoAllocMaxBlocks;
+  static constexpr size_t haloEntries = (haloCount - halo) / sizeof(uint32_t);
   static constexpr size_t particle = precond + 3 * sizeof(float4) * N;
   static constexpr size_t contact = particle + sizeof(dcu::Particle) * N;
   static constexpr size_t diag = contact + sizeof(dcu::Contact) * N;
@@ -2020,9 +2020,8 @@ struct NoAllocLayout {
 };
 static_assert(sizeof(dcu::Control) <= 248, "control block fits its region");
 static_assert(sizeof(uint16_t) * NoAllocLayout::B == 2 * sizeof(float4) * NoAllocLayout::N, "local columns fill r and p0");
-static_assert(dcu::mailWords(kNoAllocMaxSms) * sizeof(dcu::MailWord) + kNoAllocMaxSms * sizeof(uint32_t) <=
-                  NoAllocLayout::control - NoAllocLayout::partials,
-              "mailbox and halo sizes fit the partials' region");
+static_assert(dcu::mailWords(kNoAllocMaxBlocks) * sizeof(dcu::MailWord) <= NoAllocLayout::control - NoAllocLayout::partials,
+              "the mailbox fits the partials' region");
 static_assert(NoAllocLayout::total == DRAPE_PCG_NOALLOC_SCRATCH_BYTES, "scratch size matches the header");
 
 // The scratch. In host code this name is a host-side stand-in, not a device address: the address a kernel may use
@@ -2039,7 +2038,8 @@ constexpr int kNoAllocMaxDevices = 64;
 NoAllocDevice g_noAlloc[kNoAllocMaxDevices];
 std::mutex g_noAllocMutex;
 
-size_t noAllocRowsSmem(int device);  // sets and returns k_noalloc_rows's dynamic shared memory
+size_t noAllocRowsSmem(int device);  // the most dynamic shared memory k_noalloc_rows can have
+void allowNoAllocRows(size_t smem);
 
 // The device address of the scratch array and the SM count, with `device` current. The SM count is looked up once per
 // device. The address is looked up again on every call made outside a stream capture (cudaGetSymbolAddress allocates
@@ -2058,10 +2058,11 @@ NoAllocDevice& noAllocScratch(int device, cudaStream_t stream) {
     CK(cudaGetSymbolAddress(&p, g_pcgScratch));
     if (!d.ready) {
       CK(cudaDeviceGetAttribute(&d.sms, cudaDevAttrMultiProcessorCount, device));
-      if (d.sms < 1 || static_cast<uint32_t>(d.sms) > kNoAllocMaxSms)
+      if (d.sms < 1 || static_cast<uint32_t>(d.sms) > kNoAllocMaxBlocks)
         throw std::runtime_error("cuda: unsupported SM count for the no-allocation PCG");
       d.residentSmem = noAllocRowsSmem(device);
     }
+    allowNoAllocRows(d.residentSmem);  // the permission goes with the context
     d.scratch = static_cast<unsigned char*>(p);
     d.ready = true;
   }
@@ -2204,9 +2205,11 @@ size_t noAllocRowsSmem(int device) {
   cudaFuncAttributes fa{};
   CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
   CK(cudaFuncGetAttributes(&fa, dcu::k_noalloc_rows));
-  const size_t most = (static_cast<size_t>(optin) - fa.sharedSizeBytes) & ~static_cast<size_t>(15);
-  CK(cudaFuncSetAttribute(dcu::k_noalloc_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)));
-  return most;
+  return (static_cast<size_t>(optin) - fa.sharedSizeBytes) & ~static_cast<size_t>(15);
+}
+
+void allowNoAllocRows(size_t smem) {
+  CK(cudaFuncSetAttribute(dcu::k_noalloc_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
 }
 
 }  // namespace
@@ -2271,7 +2274,7 @@ extern "C" int drape_cuda_pcg_noalloc(uint32_t n, uint32_t slots, const uint32_t
     d.mailSeq = mailSeq;
     d.localCol = reinterpret_cast<const uint16_t*>(base + L::localCol);
     d.halo = reinterpret_cast<const uint32_t*>(base + L::halo);
-    d.haloCount = reinterpret_cast<const uint32_t*>(mail + dcu::mailWords(sms));
+    d.haloCount = reinterpret_cast<const uint32_t*>(base + L::haloCount);
     d.P.haloStride = static_cast<uint32_t>(L::haloEntries) / sms;
     d.P.residentNodes = per + d.P.haloStride + 1;
     d.P.residentSlots = static_cast<uint32_t>((nd.residentSmem - d.P.residentNodes * dcu::kResidentNodeBytes) /
