@@ -896,7 +896,12 @@ struct drape_batch {
   // The rule: the default variant with block-Jacobi, whenever it fits in kWaves launches. Measured (us per Newton
   // iteration's solve on one B200, k_solve_batch<false, 0, 256> in brackets): 2 garments of 500 particles 165 (571), 5 of
   // 700-3,000 182 (514), 16 of 2k-40k (175k in all, one wave) 780-960 (1,740), 243k 1,075 (2,650), 394k 2,726 (4,173),
-  // 584k 4,001 (6,249); the fastest of the other variants takes 2,130, 3,403 and 5,124 for the last three.
+  // 584k 4,001 (6,249); the fastest of the other variants takes 2,130, 3,403 and 5,124 for the last three. Not for many tiny
+  // garments: a wave takes some 155 us whatever its garments' size, and from three waves on the slot-parallel kernel, with
+  // a block a garment, is done sooner where that block has little to do: 300 garments of 60 particles 463 (430), of 100
+  // 483 (468), of 112 538 (550); 590 of 100 649 (527), of 130 668 (626), of 150 699 (756). So the line is at 104 particles
+  // for three waves and at 136 for four.
+  static constexpr size_t kTinyWaves = 3;
   bool planResident(const std::vector<int>& substeps) {
     if (!residentForm()) return false;
     const uint32_t most = dcu::kMultiMost * dcu::kRowWorkers;
@@ -928,6 +933,9 @@ struct drape_batch {
       if (fits) wave = std::move(w);
     }
     if (wave.empty()) return false;
+    if (wave.size() >= kTinyWaves && rows(live.front()) <= 8 + 32 * wave.size() &&
+        live.size() <= static_cast<size_t>(solveBlocks))
+      return false;
     residentWaves = static_cast<int>(wave.size());
     residentRun.assign(G, bcu::SegRun{});
     residentStart.assign(static_cast<size_t>(residentWaves) * (G + 1), 0);
