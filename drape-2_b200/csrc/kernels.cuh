@@ -678,8 +678,8 @@ __device__ inline void assembleSlots(const Dev& D, uint32_t rank, uint32_t size)
 
 // ---------------------------------------------------------------------------------------------------------------
 // Energy at u + alpha * step, in FP64, summed per thread over particles (inertia + friction) and terms. At alpha = 0 the
-// step is not read: the solve's other blocks may not have written theirs yet, and what an abandoned solve left there need
-// not be finite.
+// step is not read (u stands for it, so that both take the same code): the solve's other blocks may not have written theirs
+// yet, and what an abandoned solve left there need not be finite.
 
 // Virtual thread vt of a block of vdim threads: the elements idx = rank * vdim + vt + k * size * vdim (a kernel whose
 // blocks stand for larger ones sums in the larger blocks' order).
@@ -688,20 +688,17 @@ __device__ inline double energyPartial(const Dev& D, const GridSync& gs, double 
   const uint32_t n = D.P.n, S = D.P.nStretch, H = D.P.nHinge, K = D.P.nSeam;
   const uint32_t total = n + S + H + K;
   const uint32_t stride = gs.size * vdim;
-  auto moved = [&](uint32_t i) -> d3 {
-    const d3 ui = toD(ld3(D.u, i));
-    return alpha == 0.0 ? ui : ui + alpha * toD(ld3(D.step, i));
-  };
+  const float4* step = alpha == 0.0 ? D.u : D.step;
   auto pos = [&](uint32_t v0, uint32_t vk) -> d3 {
     const d3 rel = toD(ld3(D.xStart, vk)) - toD(ld3(D.xStart, v0));
-    return rel + moved(vk);
+    return rel + (toD(ld3(D.u, vk)) + alpha * toD(ld3(step, vk)));
   };
   const double invH2 = 1.0 / (D.P.hD * D.P.hD);
   for (uint32_t idx = gs.rank * vdim + vt; idx < total; idx += stride) {
     if (idx < n) {
       const uint32_t i = idx;
       const Particle pa = D.particle[i];
-      const d3 ui = moved(i);
+      const d3 ui = toD(ld3(D.u, i)) + alpha * toD(ld3(step, i));
       if (pa.pinned == 0u) {
         const d3 dd = ui - toD(ld3(D.yRel, i));
         e += 0.5 * static_cast<double>(pa.mass) * invH2 * dotd(dd, dd);
