@@ -1996,29 +1996,40 @@ int drape_cuda_inject_failure(drape_solver* s, int steps) {
 
 namespace {
 
+constexpr uint32_t kNoAllocPrepareThreads = 256;
 constexpr uint32_t kNoAllocMaxBlocks = 256;  // partials capacity (grid = one block per SM)
 
 // Byte layout of the scratch array (every region 256-byte aligned). A call uses it in one of two ways (k_noalloc_localize
-// decides): for the resident-row PCG the vectors after z hold the slots' local columns, the halos and their sizes, and the
-// partials' region the mailbox; for the 1024-thread PCG they are what their names say.
+// decides): for the resident-row PCG the vectors after z hold the slots' local columns and the halos, and the partials'
+// region the mailbox and the halos' sizes (which go to the halos' end on the grids for which it is too small); for the
+// 1024-thread PCG they are what their names say.
 struct NoAllocLayout {
   static constexpr size_t N = DRAPE_PCG_NOALLOC_MAX_PARTICLES, B = DRAPE_PCG_NOALLOC_MAX_SLOTS;
   static constexpr size_t vectors = 0;                                   // z, r, p0, p1, ap, apFull
   static constexpr size_t localCol = vectors + sizeof(float4) * N;       // 16 bits a slot, over r and p0
   static constexpr size_t halo = localCol + sizeof(uint16_t) * B;        // over p1, ap and apFull
   static constexpr size_t precond = vectors + 6 * sizeof(float4) * N;    // 3 float4 per particle
-  static constexpr size_t haloCount = precond - sizeof(uint32_t) * kNoAllocMaxBlocks;
-  static constexpr size_t haloEntries = (haloCount - halo) / sizeof(uint32_t);
   static constexpr size_t particle = precond + 3 * sizeof(float4) * N;
   static constexpr size_t contact = particle + sizeof(dcu::Particle) * N;
   static constexpr size_t diag = contact + sizeof(dcu::Contact) * N;
   static constexpr size_t cols = diag + sizeof(uint32_t) * N;
   static constexpr size_t partials = cols + sizeof(uint32_t) * B;
   static constexpr size_t control = partials + 2 * kNoAllocMaxBlocks * dcu::kPartialStride * sizeof(double);
+  static constexpr size_t badBlock = control + 216;                      // a byte per block of k_noalloc_prepare
   static constexpr size_t mailSeq = control + 248;                       // kept from call to call
   static constexpr size_t total = control + 256;
+  // The halos' sizes on a grid of `blocks` blocks, and the entries of all halos.
+  static constexpr size_t haloCount(uint32_t blocks) {
+    const size_t behindMail = partials + dcu::mailWords(blocks) * sizeof(dcu::MailWord);
+    return behindMail + sizeof(uint32_t) * blocks <= control ? behindMail : precond - sizeof(uint32_t) * blocks;
+  }
+  static constexpr size_t haloEntries(uint32_t blocks) {
+    return (std::min(haloCount(blocks), precond) - halo) / sizeof(uint32_t);
+  }
 };
-static_assert(sizeof(dcu::Control) <= 248, "control block fits its region");
+static_assert(sizeof(dcu::Control) <= NoAllocLayout::badBlock - NoAllocLayout::control, "control block fits its region");
+static_assert(NoAllocLayout::N / kNoAllocPrepareThreads <= NoAllocLayout::mailSeq - NoAllocLayout::badBlock,
+              "the flags of k_noalloc_prepare's blocks fit their region");
 static_assert(sizeof(uint16_t) * NoAllocLayout::B == 2 * sizeof(float4) * NoAllocLayout::N, "local columns fill r and p0");
 static_assert(dcu::mailWords(kNoAllocMaxBlocks) * sizeof(dcu::MailWord) <= NoAllocLayout::control - NoAllocLayout::partials,
               "the mailbox fits the partials' region");
@@ -2077,27 +2088,25 @@ namespace dcu {
 // non-decreasing from 0 to `slots`, a column index >= n, or a row without its diagonal block.
 constexpr int kNoAllocBadStructure = 3;
 
-// Clears the control block, the iteration output and the mailbox (one block) before the structure check can raise an
-// error in it.
-__global__ void k_noalloc_clear(Control* ctl, int* iterations, MailWord* mail, uint32_t words) {
-  if (threadIdx.x == 0) {
-    *ctl = Control{};
-    *iterations = 0;
-  }
-  for (uint32_t k = threadIdx.x; k < words; k += blockDim.x) mail[k] = MailWord{0.0, 0ull};
-}
-
 // Converts the caller's flags into the solver's layouts inside the scratch (particle pinned flags, contact state,
 // columns with the pinned bit, diagonal slots) and checks the structure on the way. Every read and write stays in
 // bounds whatever the caller passed: slot indices are clamped to [0, slots) and column indices are checked against n
-// before they index `pinned`; a violation raises kNoAllocBadStructure and leaves in-range placeholders behind, which
-// the solve never reads because it does not start.
+// before they index `pinned`; a violation marks the block in `badBlock` (k_noalloc_localize raises the error) and leaves
+// in-range placeholders behind, which the solve never reads because it does not start. Also clears the control block,
+// the iteration output and the mailbox, which nothing else touches here.
 __global__ void k_noalloc_prepare(uint32_t n, uint32_t slots, const uint32_t* __restrict__ rowStart,
                                   const uint32_t* __restrict__ colIndex, const uint8_t* __restrict__ pinned,
                                   const uint8_t* __restrict__ active, const float4* __restrict__ normals,
-                                  Particle* particle, Contact* contact, uint32_t* cols, uint32_t* diag, Control* ctl) {
+                                  Particle* particle, Contact* contact, uint32_t* cols, uint32_t* diag, uint8_t* badBlock,
+                                  Control* ctl, int* iterations, MailWord* mail, uint32_t mailCount) {
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
-  if (tid == 0 && (rowStart[0] != 0u || rowStart[n] != slots)) atomicExch(&ctl->error, kNoAllocBadStructure);
+  bool bad = false;
+  if (tid == 0) {
+    *ctl = Control{};
+    *iterations = 0;
+    bad = rowStart[0] != 0u || rowStart[n] != slots;
+  }
+  for (uint32_t k = tid; k < mailCount; k += stride) mail[k] = MailWord{0.0, 0ull};
   for (uint32_t i = tid; i < n; i += stride) {
     particle[i] = Particle{1.0f, 0u, 0u, pinned[i] ? 1u : 0u};
     Contact c{};
@@ -2106,7 +2115,7 @@ __global__ void k_noalloc_prepare(uint32_t n, uint32_t slots, const uint32_t* __
     if (normals) c.normal = make_float4(normals[i].x, normals[i].y, normals[i].z, 0.0f);
     contact[i] = c;
     const uint32_t rs = rowStart[i], re = rowStart[i + 1];
-    bool bad = rs > re || re > slots;
+    bad = bad || rs > re || re > slots;
     const uint32_t lo = min(rs, slots), hi = min(max(rs, re), slots);
     uint32_t d = slots;
     for (uint32_t s = lo; s < hi; ++s) {
@@ -2124,16 +2133,22 @@ __global__ void k_noalloc_prepare(uint32_t n, uint32_t slots, const uint32_t* __
       d = 0u;  // slots >= n >= 1 (checked on the host), so slot 0 exists
     }
     diag[i] = d;
-    if (bad) atomicExch(&ctl->error, kNoAllocBadStructure);
   }
+  const int any = __syncthreads_or(bad);
+  if (threadIdx.x == 0) badBlock[blockIdx.x] = any ? 1 : 0;
 }
 
-// Skipped, like the solves, once the structure check has failed (every block reads the same flag, written by an earlier
-// kernel on the stream, so a cooperative launch returns as a whole). One block per solve block: the block-Jacobi inverses
+// Raises the error where the structure check has failed; this kernel and the solves are skipped then (every block of a
+// solve reads the same flag, written by an earlier kernel on the stream, so a cooperative launch returns as a whole). One
+// block per solve block: the block-Jacobi inverses
 // of its rows, its halo and local columns, and whether it fits the resident-row PCG's layout; a block that does not sets
 // Control::newtonDone, which sends the call to the 1024-thread PCG.
-__global__ void __launch_bounds__(512) k_noalloc_localize(Dev D, const uint32_t* __restrict__ diag) {
-  if (*reinterpret_cast<volatile int*>(&D.ctl->error) != 0) return;
+__global__ void __launch_bounds__(512) k_noalloc_localize(Dev D, const uint32_t* __restrict__ diag,
+                                                          const uint8_t* __restrict__ badBlock, uint32_t prepareBlocks) {
+  if (__syncthreads_or(threadIdx.x < prepareBlocks && badBlock[threadIdx.x] != 0)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) D.ctl->error = kNoAllocBadStructure;
+    return;
+  }
   const uint32_t SP = D.P.slotsPadded, t = threadIdx.x, lane = t & 31u, w = t >> 5;
   uint32_t r0, r1;
   blockRange(D.P.n, blockIdx.x, gridDim.x, r0, r1);
@@ -2274,20 +2289,19 @@ extern "C" int drape_cuda_pcg_noalloc(uint32_t n, uint32_t slots, const uint32_t
     d.mailSeq = mailSeq;
     d.localCol = reinterpret_cast<const uint16_t*>(base + L::localCol);
     d.halo = reinterpret_cast<const uint32_t*>(base + L::halo);
-    d.haloCount = reinterpret_cast<const uint32_t*>(base + L::haloCount);
-    d.P.haloStride = static_cast<uint32_t>(L::haloEntries) / sms;
+    d.haloCount = reinterpret_cast<const uint32_t*>(base + L::haloCount(sms));
+    d.P.haloStride = static_cast<uint32_t>(L::haloEntries(sms)) / sms;
     d.P.residentNodes = per + d.P.haloStride + 1;
     d.P.residentSlots = static_cast<uint32_t>((nd.residentSmem - d.P.residentNodes * dcu::kResidentNodeBytes) /
                                               dcu::kResidentSlotBytes) & ~31u;
-    const int pg = std::max(1, static_cast<int>((n + 255) / 256));
-    dcu::k_noalloc_clear<<<1, 256, 0, st>>>(d.ctl, d_iterations, mail, static_cast<uint32_t>(dcu::mailWords(sms)));
-    CK(cudaGetLastError());
-    dcu::k_noalloc_prepare<<<pg, 256, 0, st>>>(
+    const uint32_t pg = (n + kNoAllocPrepareThreads - 1) / kNoAllocPrepareThreads;
+    auto* bad = base + L::badBlock;
+    dcu::k_noalloc_prepare<<<pg, kNoAllocPrepareThreads, 0, st>>>(
         n, slots, d_row_start, d_col_index, d_pinned, d_active, static_cast<const float4*>(d_normals),
         reinterpret_cast<dcu::Particle*>(base + L::particle), d.contact, reinterpret_cast<uint32_t*>(base + L::cols),
-        diag, d.ctl);
+        diag, bad, d.ctl, d_iterations, mail, static_cast<uint32_t>(dcu::mailWords(sms)));
     CK(cudaGetLastError());
-    dcu::k_noalloc_localize<<<nd.sms, 512, 2 * sizeof(uint32_t) * ((n + 31) / 32), st>>>(d, diag);
+    dcu::k_noalloc_localize<<<nd.sms, 512, 2 * sizeof(uint32_t) * ((n + 31) / 32), st>>>(d, diag, bad, pg);
     CK(cudaGetLastError());
     void* args[] = {&d};
     CK(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(dcu::k_noalloc_rows), dim3(nd.sms), dim3(dcu::kRowThreads),
