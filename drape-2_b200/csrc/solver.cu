@@ -1806,12 +1806,17 @@ int drape_cuda_spmv_device(uint32_t n, const uint32_t* d_row_start, const uint32
     int sms = 0;
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     // Four slots a thread where each plane's slots are 16-byte aligned alike and the blocks fill their waves better: up to
-    // one wave of wide blocks, and up to two where the narrow ones need a second wave too. Narrow -> wide, us: 40,000 rows
-    // 10.2 -> 5.4, 76,000 14.0 -> 13.4; between, one narrow wave against two wide ones: 100,000 15.7 -> 18.6; 120,000
-    // 24.3 -> 20.0, 150,000 25.8 -> 22.3; past that the narrow ones have more bytes in flight: 200,000 28.4 -> 29.9.
+    // one wave of wide blocks, and up to two where the narrow ones need a second wave too (from one whole block more than a
+    // wave on; a part of one is done soon). Narrow -> wide, us: 40,000 rows 10.2 -> 5.4, 76,000 14.0 -> 13.4; between, one
+    // narrow wave against two wide ones: 100,000 15.7 -> 18.6; 115,000 23.5 -> 19.8, 120,000 24.3 -> 20.0, 150,000 25.8 ->
+    // 22.3; past that the narrow ones have more bytes in flight: 200,000 28.4 -> 29.9. These are matrices that come from
+    // HBM. One that stays in the L2 from call to call (13 slots a row): 40,000 6.7 -> 5.4, 60,000 7.3 -> 7.5, 76,000 7.5 ->
+    // 8.1 (past 1,024 slots a block the wide ones take a second, nearly empty chunk), 130,000 14.0 -> 14.2. A matrix of at
+    // most 256 slots is one round of one narrow block: 33 rows of 3 slots 2.14 -> 2.30.
     const uint32_t resident = static_cast<uint32_t>(sms) * dcu::kSpmvWidePerSm, wave = resident * dcu::kSpmvBlockRows;
     const uint32_t narrowWave = static_cast<uint32_t>(sms) * dcu::kSpmvPerSm * dcu::kSpmvBlockRows;
-    const bool wide = (n <= wave || (n > narrowWave && n <= 2 * wave)) && slots_padded % 4 == 0 &&
+    const bool wide = (n <= wave || (n >= narrowWave + dcu::kSpmvBlockRows && n <= 2 * wave)) &&
+                      slots_padded > dcu::kSpmvThreads && slots_padded % 4 == 0 &&
                       reinterpret_cast<uintptr_t>(d_blocks) % 16 == 0 &&
                       reinterpret_cast<uintptr_t>(d_col_index) % 16 == 0;
     if (wide) {
