@@ -902,6 +902,9 @@ struct drape_batch {
   // 483 (468), of 112 538 (550); 590 of 100 649 (527), of 130 668 (626), of 150 699 (756). So the line is at 104 particles
   // for three waves and at 136 for four.
   static constexpr size_t kTinyWaves = 3;
+  // Nor for solves capped at a few iterations where a thread owns several rows: staging then costs more than they save
+  // (16 garments of 12,000, us a solve: three iterations 215 -> 234, eight 405 -> 331).
+  static constexpr int kMultiLeastCg = 5;
   bool planResident(const std::vector<int>& substeps) {
     if (!residentForm()) return false;
     const uint32_t most = dcu::kMultiMost * dcu::kRowWorkers;
@@ -969,6 +972,8 @@ struct drape_batch {
     uint64_t spillMost = 0, haloEntries = 0;
     size_t smem = 0;
     uint32_t mostRows = 0;
+    int mostCg = 0;
+    for (uint32_t g : live) mostCg = std::max(mostCg, models[g].settings.max_cg_iterations);
     for (int k = 0; k < residentWaves; ++k) {
       uint64_t spillBytes = 0;  // the waves use the spill buffer one after the other
       for (uint32_t g : wave[k]) {
@@ -999,6 +1004,8 @@ struct drape_batch {
       }
       spillMost = std::max(spillMost, spillBytes);
     }
+    residentRows = static_cast<int>((mostRows + dcu::kRowWorkers - 1) / dcu::kRowWorkers);
+    if (residentRows > 1 && mostCg < kMultiLeastCg) return false;
     if (spillMost > spill.n || !spill.p) {
       dropGraph();
       spill.alloc(std::max<uint64_t>(spillMost, 16));
@@ -1009,7 +1016,6 @@ struct drape_batch {
       halo.alloc(std::max<uint64_t>(haloEntries, 1));
       view.halo = halo.p;
     }
-    residentRows = static_cast<int>((mostRows + dcu::kRowWorkers - 1) / dcu::kRowWorkers);
     residentSmem = smem;
     writeResident();
     uploadControl();

@@ -418,7 +418,11 @@ struct drape_solver {
 
   // Picks the resident-row kernel that every solve block fits, if one does, and builds its index arrays: the halos, and
   // the columns as indices into a block's rows and halo. One row a thread with the whole matrix on chip is the fastest
-  // form; else the fewest rows a thread, with the matrix partly in the L2.
+  // form; else the fewest rows a thread, with the matrix partly in the L2. Writing that part takes as long as two iterations
+  // save: solves capped at one iteration stay on the 1024-thread kernel (us a solve, 1024 threads / several rows a thread, at
+  // 90k, 150k and 207k particles: one iteration 77 / 94, 109 / 147, 147 / 201; three 108 / 109, 162 / 168, 244 / 245;
+  // eight 188 / 143, 294 / 220, 488 / 357).
+  static constexpr int kMultiLeastCg = 3;
   void localize(uint32_t n, uint32_t B, dcu::Dev& d) {
     residentSmemBytes = learnedSmemBytes = 0;
     const uint32_t per = (n + static_cast<uint32_t>(solveGrid) - 1) / static_cast<uint32_t>(solveGrid);
@@ -456,6 +460,8 @@ struct drape_solver {
         learnedFactorOnChip = more + factorBytes <= learnedSmemCap;
         learnedSmemBytes = more + (learnedFactorOnChip ? factorBytes : 0);
       }
+    } else if (m.settings.max_cg_iterations < kMultiLeastCg) {
+      return;
     } else {
       residentRowsPerThread = per <= static_cast<uint32_t>(2 * dcu::kRowWorkers) ? 2 : 3;
       const size_t cap = residentSmemCap[residentRowsPerThread - 1];
