@@ -114,6 +114,7 @@ struct Mesh {
   const D3* v;
   const uint3* t;
   const double* tbox;  // per triangle: tmin xyz, tmax xyz
+  const double* tboxWide;  // the same, larger by 2^-48 of the largest coordinate (pass 2)
   const int* trange;   // per triangle: x0 x1 y0 y1 z0 z1 (sample box, inclusive)
   const D3* faceN;     // per triangle
   const D3* vertexN;   // per vertex
@@ -126,7 +127,7 @@ __device__ __forceinline__ D3 samplePos(const Grid& g, int x, int y, int z) {
 }
 
 // Squared distance from p to a box, lower corner then upper (the reference's cheap reject, with the triangle's bounding box).
-__device__ __forceinline__ double boxGap2(const double (&tb)[6], D3 p) {
+__device__ __forceinline__ double boxGap2(const double* tb, D3 p) {
   const double gx = fmax(fmax(dsub(tb[0], p.x), dsub(p.x, tb[3])), 0.0);
   const double gy = fmax(fmax(dsub(tb[1], p.y), dsub(p.y, tb[4])), 0.0);
   const double gz = fmax(fmax(dsub(tb[2], p.z), dsub(p.z, tb[5])), 0.0);
@@ -162,20 +163,7 @@ __global__ void __launch_bounds__(kBakeThreads) k_bake_distance(Grid g, Mesh m, 
   const int bx = r[1] - r[0] + 1, by = r[3] - r[2] + 1, bz = r[5] - r[4] + 1;
   const uint3 tri = m.t[task.tri];
   const D3 a = m.v[tri.x], b = m.v[tri.y], c = m.v[tri.z];
-  double tb[6];
-#pragma unroll
-  for (int k = 0; k < 6; ++k) tb[k] = m.tbox[6 * static_cast<size_t>(task.tri) + k];
-  if (Owner) {
-    double most = 0.0;
-#pragma unroll
-    for (int k = 0; k < 6; ++k) most = fmax(most, fabs(tb[k]));
-    const double slack = 0x1p-48 * most;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-      tb[k] = dsub(tb[k], slack);
-      tb[k + 3] = add(tb[k + 3], slack);
-    }
-  }
+  const double* tb = (Owner ? m.tboxWide : m.tbox) + 6 * static_cast<size_t>(task.tri);
   const uint32_t first = task.sub * chunk, last = min(first + chunk, static_cast<uint32_t>(bx) * by * bz);
   for (uint32_t s = first + threadIdx.x; s < last; s += kBakeThreads) {
     const uint32_t row = s / bx, slab = row / by;
@@ -471,7 +459,7 @@ int drape_bake_field(int device, const drape_mesh_desc* components, uint32_t cou
     }
     std::vector<D3> v, faceN, vertexN(allV, D3{0, 0, 0}), edgeN(3 * allT);
     std::vector<uint3> tris;
-    std::vector<double> tbox(6 * allT);
+    std::vector<double> tbox(6 * allT), tboxWide(6 * allT);
     std::vector<int> trange(6 * allT);
     v.reserve(allV);
     faceN.reserve(allT);
@@ -507,9 +495,13 @@ int drape_bake_field(int device, const drape_mesh_desc* components, uint32_t cou
                               std::min(std::min(a.z, b.z), c3.z)};
         const double mx[3] = {std::max(std::max(a.x, b.x), c3.x), std::max(std::max(a.y, b.y), c3.y),
                               std::max(std::max(a.z, b.z), c3.z)};
+        double most = 0.0;
+        for (int a3 = 0; a3 < 3; ++a3) most = std::max({most, std::fabs(mn[a3]), std::fabs(mx[a3])});
         for (int a3 = 0; a3 < 3; ++a3) {
           tbox[6 * (t0 + t) + a3] = mn[a3];
           tbox[6 * (t0 + t) + 3 + a3] = mx[a3];
+          tboxWide[6 * (t0 + t) + a3] = mn[a3] - 0x1p-48 * most;
+          tboxWide[6 * (t0 + t) + 3 + a3] = mx[a3] + 0x1p-48 * most;
           const double oa = origin[a3];
           const double i0 = std::max(0.0, std::ceil(((mn[a3] - o.band) - oa) / o.cell_size));
           const double i1 = std::min<double>(dims[a3] - 1, std::floor(((mx[a3] + o.band) - oa) / o.cell_size));
@@ -598,7 +590,7 @@ int drape_bake_field(int device, const drape_mesh_desc* components, uint32_t cou
     }
     DBuf<D3> dv, dface, dvert, dedge;
     DBuf<uint3> dtri;
-    DBuf<double> dbox;
+    DBuf<double> dbox, dboxWide;
     DBuf<int> drange, changed;
     DBuf<bake::Part> dparts;
     DBuf<bake::Task> dtasks;
@@ -613,6 +605,7 @@ int drape_bake_field(int device, const drape_mesh_desc* components, uint32_t cou
       dedge.upload(edgeN, st);
       dtri.upload(tris, st);
       dbox.upload(tbox, st);
+      dboxWide.upload(tboxWide, st);
       drange.upload(trange, st);
       dparts.upload(parts, st);
       dtasks.upload(tasks, st);
@@ -622,7 +615,7 @@ int drape_bake_field(int device, const drape_mesh_desc* components, uint32_t cou
       outside.alloc(mostWords);
       changed.alloc(2);
     }
-    const bake::Mesh dm{dv.p, dtri.p, dbox.p, drange.p, dface.p, dvert.p, dedge.p};
+    const bake::Mesh dm{dv.p, dtri.p, dbox.p, dboxWide.p, drange.p, dface.p, dvert.p, dedge.p};
     KCK(cudaStreamSynchronize(st));  // the uploads' host arrays may go
     KCK(cudaEventRecord(e0, st));
     bake::k_fill<<<pointGrid, 256, 0, st>>>(field.p, total, static_cast<float>(o.band));
