@@ -533,9 +533,10 @@ int drape_bake_field(int device, const drape_mesh_desc* components, uint32_t cou
         }
     }
     // Each component's box, the groups of components that run together (no more samples than the grid has, which one box
-    // alone never exceeds), and the groups' tasks: chunks of 2,048 samples, larger where that would make more than 2^16
+    // alone never exceeds), and the groups' tasks: chunks of 2,048 samples, larger where that would make more than 2^18
     // tasks besides one a triangle. The host writes and uploads every task: a sphere of 5,120 triangles with boxes of
-    // 500,000 samples took 38 ms with a million tasks, 27 so, and 32 with one block a triangle.
+    // 500,000 samples took 35-38 ms with 2^20 tasks, 29 with 2^18, 27 with 2^16 (32 with one block a triangle); 200 spheres
+    // with as wide a band 52, 48 and 52.
     std::vector<bake::Part> parts;
     std::vector<size_t> partTri;  // parts[k]'s triangles are [partTri[2 k], partTri[2 k + 1])
     size_t pairs = 0;
@@ -560,7 +561,7 @@ int drape_bake_field(int device, const drape_mesh_desc* components, uint32_t cou
       parts.push_back({lo[0], lo[1], lo[2], nx, hi[1] - lo[1] + 1, hi[2] - lo[2] + 1, (nx + 31) / 32, 0, 0});
       partTri.insert(partTri.end(), {t0, t1});
     }
-    const size_t chunk = std::max<size_t>(2048, (pairs >> 16) + 1);
+    const size_t chunk = std::max<size_t>(2048, (pairs >> 18) + 1);
     struct Group {
       size_t part0, part1, task0, task1, samples, lines;
     };
