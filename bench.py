@@ -910,13 +910,16 @@ def main():
                        "by messages and runs below it); us_per_pcg_iteration = in-kernel PCG time / PCG iterations over "
                        "the timed drapes (CG init amortised); onchip_gbs = the iteration's algorithmic bytes over its "
                        "time, served from shared memory and L2"}
-    roofline = {"bound": "hbm", "kernel": "k_solve", "achieved": achieved, "peak": peak, "unit": "GB/s",
+    roofline = {"bound": "latency of the grid's exchanges, then shared memory" if solve_threads == 512
+                         else "latency of the grid's exchanges",
+                "kernel": "k_solve_rows" if solve_threads == 512 else "k_solve", "achieved": achieved, "peak": peak, "unit": "GB/s",
                 "frac": achieved / peak if peak else None, "peak_source": peak_kind,
                 "traffic": traffic, "algorithmic_bytes_per_launch": solve_bytes / solve_launches,
                 "avg_launch_ms": solve_ms / solve_launches,
-                "bound_note": "HBM is not what limits k_solve: its DRAM traffic is a small part of its algorithmic "
-                              "bytes (the matrix sits in shared memory and L2); the limit is grid-exchange latency, "
-                              "see the line's k_solve_latency object",
+                "bound_note": "achieved, peak and frac set the algorithmic bytes against HBM, which does not limit the "
+                              "kernel: its DRAM traffic is a small part of them (the matrix sits in registers, shared "
+                              "memory and L2), so frac may exceed 1; the limit is grid-exchange latency, see the "
+                              "line's k_solve_latency object",
                 "kernel_share": {k: (v / total_ms if total_ms else 0.0) for k, v in share_prof["milliseconds"].items()},
                 "kernel_share_sample": "one extra drape of the workload's own start state, every kernel timed"}
 

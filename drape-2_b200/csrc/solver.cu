@@ -602,8 +602,9 @@ struct drape_solver {
     CK(cudaMemcpy(mailSeq(), &seq, sizeof(seq), cudaMemcpyHostToDevice));
   }
 
-  // The reference-order PCG runs over resident rows (k_solve_rows) where the built scene fits it; bit-identical to
-  // k_solve<false, 0>, which variant 3 forces. The learned preconditioner runs over resident rows too
+  // The reference-order PCG runs over resident rows (k_solve_cluster, k_solve_rows, k_solve_rows_multi) where the built
+  // scene fits: the products and recurrences of k_solve<false, 0>, which variant 3 forces, with the FP64 sums grouped
+  // differently (the same results wherever these round to the same FP32 scalars and decisions). The learned preconditioner runs over resident rows too
   // (k_solve_rows_learned) unless block-Jacobi iterations come first (precondSwitch) or variant 3 forces k_solve<true>.
   bool usesResidentRows(const dcu::Dev& d) const {
     if (d.P.pcgVariant != 0) return false;
@@ -779,7 +780,8 @@ struct drape_solver {
   // frames, ~14 ms of device work) do not keep a host core busy, which a CPU-quota-limited host would throttle while
   // the device drains its queue. A sleep lasts about 75 us, so it polls again without sleeping for waitSpinUs before and
   // after the length of the last wait of the same kind: a wait of a steady kind ends when the device does (the frame of
-  // the 1,600-particle sheet, its device work done in 400 us: 477 us before, 421 us so). waitSpinUs = UINT32_MAX polls without sleeping.
+  // the 1,600-particle sheet, its device work done in 400 us: 477 us before, 421 us so from the second frame on; the first
+  // wait of a kind sleeps past the device's end as before). waitSpinUs = UINT32_MAX polls without sleeping.
   enum WaitKind { kWaitStep, kWaitStats, kWaitFrames, kWaitKinds };
   uint32_t waitSpinUs = 200;
   long long lastWaitUs[kWaitKinds] = {};

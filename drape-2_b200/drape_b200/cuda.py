@@ -340,7 +340,7 @@ class CudaSolver:
     def set_pcg_variant(self, variant: int) -> None:
         """0: the reference-order block-Jacobi PCG (default; resident rows where the scene fits); 1: pipelined, one
         grid exchange per iteration; 2: Chronopoulos-Gear, one reduction and one plain barrier per iteration; 3: the
-        reference order on the 1024-thread kernel (bit-identical to 0)."""
+        reference order on the 1024-thread kernel (the products and recurrences of 0)."""
         self._check(self.L.drape_cuda_set_pcg_variant(self.h, int(variant)))
 
     def solve_threads(self) -> int:

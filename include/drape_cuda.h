@@ -223,23 +223,30 @@ int drape_cuda_frame_times(drape_solver* s, uint64_t* begin_ns, uint64_t* end_ns
 int drape_cuda_runner_host_seconds(const drape_solver* s, double* out);
 
 /* How the host waits for the solver's stream (no reference counterpart): it polls for up to `spin_microseconds`, then
-   sleeps 20 us between polls (default 200; UINT32_MAX polls without sleeping). Results do not depend on it. */
+   sleeps 20 us between polls, and polls again without sleeping from that long before until that long after the length of
+   the handle's last wait of the same kind (a step, statistics, a drape's batch of frames), so that a wait of a steady kind
+   ends when the device does (default 200; UINT32_MAX polls without sleeping; 0 always sleeps). Reads of positions and
+   velocities, which follow such a wait, poll without sleeping until they are done. Results do not depend on it. */
 int drape_cuda_set_host_wait(drape_solver* s, uint32_t spin_microseconds);
 
 /* The block-Jacobi PCG's form (no reference counterpart; each solves the reference's contact-filtered system with its
    stopping tests, cpu_solver.cpp:169-213): 0 (the default) the reference's order, two grid-wide reductions per
-   iteration, run over resident rows (one 512-thread block per SM, each row's PCG state in its thread's registers, the
-   block's matrix in a sliced layout in shared memory) where every block has at most 480 rows and its sliced matrix, its
-   rows' z and its neighbours' fit in shared memory, else up to three rows a thread with the matrix partly in the L2
-   (at most 1440 rows a block), else on one 1024-thread block per SM: the two kernels give bit-identical results; 1 pipelined
+   iteration, run over resident rows (512-thread blocks, each row's PCG state in its thread's registers, the block's
+   matrix in a sliced layout in shared memory): on one cluster of 16 blocks up to 3,500 particles; on one block per SM where
+   every block has at most 480 rows and its sliced matrix, its rows' z and its neighbours' fit in shared memory; with up to
+   three rows a thread and the matrix partly in the L2 (at most 1440 rows a block, an iteration cap of 3 or more); else on
+   one 1024-thread block per SM. All repeat the same FP32 products and recurrences and group the FP64 sums differently:
+   the results are the same bit for bit wherever these sums round to the same FP32 scalars and the same stopping and line
+   search decisions, which they did on every scene tested; 1 pipelined
    (Ghysels and Vanroose 2014), one reduction per iteration and three more work vectors, its FP32 recurrences drifting
    further from the products they stand for; 2 Chronopoulos-Gear, one reduction and one plain barrier per iteration
    with the reference order's recurrences; 3 the reference's order on the 1024-thread kernel whatever the scene (for
    comparison). Forms 0-2 give the same iterates in exact arithmetic and round differently. The learned preconditioner
    always runs its own PCG. */
 int drape_cuda_set_pcg_variant(drape_solver* s, int variant);
-/* Threads per block of the built scene's solve kernel under the current settings: 512 when the reference-order PCG runs
-   over resident rows (one or several a thread), else 1024 (the grid has one block per SM either way). */
+/* Threads per block of the built scene's solve kernel under the current settings: 512 when the reference-order or the
+   learned PCG runs over resident rows (one or several a thread), else 1024. The grid has one block per SM, except for the
+   reference-order PCG of up to 3,500 particles, which runs on one cluster of 16 blocks. */
 int drape_cuda_solve_threads(const drape_solver* s, int* threads);
 
 /* The bounded wait of the device grid barrier, in nanoseconds (0 restores the default of 2 s). A kernel whose barrier
