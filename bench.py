@@ -568,8 +568,8 @@ def batch_leg(args, device, world, rank, max_over_ranks, peak):
     settle_s = [float(t) for t, ok in zip(secs, settled) if ok]
     out = {
         "workload": f"{args.batch_garments} seamed tubes, particles log-uniform 2k-40k, each on its own seeded "
-                    "capsule-union body (32^3-128^3 field), one persistent solve launch per Newton iteration, frames "
-                    "replayed from a CUDA graph, autotuned solve variant, block-Jacobi PCG cap 50 / tol 1e-2",
+                    "capsule-union body (32^3-128^3 field), one or several persistent solve launches per Newton iteration, "
+                    "frames replayed from a CUDA graph, autotuned solve variant, block-Jacobi PCG cap 50 / tol 1e-2",
         "garments": G, "particles": N, "block_slots": B, "rank_garments": len(mine),
         "settled_per_s": sum(settled) / total if total else None,
         "settled": int(sum(settled)), "unsettled": int(len(settled) - sum(settled)),
